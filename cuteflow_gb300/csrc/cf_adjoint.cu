@@ -73,9 +73,8 @@ __global__ void __launch_bounds__(TILE_E, 8) k_rep_edges(StepArgs a, const doubl
   const size_t h = hidx(n, m, a.nmembers);
   const double dt = __ldg(dt_hist + h), t = __ldg(t_hist + h);
   if (a.xd_cmp) {   /* the context's integer-pipe setting, as the step's edge kernel (same results) */
-    constexpr bool OC = IFLUX != 3;   /* as the forward edge kernel */
-    if ((a.xd_mul_mask >> (threadIdx.x >> 5)) & 1) edge_body<IFLUX, XD<true, OC>>(a, M, e, dt, t);
-    else edge_body<IFLUX, XD<false, OC>>(a, M, e, dt, t);
+    if ((a.xd_mul_mask >> (threadIdx.x >> 5)) & 1) edge_body<IFLUX, XD<true>>(a, M, e, dt, t);
+    else edge_body<IFLUX, XD<false>>(a, M, e, dt, t);
   } else {
     edge_body<IFLUX>(a, M, e, dt, t);
   }
@@ -287,8 +286,8 @@ __device__ __forceinline__ void adj_interior_edge(const AdjArgs& A, const Member
   if (IFLUX >= 3) {
     up = ldro(a.eupw + e);
     dw = ld4(a.ewts + e);
-    upwind_state(a.Uin, up.x, up.y, dw.x, dw.y, G.ysum_a, G.nx, G.ny, M.tolisec, hl_upw, vl_upw);
-    upwind_state(a.Uin, up.z, up.w, dw.z, dw.w, G.ysum_b, G.nx, G.ny, M.tolisec, hr_upw, vr_upw);
+    upwind_state(a.Uin, up.x, up.y, dw.x, dw.y, dw.x + dw.y, G.ysum_a, G.nx, G.ny, M.tolisec, hl_upw, vl_upw);
+    upwind_state(a.Uin, up.z, up.w, dw.z, dw.w, dw.z + dw.w, G.ysum_b, G.nx, G.ny, M.tolisec, hr_upw, vr_upw);
   }
   constexpr int NDIR = (IFLUX >= 3) ? 10 : 6;
   const double w[10] = {wa.f1, wa.f2, wa.f3, wa.bx, wa.by, wb.f1, wb.f2, wb.f3, wb.bx, wb.by};

@@ -145,12 +145,14 @@ template <int N> CFD_HD bool operator<(const Dual<N>& a, const Dual<N>& b) { ret
 template <int N> CFD_HD bool operator>(const Dual<N>& a, const Dual<N>& b) { return xlt(b.v, a.v); }
 template <int N> CFD_HD bool operator<=(const Dual<N>& a, const Dual<N>& b) { return xle(a.v, b.v); }
 template <int N> CFD_HD bool operator>=(const Dual<N>& a, const Dual<N>& b) { return xle(b.v, a.v); }
-template <int N> CFD_HD bool operator<(const Dual<N>& a, double b) { return xlt(a.v, b); }
-template <int N> CFD_HD bool operator>(const Dual<N>& a, double b) { return xlt(b, a.v); }
-template <int N> CFD_HD bool operator<=(const Dual<N>& a, double b) { return xle(a.v, b); }
+template <int N> CFD_HD bool operator<(const Dual<N>& a, double b) { return xlt_c(a.v, b); }
+template <int N> CFD_HD bool operator>(const Dual<N>& a, double b) { return xgt_c(a.v, b); }
+template <int N> CFD_HD bool operator<=(const Dual<N>& a, double b) { return xle_c(a.v, b); }
 template <int N> CFD_HD bool operator>=(const Dual<N>& a, double b) { return xle(b, a.v); }
-template <int N> CFD_HD bool operator<(double a, const Dual<N>& b) { return xlt(a, b.v); }
-template <int N> CFD_HD bool operator>(double a, const Dual<N>& b) { return xlt(b.v, a); }
+template <int N> CFD_HD bool operator<(double a, const Dual<N>& b) { return xgt_c(b.v, a); }
+template <int N> CFD_HD bool operator>(double a, const Dual<N>& b) { return xlt_c(b.v, a); }
+template <int N> CFD_HD bool lt_nonneg(const Dual<N>& a, const Dual<N>& b) { return xlt_nonneg(a.v, b.v); }
+template <int N> CFD_HD bool operator!=(const Dual<N>& a, double b) { return !xeq(a.v, b); }
 template <int N> CFD_HD bool operator==(const Dual<N>& a, const Dual<N>& b) { return xeq(a.v, b.v); }
 template <int N> CFD_HD bool operator!=(const Dual<N>& a, const Dual<N>& b) { return !xeq(a.v, b.v); }
 

@@ -56,13 +56,9 @@ __device__ __forceinline__ void edge_in_step(const StepArgs& a, const MemberDev&
                                              double t) {
   if (a.xd_cmp) {
     /* the same arithmetic with exact integer comparisons and, in the warps of xd_mul_mask,
-     * exact integer products: the FP64 pipe and the integer pipes share the work.  The WAF edge
-     * keys its comparisons on the plain bit patterns (faster there: 0.261 against 0.269 ms on the
-     * 1M step), the other schemes on the opaque ones (MUSCL edge 0.585 -> 0.534 ms, first-order
-     * HLLC forward ~4 % faster) */
-    constexpr bool OC = IFLUX != 3;
-    if ((a.xd_mul_mask >> ((e % TILE_E) >> 5)) & 1) edge_body<IFLUX, XD<true, OC>>(a, M, e, dt, t, S->surf);
-    else edge_body<IFLUX, XD<false, OC>>(a, M, e, dt, t, S->surf);
+     * exact integer products: the FP64 pipe and the integer pipes share the work.  */
+    if ((a.xd_mul_mask >> ((e % TILE_E) >> 5)) & 1) edge_body<IFLUX, XD<true>>(a, M, e, dt, t, S->surf);
+    else edge_body<IFLUX, XD<false>>(a, M, e, dt, t, S->surf);
   } else {
     edge_body<IFLUX>(a, M, e, dt, t, S->surf);
   }

@@ -110,6 +110,27 @@ CF_HD CF_INLINE T dmax(const T& a, const T& b) { return (a < b) ? b : a; } /* Fo
 template <class T>
 CF_HD CF_INLINE T dmin(const T& a, const T& b) { return (b < a) ? b : a; } /* Fortran min */
 
+template <class T>
+CF_HD CF_INLINE T dmax0(const T& x) { return dmax(T(0.0), x); }
+
+/* a < b where b is +0 or above and not NaN (the integer type has a shorter test for that) */
+template <class T>
+CF_HD CF_INLINE bool lt_nonneg(const T& a, const T& b) { return a < b; }
+
+/* Operations on an edge's constants (geometry, dt, g) in the arithmetic of the scalar type T: the
+ * quotient a / d given y = RN(1/d), x / 2 and 2 x, the same results for every T.  cf_xd.h keeps them
+ * off the FP64 pipe for its type. */
+template <class T>
+struct ConstOps {
+  static CF_HD CF_INLINE double quot(double a, double d, double y);
+  static CF_HD CF_INLINE double half(double x) { return x * 0.5; }
+  static CF_HD CF_INLINE double dbl(double x) { return x * 2.0; }
+};
+
+/* RN(1/d) of a denominator that several quotients share (div_rn) */
+template <class T>
+CF_HD CF_INLINE T recip(const T& d) { return 1.0 / d; }
+
 /* x / 2, x / 4 and 2 x.  A scaling by a power of two rounds once whichever way it is written, so
  * these give the bits of the quotient or product they stand for; the integer-product type (cf_xd.h)
  * overloads them with an exponent change. */
@@ -135,6 +156,9 @@ CF_HD CF_INLINE double div_rn(double a, double d, double y) {
   memcpy(&ab, &a, sizeof(ab));
   return zero_u(ab) ? q : q1;
 }
+
+template <class T>
+CF_HD CF_INLINE double ConstOps<T>::quot(double a, double d, double y) { return div_rn(a, d, y); }
 
 /* ---- x**(-1/3) -------------------------------------------------------------------------- */
 
@@ -254,9 +278,9 @@ CF_HD CF_INLINE bool wave_speeds(double g, double eps, T hl, T ul, T hr, T ur, T
   const T ar = sqrt(g * hr);
   const T het = halve(hl + hr) - quarter((ur - ul) * (hl + hr) / (al + ar));
   T pql, pqr;
-  if (het < hl) pql = T(1.);
+  if (lt_nonneg(het, hl)) pql = T(1.);
   else pql = (hl > eps) ? sqrt(halve(het + hl) * het / (hl * hl)) : T(0.);
-  if (het < hr) pqr = T(1.);
+  if (lt_nonneg(het, hr)) pqr = T(1.);
   else pqr = (hr > eps) ? sqrt(halve(het + hr) * het / (hr * hr)) : T(0.);
   if (hl > eps) {
     sl = ul - al * pql;
@@ -329,7 +353,7 @@ CF_HD CF_INLINE void first_order_flux(double g, double nx, double ny, T hl, T ul
     const int rb = (-sr > 0.) ? 1 : ((-sl < 0.) ? 0 : 2);
     T h1 = T(0.0), h2 = T(0.0);
     if (ra == 2 || rb == 2) {
-      const T den = sr - sl + eps, yden = 1.0 / den;
+      const T den = sr - sl + eps, yden = recip(den);
       h1 = div_rn(sr * fl1 - sl * fr1 + sl * sr * (hr - hl), den, yden);
       h2 = div_rn(sr * fl2 - sl * fr2 + sl * sr * (hr * ur - hl * ul), den, yden);
     }
@@ -440,7 +464,7 @@ CF_HD CF_INLINE void waf_flux(double g, int ilim, double nx, double ny, double d
   const int rb = (-sr > 0.) ? 1 : ((-sl < 0.) ? 0 : 2);
   T h1 = T(0.0), h2 = T(0.0);
   if (ra == 2 || rb == 2) {
-    const T den = sr - sl + eps, yden = 1.0 / den;
+    const T den = sr - sl + eps, yden = recip(den);
     h1 = div_rn(sr * fl1 - sl * fr1 + sl * sr * (hr - hl), den, yden);
     h2 = div_rn(sr * fl2 - sl * fr2 + sl * sr * (hr * ur - hl * ul), den, yden);
   }
@@ -449,7 +473,7 @@ CF_HD CF_INLINE void waf_flux(double g, int ilim, double nx, double ny, double d
   const T hb1 = (rb == 0) ? fl1 : ((rb == 1) ? fr1 : h1);
   const T hb2 = (rb == 0) ? fl2 : ((rb == 1) ? fr2 : h2);
 
-  const double dtoverdx = div_rn(dt, d_mrl, y_mrl);
+  const double dtoverdx = ConstOps<T>::quot(dt, d_mrl, y_mrl);
   const T cr = sr * dtoverdx, cl = sl * dtoverdx, cet = set * dtoverdx;
   const T dloc = div_rn(hr - hl, d_mrl, y_mrl);          /* delta_loc_l = delta_loc_r */
   const T dloc_et = div_rn(vr - vl, d_mrl, y_mrl);
@@ -461,7 +485,7 @@ CF_HD CF_INLINE void waf_flux(double g, int ilim, double nx, double ny, double d
 
   /* side A (:854-899) */
   {
-    const T den = dloc + eps, yd = 1.0 / den;
+    const T den = dloc + eps, yd = recip(den);
     const T rl = held(div_rn((sl > 0.) ? upl : upr, den, yd), freeze_r);
     const T rr = held(div_rn((sr > 0.) ? upl : upr, den, yd), freeze_r);
     const T ll = waf_limiter(ilim, rl, cl);
@@ -483,7 +507,7 @@ CF_HD CF_INLINE void waf_flux(double g, int ilim, double nx, double ny, double d
    * (hl - hr)/d = -dloc, its upwind differences are minus A's (for the wave it tests), the
    * tangential ones coincide; its Courant numbers are -cr, -cl, -cet. */
   {
-    const T den = -dloc + eps, yd = 1.0 / den;
+    const T den = -dloc + eps, yd = recip(den);
     const T rl = held(div_rn((-sr > 0.) ? -upr : -upl, den, yd), freeze_r);
     const T rr = held(div_rn((-sl > 0.) ? -upr : -upl, den, yd), freeze_r);
     /* B's tangential ratio differs from A's only when s* == 0 (or is NaN) */
@@ -543,8 +567,8 @@ CF_HD CF_INLINE void muscl_side(double g, double tolisec, int ilim, double dtove
   const T dloc2 = div_rn(ur - ul, d_mrl, y_mrl);
   const T dloc3 = div_rn(vr - vl, d_mrl, y_mrl);
   const T dhl = simple_limiter(ilim, div_rn(hl - hl_upw, d_up_l, y_up_l), dloc1);
-  const T hll = dmax(T(0.), hl - halve(dhl) * d_mrl);
-  const T hlr = dmax(T(0.), hl + halve(dhl) * d_mrl);
+  const T hll = dmax0(hl - halve(dhl) * d_mrl);
+  const T hlr = dmax0(hl + halve(dhl) * d_mrl);
   T ull, vll, ulr, vlr;
   if (hlr < tolisec || hll < tolisec) {
     ulr = vlr = ull = vll = T(0.);
@@ -557,8 +581,8 @@ CF_HD CF_INLINE void muscl_side(double g, double tolisec, int ilim, double dtove
     vlr = vl + halve(dvl) * d_mrl;
   }
   const T dhr = simple_limiter(ilim, dloc1, div_rn(hr_upw - hr, d_up_r, y_up_r));
-  const T hrr = dmax(T(0.), hr + halve(dhr) * d_mrl);
-  const T hrl = dmax(T(0.), hr - halve(dhr) * d_mrl);
+  const T hrr = dmax0(hr + halve(dhr) * d_mrl);
+  const T hrl = dmax0(hr - halve(dhr) * d_mrl);
   T url, vrl, urr, vrr;
   if (hrl < tolisec || hrr < tolisec) {
     url = vrl = urr = vrr = T(0.);
@@ -571,14 +595,15 @@ CF_HD CF_INLINE void muscl_side(double g, double tolisec, int ilim, double dtove
     vrl = vr - halve(dvr) * d_mrl;
   }
   /* data reconstruction II (:615-621) */
-  const T h1 = hlr + 0.5 * dtoverdx * (hll * ull - hlr * ulr);
-  const T u1 = ulr + 0.5 * dtoverdx *
-                         (hll * (ull * ull) + 0.5 * g * (hll * hll) - (hlr * (ulr * ulr) + 0.5 * g * (hlr * hlr)));
-  const T v1 = vlr + 0.5 * dtoverdx * (hll * ull * vll - hlr * ulr * vlr);
-  const T h2 = hrl + 0.5 * dtoverdx * (hrl * url - hrr * urr);
-  const T u2 = url + 0.5 * dtoverdx *
-                         (hrl * (url * url) + 0.5 * g * (hrl * hrl) - (hrr * (urr * urr) + 0.5 * g * (hrr * hrr)));
-  const T v2 = vrl + 0.5 * dtoverdx * (hrl * url * vrl - hrr * urr * vrr);
+  const double hdt = ConstOps<T>::half(dtoverdx), hg = ConstOps<T>::half(g);
+  const T h1 = hlr + hdt * (hll * ull - hlr * ulr);
+  const T u1 = ulr + hdt *
+                         (hll * (ull * ull) + hg * (hll * hll) - (hlr * (ulr * ulr) + hg * (hlr * hlr)));
+  const T v1 = vlr + hdt * (hll * ull * vll - hlr * ulr * vlr);
+  const T h2 = hrl + hdt * (hrl * url - hrr * urr);
+  const T u2 = url + hdt *
+                         (hrl * (url * url) + hg * (hrl * hrl) - (hrr * (urr * urr) + hg * (hrr * hrr)));
+  const T v2 = vrl + hdt * (hrl * url * vrl - hrr * urr * vrr);
   /* HLLC (:623-714) */
   T sl, sr, set;
   if (!wave_speeds(g, eps, h1, u1, h2, u2, sl, sr, set)) {
@@ -596,7 +621,7 @@ CF_HD CF_INLINE void muscl_side(double g, double tolisec, int ilim, double dtove
   } else {
     const T fl1 = h1 * u1, fl2 = h1 * (u1 * u1) + halve(g * h1 * h1);
     const T fr1 = h2 * u2, fr2 = h2 * (u2 * u2) + halve(g * h2 * h2);
-    const T den = sr - sl + eps, yden = 1.0 / den;
+    const T den = sr - sl + eps, yden = recip(den);
     x1 = div_rn(sr * fl1 - sl * fr1 + sl * sr * (h2 - h1), den, yden);
     x2 = div_rn(sr * fl2 - sl * fr2 + sl * sr * (h2 * u2 - h1 * u1), den, yden);
     x3 = (set > 0.) ? x1 * v1 : x1 * v2;
@@ -665,8 +690,8 @@ CF_HD CF_INLINE void boundary_flux(int iflux, const MemberDev& M, int kind, int 
        * right (:173-181); second-order schemes use first-order HLLC here (their centroid
        * distance to themselves is zero). */
       const double zij = dmax(z, z);
-      T hsl = dmax(T(0.0), hautl + z - zij);
-      T hsr = dmax(T(0.0), ((iflux <= 2) ? h : hautl) + z - zij);
+      T hsl = dmax0(hautl + z - zij);
+      T hsr = dmax0(((iflux <= 2) ? h : hautl) + z - zij);
       T ul = vitul, vl = vitvl, ur = vitul, vr = vitvl;
       if (hsl < tolisec) { hsl = T(0.); ul = T(0.); vl = T(0.); }
       if (hsr < tolisec) { hsr = T(0.); ur = T(0.); vr = T(0.); }
@@ -683,7 +708,8 @@ CF_HD CF_INLINE void boundary_flux(int iflux, const MemberDev& M, int kind, int 
  * element, or the first-order fallback), else the centroid-distance weighted average of two. */
 template <class T>
 CF_HD CF_INLINE void upwind_mix(T h1, T hu1, T hv1, double yh1, T h2, T hu2, T hv2, double yh2, double d1,
-                                double d2, double ysum, double nx, double ny, double tolisec, T& hu_, T& vu_) {
+                                double d2, double ds, double ysum, double nx, double ny, double tolisec, T& hu_,
+                                T& vu_) {
   T a, va;
   to_frame_t(h1, hu1, hv1, yh1, nx, ny, tolisec, a, va);
   if (T(d1) < 0.0) {
@@ -693,9 +719,13 @@ CF_HD CF_INLINE void upwind_mix(T h1, T hu1, T hv1, double yh1, T h2, T hu2, T h
   }
   T b, vb;
   to_frame_t(h2, hu2, hv2, yh2, nx, ny, tolisec, b, vb);
-  const double ds = d1 + d2;
   hu_ = div_rn(d1 * a + d2 * b, ds, ysum);
   vu_ = div_rn(d1 * va + d2 * vb, ds, ysum);
+}
+template <class T>
+CF_HD CF_INLINE void upwind_mix(T h1, T hu1, T hv1, double yh1, T h2, T hu2, T hv2, double yh2, double d1,
+                                double d2, double ysum, double nx, double ny, double tolisec, T& hu_, T& vu_) {
+  upwind_mix(h1, hu1, hv1, yh1, h2, hu2, hv2, yh2, d1, d2, d1 + d2, ysum, nx, ny, tolisec, hu_, vu_);
 }
 
 /* The bed elevation of an upwind reconstruction (flux_riemann.cuf:320-366): static, so the host
@@ -704,26 +734,27 @@ CF_HD CF_INLINE double upwind_bed(double z1, double z2, double d1, double d2, do
   return (d1 < 0.0) ? z1 : div_rn(d1 * z1 + d2 * z2, d1 + d2, ysum);
 }
 
-/* The same, loading the elements' states (w = RN(1/h)), in the edge's arithmetic type T. */
+/* The same, loading the elements' states (w = RN(1/h)), in the edge's arithmetic type T; ds = d1 + d2
+ * of a pair (twice its d_mkvol, which the preprocessing forms as (d1 + d2) / 2). */
 template <class T>
-CF_HD CF_INLINE void upwind_state(const double4* U, int i1, int i2, double d1, double d2, double ysum, double nx,
-                                  double ny, double tolisec, T& hu_, T& vu_) {
+CF_HD CF_INLINE void upwind_state(const double4* U, int i1, int i2, double d1, double d2, double ds, double ysum,
+                                  double nx, double ny, double tolisec, T& hu_, T& vu_) {
   const double4 A1 = ld4(U + i1);
   if (T(d1) < 0.0) {
-    upwind_mix(T(A1.x), T(A1.y), T(A1.z), A1.w, T(0.0), T(0.0), T(0.0), 0.0, d1, d2, ysum, nx, ny, tolisec, hu_,
-               vu_);
+    upwind_mix(T(A1.x), T(A1.y), T(A1.z), A1.w, T(0.0), T(0.0), T(0.0), 0.0, d1, d2, ds, ysum, nx, ny, tolisec,
+               hu_, vu_);
     return;
   }
   const double4 A2 = ld4(U + i2);
-  upwind_mix(T(A1.x), T(A1.y), T(A1.z), A1.w, T(A2.x), T(A2.y), T(A2.z), A2.w, d1, d2, ysum, nx, ny, tolisec, hu_,
-             vu_);
+  upwind_mix(T(A1.x), T(A1.y), T(A1.z), A1.w, T(A2.x), T(A2.y), T(A2.z), A2.w, d1, d2, ds, ysum, nx, ny, tolisec,
+             hu_, vu_);
 }
 
 /* The MUSCL form: (h, u_n, u_t) of one side's upwind reconstruction (flux_riemann.cuf:240-366
  * with the normal velocity as well). */
 template <class T>
-CF_HD CF_INLINE void upwind_state3(const double4* U, int i1, int i2, double d1, double d2, double ysum, double nx,
-                                   double ny, double tolisec, T& hu_, T& uu_, T& vu_) {
+CF_HD CF_INLINE void upwind_state3(const double4* U, int i1, int i2, double d1, double d2, double ds, double ysum,
+                                   double nx, double ny, double tolisec, T& hu_, T& uu_, T& vu_) {
   const double4 A1 = ld4(U + i1);
   T a, ua, va;
   to_frame(T(A1.x), T(A1.y), T(A1.z), A1.w, nx, ny, tolisec, a, ua, va);
@@ -736,7 +767,6 @@ CF_HD CF_INLINE void upwind_state3(const double4* U, int i1, int i2, double d1, 
   const double4 A2 = ld4(U + i2);
   T b, ub, vb;
   to_frame(T(A2.x), T(A2.y), T(A2.z), A2.w, nx, ny, tolisec, b, ub, vb);
-  const double ds = d1 + d2;
   hu_ = div_rn(d1 * a + d2 * b, ds, ysum);
   uu_ = div_rn(d1 * ua + d2 * ub, ds, ysum);
   vu_ = div_rn(d1 * va + d2 * vb, ds, ysum);
@@ -766,19 +796,24 @@ CF_HD CF_INLINE void interior_edge(const MemberDev& M, int ilim, int flux_mode, 
   T hautl, vitul, vitvl, hautr, vitur, vitvr;
   to_frame(hA, huA, hvA, yhA, nx, ny, tolisec, hautl, vitul, vitvl);
   to_frame(hB, huB, hvB, yhB, nx, ny, tolisec, hautr, vitur, vitvr);
+  /* the depths above the higher bed, of the raw depths (the bed source's, and the reconstruction of a
+   * wet side).  A masked depth of 0 reconstructs to +0 on any bed: z - max(z, z') is not positive, or
+   * NaN, and the max with 0 gives +0. */
+  const bool wetA = hA > tolisec, wetB = hB > tolisec;
+  const T ha = dmax0(hA + zml - zij), hb = dmax0(hB + zmr - zij);
   TwoFluxT<T> F;
   if (IFLUX <= 2) {
     /* hydrostatic reconstruction (:176-181, :200-210): A from its masked depth, B from its
      * raw depth; the raw and masked depths differ only for 0 < h <= tolisec, where side B's
      * own evaluation (B masked, A raw) is computed separately. */
-    T hijet = dmax(T(0.0), hautl + zml - zij);
-    T hjiet = dmax(T(0.0), hB + zmr - zij);
+    T hijet = wetA ? ha : T(0.0);
+    T hjiet = hb;
     T ul = vitul, vl = vitvl, ur = vitur, vr = vitvr;
     if (hijet < tolisec) { hijet = T(0.); ul = T(0.); vl = T(0.); }
     if (hjiet < tolisec) { hjiet = T(0.); ur = T(0.); vr = T(0.); }
     first_order_flux<IFLUX>(g, nx, ny, hijet, ul, vl, hjiet, ur, vr, F);
-    if (hautl != hA || hautr != hB) {
-      T bl = dmax(T(0.0), hautr + zmr - zij), br = dmax(T(0.0), hA + zml - zij);
+    if ((!wetA && hA != 0.0) || (!wetB && hB != 0.0)) {   /* a side's masked depth differs from its raw one */
+      T bl = wetB ? hb : T(0.0), br = ha;
       T bul = -vitur, bvl = -vitvr, bur = -vitul, bvr = -vitvl;
       if (bl < tolisec) { bl = T(0.); bul = T(0.); bvl = T(0.); }
       if (br < tolisec) { br = T(0.); bur = T(0.); bvr = T(0.); }
@@ -790,10 +825,10 @@ CF_HD CF_INLINE void interior_edge(const MemberDev& M, int ilim, int flux_mode, 
     }
   } else {
     /* hydrostatic reconstruction of the four states (:370-400) */
-    T hijet = dmax(T(0.0), hautl + zml - zij);
-    T hlu = dmax(T(0.0), hl_upw + zl_upw - zij);
-    T hjiet = dmax(T(0.0), hautr + zmr - zij);
-    T hru = dmax(T(0.0), hr_upw + zr_upw - zij);
+    T hijet = wetA ? ha : T(0.0);
+    T hlu = dmax0(hl_upw + zl_upw - zij);
+    T hjiet = wetB ? hb : T(0.0);
+    T hru = dmax0(hr_upw + zr_upw - zij);
     T ul = vitul, vl = vitvl, ur = vitur, vr = vitvr, vlu = vl_upw, vru = vr_upw;
     if (hijet < tolisec) { hijet = T(0.); ul = T(0.); vl = T(0.); }
     if (hlu < tolisec) { hlu = T(0.); vlu = T(0.); }
@@ -808,10 +843,9 @@ CF_HD CF_INLINE void interior_edge(const MemberDev& M, int ilim, int flux_mode, 
     F.b3 = -F.a3;
   }
   /* bed-slope source of both sides from the raw depths (source_terms.cuf:90-97) */
-  const T ha = dmax(T(0.0), hA + zml - zij);
-  const T hb = dmax(T(0.0), hB + zmr - zij);
-  const T ta = g / 2.0 * (ha * ha - hA * hA) * len;
-  const T tb = g / 2.0 * (hb * hb - hB * hB) * len;
+  const double hg = ConstOps<T>::half(g);
+  const T ta = hg * (ha * ha - hA * hA) * len;
+  const T tb = hg * (hb * hb - hB * hB) * len;
   out[0] = F.a1 * len;
   out[1] = F.a2 * len;
   out[2] = F.a3 * len;
@@ -841,18 +875,20 @@ CF_HD CF_INLINE void interior_edge_muscl(const MemberDev& M, int ilim, int flux_
   T hautl, vitul, vitvl, hautr, vitur, vitvr;
   to_frame(hA, huA, hvA, yhA, nx, ny, tolisec, hautl, vitul, vitvl);
   to_frame(hB, huB, hvB, yhB, nx, ny, tolisec, hautr, vitur, vitvr);
-  /* hydrostatic reconstruction of the four states (:370-400) */
-  T hijet = dmax(T(0.0), hautl + zml - zij);
-  T hlu = dmax(T(0.0), upA[0] + zl_upw - zij);
-  T hjiet = dmax(T(0.0), hautr + zmr - zij);
-  T hru = dmax(T(0.0), upB[0] + zr_upw - zij);
+  /* hydrostatic reconstruction of the four states (:370-400); a masked depth reconstructs to +0 (see
+   * interior_edge) */
+  const T ha = dmax0(hA + zml - zij), hb = dmax0(hB + zmr - zij);
+  T hijet = hA > tolisec ? ha : T(0.0);
+  T hlu = dmax0(upA[0] + zl_upw - zij);
+  T hjiet = hB > tolisec ? hb : T(0.0);
+  T hru = dmax0(upB[0] + zr_upw - zij);
   T ul = vitul, vl = vitvl, ur = vitur, vr = vitvr;
   T ulu = upA[1], vlu = upA[2], uru = upB[1], vru = upB[2];
   if (hijet < tolisec) { hijet = T(0.); ul = T(0.); vl = T(0.); }
   if (hlu < tolisec) { hlu = T(0.); ulu = T(0.); vlu = T(0.); }
   if (hjiet < tolisec) { hjiet = T(0.); ur = T(0.); vr = T(0.); }
   if (hru < tolisec) { hru = T(0.); uru = T(0.); vru = T(0.); }
-  const double dtoverdx = div_rn(dt, G.d_mrl, G.y_mrl);
+  const double dtoverdx = ConstOps<T>::quot(dt, G.d_mrl, G.y_mrl);
   TwoFluxT<T> F;
   T x1, x2, x3;
   muscl_side(g, tolisec, ilim, dtoverdx, G.d_mrl, G.y_mrl, G.d_mkvol, G.y_mkvol, G.d_mkvoisin, G.y_mkvoisin, hijet,
@@ -874,10 +910,9 @@ CF_HD CF_INLINE void interior_edge_muscl(const MemberDev& M, int ilim, int flux_
     F.b3 = my * y2 + mx * y3;
   }
   /* bed-slope source of both sides from the raw depths (source_terms.cuf:90-97) */
-  const T ha = dmax(T(0.0), hA + zml - zij);
-  const T hb = dmax(T(0.0), hB + zmr - zij);
-  const T ta = g / 2.0 * (ha * ha - hA * hA) * len;
-  const T tb = g / 2.0 * (hb * hb - hB * hB) * len;
+  const double hg = ConstOps<T>::half(g);
+  const T ta = hg * (ha * ha - hA * hA) * len;
+  const T tb = hg * (hb * hb - hB * hB) * len;
   out[0] = F.a1 * len;
   out[1] = F.a2 * len;
   out[2] = F.a3 * len;
@@ -1086,8 +1121,8 @@ CF_HD CF_INLINE void edge_body(const StepArgs& a, const MemberDev& M, int e, dou
     const int4 up = ldro(a.eupw + e);
     const double4 dw = ld4(a.ewts + e);
     S upA[3], upB[3], om[10];
-    upwind_state3(a.Uin, up.x, up.y, dw.x, dw.y, G.ysum_a, G.nx, G.ny, M.tolisec, upA[0], upA[1], upA[2]);
-    upwind_state3(a.Uin, up.z, up.w, dw.z, dw.w, G.ysum_b, G.nx, G.ny, M.tolisec, upB[0], upB[1], upB[2]);
+    upwind_state3(a.Uin, up.x, up.y, dw.x, dw.y, ConstOps<S>::dbl(G.d_mkvol), G.ysum_a, G.nx, G.ny, M.tolisec, upA[0], upA[1], upA[2]);
+    upwind_state3(a.Uin, up.z, up.w, dw.z, dw.w, ConstOps<S>::dbl(G.d_mkvoisin), G.ysum_b, G.nx, G.ny, M.tolisec, upB[0], upB[1], upB[2]);
     interior_edge_muscl(M, a.ilimiteur, a.flux_mode, G, dt, S(UA.x), S(UA.y), S(UA.z), ez.x, UA.w, S(UB.x), S(UB.y),
                         S(UB.z), ez.y, UB.w, upA, ez.z, upB, ez.w, om);
 #pragma unroll
@@ -1099,8 +1134,8 @@ CF_HD CF_INLINE void edge_body(const StepArgs& a, const MemberDev& M, int e, dou
   if (IFLUX == 3) {
     const int4 up = ldro(a.eupw + e);
     const double4 dw = ld4(a.ewts + e);   /* d1, d2 of side A, d1, d2 of side B */
-    upwind_state(a.Uin, up.x, up.y, dw.x, dw.y, G.ysum_a, G.nx, G.ny, M.tolisec, hl_upw, vl_upw);
-    upwind_state(a.Uin, up.z, up.w, dw.z, dw.w, G.ysum_b, G.nx, G.ny, M.tolisec, hr_upw, vr_upw);
+    upwind_state(a.Uin, up.x, up.y, dw.x, dw.y, ConstOps<S>::dbl(G.d_mkvol), G.ysum_a, G.nx, G.ny, M.tolisec, hl_upw, vl_upw);
+    upwind_state(a.Uin, up.z, up.w, dw.z, dw.w, ConstOps<S>::dbl(G.d_mkvoisin), G.ysum_b, G.nx, G.ny, M.tolisec, hr_upw, vr_upw);
   }
   S os[10];
   interior_edge<(IFLUX == 4 ? 3 : IFLUX)>(M, a.ilimiteur, a.flux_mode, G, dt, S(UA.x), S(UA.y), S(UA.z), ez.x,
@@ -1148,7 +1183,7 @@ CF_HD CF_INLINE void friction_terms(const MemberDev& M, double area, double dt, 
     if (normvit > tol) {
       const T p43 = div_rn(p13, q1, yq);     /* q1**(-4/3) */
       if (M.fricimplic == 1) {
-        const T yn = 1.0 / normvit;
+        const T yn = recip(normvit);
         const T dtgn2h = dt / 2.0 * gp * manning * manning * p43;
         const T af21 = -(7.0 / 3.0 * dtgn2h * vitu * normvit);
         const T af22 = 1.0 + div_rn(dtgn2h * (twice(vitu * vitu) + vitv * vitv), normvit, yn);
@@ -1157,7 +1192,7 @@ CF_HD CF_INLINE void friction_terms(const MemberDev& M, double area, double dt, 
         const T af32 = af23;
         const T af33 = 1.0 + div_rn(dtgn2h * (vitu * vitu + twice(vitv * vitv)), normvit, yn);
         const T detaf = af22 * af33 - af23 * af32;
-        const T yd = 1.0 / detaf;
+        const T yd = recip(detaf);
         m[0] = div_rn(-(af21 * af33 - af23 * af31), detaf, yd);
         m[1] = div_rn(af33, detaf, yd);
         m[2] = div_rn(-af23, detaf, yd);

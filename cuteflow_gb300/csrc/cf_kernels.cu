@@ -578,9 +578,12 @@ __global__ void __launch_bounds__(256) k_selftest_xd(long long n, unsigned long 
     nbad += !st_same(em_div(a, b), a / b);
     nbad += !st_same(xscale<-2>(a), a * 0.25) + !st_same(xscale<-1>(a), a * 0.5) + !st_same(xscale<1>(a), a * 2.0);
     nbad += !st_same(val(-XD<true>(a)), -a);
-    /* the key comparisons on opaque and on plain bit patterns */
+    /* the comparisons: of any two values, and against constants and depths */
     nbad += (xlt(a, b) != (a < b)) + (xle(a, b) != (a <= b)) + (xeq(a, b) != (a == b));
-    nbad += (xlt<false>(a, b) != (a < b)) + (xle<false>(a, b) != (a <= b)) + (xeq<false>(a, b) != (a == b));
+    nbad += (xlt_c(a, b) != (a < b)) + (xgt_c(a, b) != (a > b)) + (xle_c(a, b) != (a <= b));
+    nbad += (xlt_c(a, 0.0) != (a < 0.0)) + (xgt_c(a, 0.0) != (a > 0.0)) + (xle_c(a, 0.0) != (a <= 0.0));
+    nbad += (xlt_c(a, 1.0) != (a < 1.0)) + (xgt_c(a, 0.5) != (a > 0.5)) + (xle_c(a, 2.0) != (a <= 2.0));
+    nbad += (b >= 0.0 && xlt_nonneg(a, fabs(b)) != (a < b));
   }
   if (nbad) atomicAdd(bad, nbad);
 }

@@ -1,28 +1,34 @@
 /*
  * cf_xd.h -- binary64 arithmetic that keeps GB300's FP64 pipe for the operations only it can do.
  *
- * GB300 issues two FP64 operations per clock per SM; its integer pipes issue ~30x more 32-bit
- * operations, run beside the FP64 pipe, and sit idle in an all-FP64 step (ncu: FP64 pipe 85 %
- * busy, ALU 1.4 %).  Exact substitutions move FP64-pipe work onto them:
+ * GB300 issues one FP64 instruction per warp and SM sub-partition in 76 cycles (16 when it reads one
+ * register pair fewer; 5.0e11/s on 152 SMs), a 32-bit integer one in 2 (shifts, logic, additions,
+ * IMAD; 64 lanes per clock and SM on each of two pipes) and a 32 x 32 -> 64 multiply-add in 4, beside
+ * the FP64 pipe.  So integer sequences of up to ~40 instructions that give the IEEE result exactly
+ * replace FP64 instructions at a profit:
  *
- *   comparisons  x < y etc. on ordered integer keys of the bit patterns (negative values
- *                mirrored, -0 and +0 one key, NaN compares false): the IEEE result, on the ALU;
- *   products     x * y by integer multiplication of the significands with round to nearest
- *                even (em_mul);
- *   quotients    a / b from a float reciprocal seed, a fixed-point refinement and the exact
- *                remainder, which decides the rounding (em_div);
- *   roots        sqrt(x) the same way from a float reciprocal-root seed (em_sqrt);
- *   scalings     x / 2, x / 4, 2 x and negation as exponent-field and sign-bit operations.
+ *   comparisons  on the words of the patterns (-0 = +0, NaN compares false), 4 to 6 instructions
+ *                against a constant;
+ *   products     x * y by four 32-bit multiply-adds of the significands (em_mul, 28);
+ *   quotients    a / b by a two-digit long division with a float reciprocal seed (em_div, 44);
+ *   roots        sqrt(x) by a two-digit root extraction the same way (em_sqrt, 45);
+ *   scalings     x / 2, x / 4, 2 x, negation, |x| and sign transfers as operations on the high word.
  * Each takes the FP64 instruction (out of line, so that the compiler does not evaluate it
- * speculatively on the fast path) wherever the integer path does not cover the case: a zero,
- * subnormal, infinite or NaN operand (a zero numerator of em_div is covered), a result outside
- * the normal range, and, for em_div and em_sqrt, a remainder check that fails.
+ * speculatively on the fast path) wherever the integer path does not cover the case: exponents
+ * outside the window of xwindow (zero operands of a product and zero numerators are covered), a tie
+ * of a product, subnormal, infinite and NaN operands.
  *
- * XD<MUL, OC> is a double that compares on integer keys and, with MUL, multiplies, divides (div_rn
+ * XD<MUL> is a double that compares on integers and, with MUL, multiplies, divides (div_rn
  * included) and takes square roots with em_mul, em_div and em_sqrt; sums stay FP64
  * instructions.  Every result is the IEEE binary64 result of the same operation, so code
  * instantiated on XD<...> rounds exactly like the same code on double; which warps use the
  * integer arithmetic is a tuning choice, not a numerical one.
+ *
+ * Products are expanded in place, quotients and roots called: the product's 28 instructions are
+ * little more than a call of them costs, and the rest of an edge's straight-line code has to stay in
+ * the instruction cache (dam break of 134k triangles, first-order HLLC: 109 us per step before these
+ * sequences, 83 with every one called, 76 as it is, 74 with all in place; flood of 201k triangles,
+ * WAF: 246, 315, 186, 189).
  */
 #ifndef CF_XD_H
 #define CF_XD_H
@@ -36,6 +42,9 @@
 #define XD_HD inline
 #define XD_NOINLINE static __attribute__((noinline))
 #endif
+#define XD_FN_MUL XD_HD
+#define XD_FN_DIV XD_NOINLINE
+#define XD_FN_SQRT XD_NOINLINE
 
 namespace cf {
 
@@ -53,233 +62,312 @@ XD_HD double xdbl(uint64_t b) {
   return x;
 }
 
-XD_HD uint64_t xmulhi(uint64_t a, uint64_t b) {
+/* The 32-bit words of a double and back.  On the device opaque register moves: the bit operations
+ * then work on the registers of the value as they are, and the compiler neither turns them into FP64
+ * instructions nor forms an FP64 sum a second time for its bits. */
+XD_HD void xwords(double x, uint32_t& lo, uint32_t& hi) {
 #ifdef __CUDA_ARCH__
-  return __umul64hi(a, b);
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "d"(x));
 #else
-  return (uint64_t)(((unsigned __int128)a * b) >> 64);
+  const uint64_t b = xbits(x);
+  lo = (uint32_t)b;
+  hi = (uint32_t)(b >> 32);
 #endif
 }
-
-/* the FP64 instruction, for the operands and results the integer path does not cover */
-XD_NOINLINE double xmul_slow(double a, double b) { return a * b; }
-
-/* a * b, round to nearest even, in integer arithmetic (normal operands, normal result).  Out of
- * line: the edge kernel makes ~60 products per edge, and inlining each one multiplies the size of
- * a kernel whose instruction working set is already large (measured: WAF edge kernel 0.609 ms
- * inlined, 0.545 ms called, 1M triangles). */
-XD_NOINLINE double em_mul(double a, double b) {
-  const uint64_t ua = xbits(a), ub = xbits(b);
-  const uint32_t ea = (uint32_t)(ua >> 52) & 0x7ffu, eb = (uint32_t)(ub >> 52) & 0x7ffu;
-  if (ea - 1u >= 2046u || eb - 1u >= 2046u) return xmul_slow(a, b);
-  const uint64_t M = (1ull << 52) - 1;
-  const uint64_t ma = ((ua & M) | (1ull << 52)) << 11, mb = ((ub & M) | (1ull << 52)) << 1;
-  const uint64_t hi = xmulhi(ma, mb);  /* the product's bits from 2^52 up: 53 or 54 bits */
-  const uint64_t lo = ma * mb;         /* the product's bits below 2^52, shifted left by 12 */
-  const uint32_t top = (uint32_t)(hi >> 53);
-  const int e = (int)ea + (int)eb - 1023 + (int)top;
-  uint64_t mant = hi >> top;
-  const uint64_t rb = top ? (hi & 1u) : (lo >> 63);
-  const uint64_t sticky = top ? (lo != 0) : ((lo << 1) != 0);
-  mant += rb & (sticky | (mant & 1u));
-  if ((uint32_t)(e - 1) >= 2046u) return xmul_slow(a, b);
-  return xdbl((((uint64_t)(e - 1) << 52) + mant) | ((ua ^ ub) & (1ull << 63)));
+XD_HD double xjoin(uint32_t lo, uint32_t hi) {
+#ifdef __CUDA_ARCH__
+  double x;
+  asm("mov.b64 %0, {%1, %2};" : "=d"(x) : "r"(lo), "r"(hi));
+  return x;
+#else
+  return xdbl(((uint64_t)hi << 32) | lo);
+#endif
+}
+XD_HD uint32_t xmulhi32(uint32_t a, uint32_t b) {
+#ifdef __CUDA_ARCH__
+  return __umulhi(a, b);
+#else
+  return (uint32_t)(((uint64_t)a * b) >> 32);
+#endif
+}
+/* words (lo, hi) shifted left (right) by n in 0..31: the high (low) word of the result */
+XD_HD uint32_t xshl(uint32_t lo, uint32_t hi, uint32_t n) {
+#ifdef __CUDA_ARCH__
+  return __funnelshift_l(lo, hi, n);
+#else
+  return (uint32_t)(((((uint64_t)hi << 32) | lo) << n) >> 32);
+#endif
+}
+XD_HD uint32_t xshr(uint32_t lo, uint32_t hi, uint32_t n) {
+#ifdef __CUDA_ARCH__
+  return __funnelshift_r(lo, hi, n);
+#else
+  return (uint32_t)((((uint64_t)hi << 32) | lo) >> n);
+#endif
+}
+/* (hi, lo) + bit 31 of r + (e << 32): the rounding increment and the exponent and sign word join the
+ * significand in one carry chain */
+XD_HD double xround(uint32_t lo, uint32_t hi, uint32_t r, uint32_t e) {
+#ifdef __CUDA_ARCH__
+  uint32_t t, l, h;
+  asm("add.cc.u32 %0, %3, %3;\n\taddc.cc.u32 %1, %4, 0;\n\taddc.u32 %2, %5, %6;"
+      : "=r"(t), "=r"(l), "=r"(h) : "r"(r), "r"(lo), "r"(hi), "r"(e));
+  (void)t;
+  return xjoin(l, h);
+#else
+  const uint64_t s = ((((uint64_t)hi << 32) | lo) + (r >> 31)) + ((uint64_t)e << 32);
+  return xdbl(s);
+#endif
+}
+/* both high words have exponent fields in [767, 1278] (2^-256 .. 2^256): the window in which products
+ * and quotients are normal numbers whatever the significands */
+XD_HD bool xwindow(uint32_t ah, uint32_t bh) {
+  const uint32_t k = 0u - (767u << 21);
+  return (((ah * 2u + k) | (bh * 2u + k)) & 0xc0000000u) == 0;
 }
 
-/* the FP64 quotient, for the operands and results the integer path does not cover */
-XD_NOINLINE double xdiv_slow(double a, double b) { return a / b; }
+/* the FP64 instruction, for the operands and results the integer path does not cover (out of line, so
+ * that it is not evaluated speculatively on the fast path) */
+XD_NOINLINE double xmul_slow(double a, double b) { return a * b; }
 
-/* bits of an approximation to 1/f, f in [1, 2): on the device the single-precision reciprocal
+/* a * b, round to nearest even, in integer arithmetic.  The 53-bit significands are multiplied as
+ * 21 + 32 bit words: four 32 x 32 -> 64 multiply-adds without a carry between them (the middle sum
+ * stays below 2^55).  With the product in [2^104, 2^106), top tells its length; the result is its
+ * leading 53 bits plus the next one (round half up; a tie, where the bits after that one are all zero,
+ * goes to the FP64 instruction with the operands outside the window). */
+XD_FN_MUL double em_mul(double a, double b) {
+  uint32_t al, ah, bl, bh;
+  xwords(a, al, ah);
+  xwords(b, bl, bh);
+  const uint32_t ma = (ah & 0xfffffu) | 0x100000u, mb = (bh & 0xfffffu) | 0x100000u;
+  const uint64_t p = (uint64_t)al * bl;
+  uint64_t m = (uint64_t)ma * bl + (p >> 32);
+  m = (uint64_t)al * mb + m;
+  const uint64_t v = (uint64_t)ma * mb + (m >> 32);
+  const uint32_t w0 = (uint32_t)m, w1 = (uint32_t)v, w2 = (uint32_t)(v >> 32);
+  const uint32_t top = w2 >> 9;                       /* 1: the product is at least 2^105 */
+  const uint32_t rest = w0 << (12u - top);            /* the bits after the 53rd, round bit first */
+  const uint32_t e = (ah - ma) + (bh - mb) + (top << 20) - (1022u << 20);
+  if (!xwindow(ah, bh) || ((rest ^ 0x80000000u) | (uint32_t)p) == 0) {
+    /* a signed zero for a zero and a finite operand */
+    if (((((ah << 1) | al) == 0) | (((bh << 1) | bl) == 0)) & ((~ah & 0x7ff00000u) != 0) & ((~bh & 0x7ff00000u) != 0))
+      return xjoin(0u, (ah ^ bh) & 0x80000000u);
+    return xmul_slow(a, b);
+  }
+  return xround(xshr(w0, w1, 20u + top), xshr(w1, w2, 20u + top), rest, e);
+}
+
+/* Quotients outside the integer path: a signed zero for a zero over a normal number, else FP64 */
+XD_NOINLINE double xdiv_slow(double a, double b) {
+  uint32_t al, ah, bl, bh;
+  xwords(a, al, ah);
+  xwords(b, bl, bh);
+  if (((ah << 1) | al) == 0 && ((bh >> 20) & 0x7ffu) - 1u < 2046u) return xjoin(0u, (ah ^ bh) & 0x80000000u);
+  return a / b;
+}
+
+/* bits of an approximation to 1/f, f in (1, 2]: on the device the single-precision reciprocal
  * (rcp.approx.ftz.f32, error at most one unit in the last place); on the host the IEEE float
  * quotient moved by -1, 0 or +1 unit, so host runs exercise the device's error bound */
-XD_HD uint32_t xrcp_seed(float f, uint64_t salt) {
+XD_HD uint32_t xrcp_seed(uint32_t fb, uint32_t salt) {
 #ifdef __CUDA_ARCH__
   (void)salt;
   float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(f));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint_as_float(fb)));
   return __float_as_uint(r);
 #else
+  float f;
+  memcpy(&f, &fb, sizeof(f));
   const float r = 1.0f / f;
   uint32_t rb;
   memcpy(&rb, &r, sizeof(rb));
-  return rb + (uint32_t)(salt % 3u) - 1u;
+  return f == 2.0f ? rb : rb + salt % 3u - 1u;
 #endif
 }
 
-/* a / b rounded to nearest even, in integer arithmetic (normal operands, normal result; zero
- * numerators too).  With A, B the significands (2^52 <= A, B < 2^53) and t = (A < B), the
- * result's significand is N = RN(X / B), X = A 2^(52 + t), in [2^52, 2^53]:
- *  1. R0 ~ 2^84 / B from a float reciprocal of B's leading 24 bits (relative error < 2^-22;
- *     the reciprocal is clamped to the interval the exact one lies in);
- *  2. R ~ 2^115 / B = R0 2^31 (1 + e + e^2), e = 1 - B R0 / 2^84 (error e^3 plus truncations,
- *     below 2^-60), all in 64-bit fixed point;
- *  3. Q = floor(X R / 2^115), within one of floor(X / B); the remainder X - Q B is formed
- *     exactly (its magnitude is below 2^55, so 64-bit wrap-around arithmetic holds it) and
- *     brings Q to floor(X / B) with 0 <= remainder < B, which is checked: any other outcome takes
- *     the FP64 quotient;
- *  4. N = Q + 1 when twice the remainder exceeds B (or equals it, Q odd: a tie, which a quotient
- *     of two 53-bit numbers cannot produce).
- * Every result is the IEEE quotient's bits; the approximations of steps 1-2 only decide how
- * often the correction of step 3 is needed. */
-XD_NOINLINE double em_div(double a, double b) {
-  const uint64_t ua = xbits(a), ub = xbits(b);
-  const uint32_t ea = (uint32_t)(ua >> 52) & 0x7ffu, eb = (uint32_t)(ub >> 52) & 0x7ffu;
-  const uint64_t S = (ua ^ ub) & 0x8000000000000000ull;
-  if (eb - 1u >= 2046u) return xdiv_slow(a, b);
-  /* a zero numerator has a zero exponent field: its test runs behind the exponent test (written
-   * on the whole pattern ahead of it, the compiler made it an FP64 comparison on every call) */
-  if (ea - 1u >= 2046u) return zero_u(ua) ? xdbl(S) : xdiv_slow(a, b);  /* +-0 / normal: +-0 */
-  const uint64_t M = (1ull << 52) - 1;
-  const uint64_t A = (ua & M) | (1ull << 52), B = (ub & M) | (1ull << 52);
-  const uint32_t t = (A < B) ? 1u : 0u;
-  const int e = (int)ea - (int)eb + 1023 - (int)t;  /* the result's exponent field */
-  if ((uint32_t)(e - 1) >= 2045u) return xdiv_slow(a, b);
-  /* 1. */
-  const uint32_t fb = 0x3f800000u | ((uint32_t)(B >> 29) & 0x7fffffu);
-  float f;
-  memcpy(&f, &fb, sizeof(f));
-  const uint32_t rb = xrcp_seed(f, B);
-  /* R0 = 2^32 r with r clamped to [1/2, 1 - 2^-32] (1/f lies in (1/2, 1]) */
-  const uint64_t R0 = (rb >= 0x3f800000u) ? 0xffffffffull
-                      : (rb < 0x3f000000u) ? 0x80000000ull : ((uint64_t)((rb & 0x7fffffu) | 0x800000u) << 8);
-  /* 2. E0 = 2^84 e (|E0| < 2^63); T = 2^84 (e + e^2), the square from E0's leading bits */
-  const int64_t E0 = (int64_t)(0ull - B * R0);
-  const int64_t Eh = E0 >> 32;
-  const int64_t T = E0 + ((Eh * Eh) >> 20);
-  const int64_t Ph = (int64_t)R0 * (T >> 32);
-  const uint64_t Pl = R0 * (uint64_t)(uint32_t)T;
-  const int64_t P = Ph + (int64_t)(Pl >> 32);  /* floor(R0 T / 2^32) */
-  const uint64_t R = (R0 << 31) + (uint64_t)(P >> 21);
+/* a / b rounded to nearest, in integer arithmetic, by two digits of a long division.  With A, B the
+ * significands (2^52 <= A, B < 2^53) and t = (A < B), the result's significand is RN(q),
+ * q = A 2^(52 + t) / B in [2^52, 2^53).  Write R* = 2^84 / B (in (2^31, 2^32]) and b = B 2^8.
+ *  1. R0 < R*: a float reciprocal of B's leading 24 bits plus one, less 512: R* - R0 <= 1280.
+ *  2. R1 = R0 (1 + e), e = 1 - R0 / R* to 31 bits, lowered by 4 units: R* - 5.01 <= R1 <= R*.
+ *  3. q1 = floor(X R1 / 2^32), X the leading 32 bits of A 2^(10 + t): 0 <= A 2^(30 + t) / B - q1 <=
+ *     7.02, so the remainder r1 = A 2^(38 + t) - q1 b is in [0, 7.02 b), below 2^64: formed exactly
+ *     modulo 2^64.
+ *  4. q2 = floor(r1 R1 / 2^70) from r1's high word: 0 <= r1 2^22 / b - q2 < 1.11.  Q = q1 2^22 + q2
+ *     is then within [q - 1.11, q], and RN(q) = Q + 1 exactly when 2 (r1 2^22 - q2 b) > b: the sign
+ *     of (2 q2 + 1) b - r1 2^23, again exact modulo 2^64.  (A quotient of two 53-bit numbers is
+ *     never a tie.)
+ * Only the seed is approximate, and its error is inside the bounds above; every result is the IEEE
+ * quotient. */
+XD_FN_DIV double em_div(double a, double b) {
+  uint32_t al, ah, bl, bh;
+  xwords(a, al, ah);
+  xwords(b, bl, bh);
+  if (!xwindow(ah, bh)) return xdiv_slow(a, b);
+  const uint32_t ma = (ah & 0xfffffu) | 0x100000u, mb = (bh & 0xfffffu) | 0x100000u;
+  /* 1., 2. */
+  const uint32_t bn = xshl(bl, mb, 11);               /* B's leading 32 bits */
+  const uint32_t R0 = xrcp_seed((bn >> 8) + 0x3f000001u, bl) * 256u + (0x80000000u - 0x200u);
+  const uint32_t d2 = xmulhi32(bn, R0) * 0xfffffffeu - 4u;
+  const uint32_t R1 = xmulhi32(R0, d2) + R0;
   /* 3. */
-  uint64_t Q = xmulhi(A << 11, R) >> (10 - t);
-  int64_t rem = (int64_t)((A << (52 + t)) - Q * B);
-  if (rem < 0) { Q -= 1; rem += (int64_t)B; }
-  else if (rem >= (int64_t)B) { Q += 1; rem -= (int64_t)B; }
-  if ((uint64_t)rem >= B) return xdiv_slow(a, b);
+  const bool lt = (((uint64_t)ma << 32) | al) < (((uint64_t)mb << 32) | bl);
+  const uint32_t X = xshl(al, ma, lt ? 11u : 10u);
+  const uint32_t b8l = bl << 8, b8h = xshl(bl, mb, 8);
+  const uint32_t q1 = xmulhi32(X, R1);
+  const uint64_t b8 = ((uint64_t)b8h << 32) | b8l;
+  const uint64_t r1 = ((uint64_t)(al << (lt ? 7u : 6u)) << 32) - (uint64_t)q1 * b8;
   /* 4. */
-  const uint64_t r2 = (uint64_t)rem << 1;
-  Q += (r2 > B || (r2 == B && (Q & 1u))) ? 1u : 0u;
-  return xdbl((((uint64_t)(e - 1) << 52) + Q) | S);
+  const uint32_t q2 = xmulhi32((uint32_t)(r1 >> 32), R1) >> 6;
+  const uint64_t D = (uint64_t)(2u * q2 + 1u) * b8 - (r1 << 23);
+  const uint64_t Q = (uint64_t)q1 * (1u << 22) + q2;
+  const uint32_t e = (ah - ma) - (bh - mb) + (lt ? (1021u << 20) : (1022u << 20));
+  return xround((uint32_t)Q, (uint32_t)(Q >> 32), (uint32_t)(D >> 32), e);
 }
 
-XD_HD int64_t xmulhi_s(int64_t a, int64_t b) {
-#ifdef __CUDA_ARCH__
-  return __mul64hi(a, b);
-#else
-  return (int64_t)(((__int128)a * b) >> 64);
-#endif
+/* the FP64 square root, for the operands the integer path does not cover; zeros are their own roots */
+XD_NOINLINE double xsqrt_slow(double x) {
+  uint32_t lo, hi;
+  xwords(x, lo, hi);
+  if (((hi << 1) | lo) == 0) return x;
+  return ::sqrt(x);
 }
 
-/* the FP64 square root, for the operands the integer path does not cover */
-XD_NOINLINE double xsqrt_slow(double x) { return ::sqrt(x); }
-
-/* bits of an approximation to 1/sqrt(f), f in [1, 4): rsqrt.approx.ftz.f32 on the device; on the
- * host the quotient of 1 and the float root moved by -1, 0 or +1 unit */
-XD_HD uint32_t xrsqrt_seed(float f, uint64_t salt) {
+/* bits of an approximation to 1/sqrt(f), f in (1, 4], within [1/2, 1 - 2^-24]: rsqrt.approx.ftz.f32 on
+ * the device (relative error below 2^-22.9); on the host the quotient of 1 and the float root moved
+ * by -1, 0 or +1 unit */
+XD_HD uint32_t xrsqrt_seed(uint32_t fb, uint32_t salt) {
+  uint32_t gb;
 #ifdef __CUDA_ARCH__
   (void)salt;
-  float r;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(f));
-  return __float_as_uint(r);
+  float g;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(g) : "f"(__uint_as_float(fb)));
+  gb = __float_as_uint(g);
 #else
-  const float r = 1.0f / std::sqrt(f);
-  uint32_t rb;
-  memcpy(&rb, &r, sizeof(rb));
-  return rb + (uint32_t)(salt % 3u) - 1u;
-#endif
-}
-
-/* sqrt(x) rounded to nearest even, in integer arithmetic (positive normal x; zeros too).  With X
- * the significand and p the parity of the unbiased exponent, the result's significand is
- * N = RN(sqrt(Y)), Y = X 2^(52 + p) in [2^104, 2^106):
- *  1. G0 ~ 2^32 / sqrt(X 2^(p - 52)) from the float reciprocal square root of X's leading 24
- *     bits (clamped to the interval (1/2, 1] the exact one lies in);
- *  2. e = 1 - Y G0^2 / 2^168 and S = X G0 2^(p - 32) (1 + e/2 + 3 e^2 / 8) (error 5 e^3 / 16 plus
- *     truncations), plus one, which puts S within one of floor(sqrt(Y));
- *  3. the remainder Y - S^2, exact in 64-bit wrap-around arithmetic (its magnitude is below
- *     2^57), brings S to floor(sqrt(Y)) with 0 <= remainder <= 2 S, which is checked: any other
- *     outcome takes the FP64 root;
- *  4. N = S + 1 when the remainder exceeds S (sqrt(Y) above S + 1/2; never equal to it).
- * Every result is the IEEE root's bits. */
-XD_NOINLINE double em_sqrt(double x) {
-  const uint64_t ux = xbits(x);
-  const uint32_t ex = (uint32_t)(ux >> 52);  /* sign bit included: negative x fails the test */
-  /* +-0 is its own root (tested behind the exponent test, as in em_div) */
-  if (ex - 1u >= 2046u) return zero_u(ux) ? x : xsqrt_slow(x);
-  const uint64_t X = (ux & ((1ull << 52) - 1)) | (1ull << 52);
-  const uint32_t p = (ex & 1u) ^ 1u;
-  const int er = (((int)ex - 1023 - (int)p) >> 1) + 1023;  /* the result's exponent field */
-  /* 1. */
-  const uint32_t fb = ((127u + p) << 23) | ((uint32_t)(X >> 29) & 0x7fffffu);
   float f;
   memcpy(&f, &fb, sizeof(f));
-  const uint32_t gb = xrsqrt_seed(f, X);
-  const uint64_t G0 = (gb >= 0x3f800000u) ? 0xffffffffull
-                      : (gb < 0x3f000000u) ? 0x80000000ull : ((uint64_t)((gb & 0x7fffffu) | 0x800000u) << 8);
-  /* 2. Ee = 2^63 e, C = 2^64 (e/2 + 3 e^2 / 8) */
-  const uint64_t hi = xmulhi(X << 11, G0 * G0);  /* floor(X G0^2 / 2^53) ~ 2^(63 - p) (1 - e) */
-  const int64_t Ee = (int64_t)((1ull << (63 - p)) - hi) << p;
-  const int64_t Eh = Ee >> 20;
-  const int64_t Cc = Ee + ((3 * Eh * Eh) >> 25);
-  const uint64_t lo = X * G0, xh = xmulhi(X, G0);
-  const int64_t Sb = (int64_t)((xh << (32 + p)) | (lo >> (32 - p)));  /* floor(X G0 2^(p - 32)) */
-  uint64_t S = (uint64_t)(Sb + xmulhi_s(Sb, Cc)) + 1u;
-  /* 3. */
-  int64_t rem = (int64_t)((X << (52 + p)) - S * S);
-  if (rem < 0) { rem += (int64_t)(2 * S - 1); S -= 1; }
-  else if (rem > (int64_t)(2 * S)) { rem -= (int64_t)(2 * S + 1); S += 1; }
-  if (rem < 0 || rem > (int64_t)(2 * S)) return xsqrt_slow(x);
-  /* 4. */
-  S += (rem > (int64_t)S) ? 1u : 0u;
-  return xdbl(((uint64_t)(er - 1) << 52) + S);
-}
-
-/* The bit pattern a comparison keys on.  On the device an opaque register move: when a value that
- * an FP64 sum has just formed is compared on its bits, the compiler otherwise forms the sum twice,
- * once for the double and once for its bits (measured: 16 key comparisons of running sums took 35
- * FP64 additions instead of 18).  (The same move in every bit operation of this file made the WAF
- * edge slower: it also blocks the folding of its sign flips and scalings.) */
-XD_HD uint64_t xbits_cmp(double x) {
-  uint64_t b;
-#ifdef __CUDA_ARCH__
-  asm("mov.b64 %0, %1;" : "=l"(b) : "d"(x));
-#else
-  memcpy(&b, &x, sizeof(b));
+  const float g = 1.0f / std::sqrt(f);
+  memcpy(&gb, &g, sizeof(gb));
+  gb = gb + salt % 3u - 1u;
 #endif
-  return b;
+  gb = gb > 0x3f7fffffu ? 0x3f7fffffu : gb;
+  return gb < 0x3f000000u ? 0x3f000000u : gb;
 }
 
+/* sqrt(x) rounded to nearest, in integer arithmetic (positive normal x), by two digits.  With X the
+ * significand and p the parity of the unbiased exponent, the result's significand is RN(s),
+ * s = sqrt(Y), Y = X 2^(52 + p) in [2^104, 2^106).  Write f = X 2^(p - 52) in [1, 4) and
+ * G* = 2^32 / sqrt(f).
+ *  1. G0 < G*: a float reciprocal root of f's leading 24 bits plus one, less 1024 units.
+ *  2. G1 = G0 (1 + (1 - f g^2) / 2) to 31 bits, lowered by 6 units: G* - 8 <= G1 <= G*.
+ *  3. s1 = floor(F G1 / 2^32), F the leading 32 bits of f: 0 <= sqrt(f) 2^30 - s1 <= 10, and the
+ *     remainder r1 = X 2^(8 + p) - s1^2 is in [0, 2^35.4).
+ *  4. s2 = floor(r1 G1 / 2^41) from r1's leading 32 bits: S = s1 2^22 + s2 has 0 <= s - S < 1.41 (the
+ *     square of s2 adds at most 0.19), and RN(s) = S + 1 exactly when Y - S^2 > S: the sign of
+ *     S^2 + S - Y modulo 2^64.  (s is never halfway between two integers.)
+ * Every result is the IEEE root. */
+XD_FN_SQRT double em_sqrt(double x) {
+  uint32_t xl, xh;
+  xwords(x, xl, xh);
+  if (xh - 0x100000u >= 0x7fe00000u) return xsqrt_slow(x);   /* zero, subnormal, negative, inf, NaN */
+  const uint32_t xm = (xh & 0xfffffu) | 0x100000u;
+  const uint32_t p = (~xh >> 20) & 1u;
+  /* 1., 2. */
+  const uint32_t F = xshr(xl, xm, 22u - p);
+  const uint32_t G0 = xrsqrt_seed(xshr(xl, xm, 29) + 0x3f000001u + (p << 23), xl) * 256u + (0x80000000u - 0x400u);
+  const uint32_t t = xmulhi32(xmulhi32(G0, G0), F);
+  const uint32_t G1 = xmulhi32(G0, 0x7ffffffau - 2u * t) + G0;
+  /* 3. */
+  const uint32_t s1 = xmulhi32(F, G1);
+  const uint64_t r1 = (((((uint64_t)xm << 32) | xl) << 8) << p) - (uint64_t)s1 * s1;
+  /* 4. */
+  const uint32_t s2 = xmulhi32((uint32_t)(r1 >> 4), G1) >> 5;
+  const uint64_t S = (uint64_t)s1 * (1u << 22) + s2;
+  const uint64_t D = S * S + S - ((uint64_t)(xl << (20u + p)) << 32);
+  const uint32_t e = (((xh + (1023u << 20)) >> 1) & 0x7ff00000u) - 0x100000u;
+  return xround((uint32_t)S, (uint32_t)(S >> 32), (uint32_t)(D >> 32), e);
+}
+
+/* Comparisons on the words of the patterns: the IEEE results, on the integer pipes.
+ *
+ * Against a finite constant c of +0 or above the pattern of x compares as a signed integer (a negative x is
+ * below every c, a NaN of positive sign above them all, so that one NaN sign is left to exclude). */
+XD_HD bool xzero(double x) {
+  uint32_t lo, hi;
+  xwords(x, lo, hi);
+  return ((hi << 1) | lo) == 0;
+}
+XD_HD bool xcmp_const(uint32_t ch) { return ch < 0x7ff00000u; }   /* c: not negative, finite */
+XD_HD long long xsword(uint32_t lo, uint32_t hi) { return (long long)(((uint64_t)hi << 32) | lo); }
+XD_HD bool xnan(uint32_t lo, uint32_t hi) { return (((uint64_t)(hi & 0x7fffffffu) << 32) | lo) > 0x7ff0000000000000ull; }
 /* ordered integer key of a non-NaN double: order of the values, -0 and +0 equal */
-XD_HD long long xkey(uint64_t b) {
-  const long long s = (long long)b >> 63;
-  return (long long)((b & 0x7fffffffffffffffull) ^ (uint64_t)s) - s;
+XD_HD long long xkey(uint32_t lo, uint32_t hi) {
+  const uint32_t s = (uint32_t)((int32_t)hi >> 31);
+  return (long long)((((uint64_t)((hi & 0x7fffffffu) ^ s)) << 32) | (lo ^ s)) - (long long)(int32_t)s;
 }
-XD_HD bool xnan(uint64_t b) { return (b & 0x7fffffffffffffffull) > 0x7ff0000000000000ull; }
-/* a < b, a <= b, a == b (IEEE results, NaN compares false) on ordered keys; OC: the keys of the
- * opaque bit patterns (xbits_cmp), else of the plain ones */
-template <bool OC> XD_HD uint64_t xbits_key(double x) { return OC ? xbits_cmp(x) : xbits(x); }
-template <bool OC = true> XD_HD bool xlt(double a, double b) {
-  const uint64_t ua = xbits_key<OC>(a), ub = xbits_key<OC>(b);
-  return !(xnan(ua) | xnan(ub)) & (xkey(ua) < xkey(ub));
+XD_HD bool xlt(double a, double b) {
+  uint32_t al, ah, bl, bh;
+  xwords(a, al, ah);
+  xwords(b, bl, bh);
+  return !(xnan(al, ah) | xnan(bl, bh)) & (xkey(al, ah) < xkey(bl, bh));
 }
-template <bool OC = true> XD_HD bool xle(double a, double b) {
-  const uint64_t ua = xbits_key<OC>(a), ub = xbits_key<OC>(b);
-  return !(xnan(ua) | xnan(ub)) & (xkey(ua) <= xkey(ub));
+XD_HD bool xle(double a, double b) {
+  uint32_t al, ah, bl, bh;
+  xwords(a, al, ah);
+  xwords(b, bl, bh);
+  return !(xnan(al, ah) | xnan(bl, bh)) & (xkey(al, ah) <= xkey(bl, bh));
 }
-template <bool OC = true> XD_HD bool xeq(double a, double b) {
-  const uint64_t ua = xbits_key<OC>(a), ub = xbits_key<OC>(b);
-  return !(xnan(ua) | xnan(ub)) & (xkey(ua) == xkey(ub));
+XD_HD bool xeq(double a, double b) {
+  uint32_t al, ah, bl, bh;
+  xwords(a, al, ah);
+  xwords(b, bl, bh);
+  return !(xnan(al, ah) | xnan(bl, bh)) & (xkey(al, ah) == xkey(bl, bh));
+}
+/* x < c, x > c, x <= c for the constants of the flux code (0, 1/2, 1, 2, eps, tolisec, tol): the
+ * test of c folds away for a literal and is the same for every thread otherwise */
+XD_HD bool xlt_c(double x, double c) {
+  const uint64_t bc = xbits(c);
+  if (!xcmp_const((uint32_t)(bc >> 32))) return xlt(x, c);
+  uint32_t lo, hi;
+  xwords(x, lo, hi);
+  const long long sx = xsword(lo, hi);
+  if (bc == 0) return (uint64_t)sx - 0x8000000000000001ull < 0x7ff0000000000000ull;
+  return (sx < (long long)bc) & ((uint64_t)sx <= 0xfff0000000000000ull);
+}
+XD_HD bool xgt_c(double x, double c) {
+  const uint64_t bc = xbits(c);
+  if (!xcmp_const((uint32_t)(bc >> 32))) return xlt(c, x);
+  uint32_t lo, hi;
+  xwords(x, lo, hi);
+  const long long sx = xsword(lo, hi);
+  return (sx > (long long)bc) & (sx <= 0x7ff0000000000000ll);
+}
+/* x < b for a b of +0 .. +inf that is not a literal: as xlt_c, and -0 is not below +0 */
+XD_HD bool xlt_nonneg(double x, double b) {
+  uint32_t lo, hi, bl, bh;
+  xwords(x, lo, hi);
+  xwords(b, bl, bh);
+  const long long sx = xsword(lo, hi), sb = xsword(bl, bh);
+  return (sx < sb) & ((uint64_t)sx <= 0xfff0000000000000ull) & ((hi != 0x80000000u) | (((bl | bh | lo)) != 0));
+}
+XD_HD bool xle_c(double x, double c) {
+  const uint64_t bc = xbits(c);
+  if (!xcmp_const((uint32_t)(bc >> 32))) return xle(x, c);
+  uint32_t lo, hi;
+  xwords(x, lo, hi);
+  const long long sx = xsword(lo, hi);
+  return (sx <= (long long)bc) & ((uint64_t)sx <= 0xfff0000000000000ull);
 }
 
-template <bool MUL, bool OC = true>
+template <bool MUL>
 struct XD {
   double v;
   XD_HD XD() : v(0.0) {}
   XD_HD XD(double x) : v(x) {}  // NOLINT: constants promote implicitly
 };
 
-template <bool MUL, bool OC>
-XD_HD double val(const XD<MUL, OC>& x) { return x.v; }
+template <bool MUL>
+XD_HD double val(const XD<MUL>& x) { return x.v; }
 
 template <bool MUL>
 XD_HD double xd_mul(double a, double b) {
@@ -293,36 +381,69 @@ XD_HD double xd_div(double a, double b) {
 }
 
 #define CF_XD_BIN(op, expr)                                                                               \
-  template <bool MUL, bool OC> XD_HD XD<MUL, OC> operator op(const XD<MUL, OC>& a, const XD<MUL, OC>& b) { double x = a.v, y = b.v; return XD<MUL, OC>(expr); } \
-  template <bool MUL, bool OC> XD_HD XD<MUL, OC> operator op(const XD<MUL, OC>& a, double y) { double x = a.v; return XD<MUL, OC>(expr); } \
-  template <bool MUL, bool OC> XD_HD XD<MUL, OC> operator op(double x, const XD<MUL, OC>& b) { double y = b.v; return XD<MUL, OC>(expr); }
+  template <bool MUL> XD_HD XD<MUL> operator op(const XD<MUL>& a, const XD<MUL>& b) { double x = a.v, y = b.v; return XD<MUL>(expr); } \
+  template <bool MUL> XD_HD XD<MUL> operator op(const XD<MUL>& a, double y) { double x = a.v; return XD<MUL>(expr); } \
+  template <bool MUL> XD_HD XD<MUL> operator op(double x, const XD<MUL>& b) { double y = b.v; return XD<MUL>(expr); }
 CF_XD_BIN(+, x + y)
 CF_XD_BIN(-, x - y)
 CF_XD_BIN(*, xd_mul<MUL>(x, y))
 CF_XD_BIN(/, xd_div<MUL>(x, y))
 #undef CF_XD_BIN
 
+/* x with its high word combined: the sign-bit operations below */
+XD_HD double xhi_xor(double x, uint32_t m) {
+  uint32_t lo, hi;
+  xwords(x, lo, hi);
+  return xjoin(lo, hi ^ m);
+}
+XD_HD uint32_t xhi(double x) {
+  uint32_t lo, hi;
+  xwords(x, lo, hi);
+  return hi;
+}
 /* negation as a sign-bit flip: an FP64 negation that is not folded into its consumer is an FP64
  * instruction, and most consumers here are integer code (products, comparisons) */
-template <bool MUL, bool OC> XD_HD XD<MUL, OC> operator-(const XD<MUL, OC>& a) { return XD<MUL, OC>(xdbl(xbits(a.v) ^ 0x8000000000000000ull)); }
+template <bool MUL> XD_HD XD<MUL> operator-(const XD<MUL>& a) { return XD<MUL>(xhi_xor(a.v, 0x80000000u)); }
 
-#define CF_XD_CMP(op, expr)                                                                               \
-  template <bool MUL, bool OC> XD_HD bool operator op(const XD<MUL, OC>& a, const XD<MUL, OC>& b) { double x = a.v, y = b.v; return expr; } \
-  template <bool MUL, bool OC> XD_HD bool operator op(const XD<MUL, OC>& a, double y) { double x = a.v; return expr; } \
-  template <bool MUL, bool OC> XD_HD bool operator op(double x, const XD<MUL, OC>& b) { double y = b.v; return expr; }
-CF_XD_CMP(<, xlt<OC>(x, y))
-CF_XD_CMP(>, xlt<OC>(y, x))
-CF_XD_CMP(<=, xle<OC>(x, y))
-CF_XD_CMP(>=, xle<OC>(y, x))
-CF_XD_CMP(==, xeq<OC>(x, y))
-CF_XD_CMP(!=, !xeq<OC>(x, y))
-#undef CF_XD_CMP
+template <bool MUL> XD_HD bool operator<(const XD<MUL>& a, const XD<MUL>& b) { return xlt(a.v, b.v); }
+template <bool MUL> XD_HD bool operator>(const XD<MUL>& a, const XD<MUL>& b) { return xlt(b.v, a.v); }
+template <bool MUL> XD_HD bool operator<=(const XD<MUL>& a, const XD<MUL>& b) { return xle(a.v, b.v); }
+template <bool MUL> XD_HD bool operator>=(const XD<MUL>& a, const XD<MUL>& b) { return xle(b.v, a.v); }
+template <bool MUL> XD_HD bool operator==(const XD<MUL>& a, const XD<MUL>& b) { return xeq(a.v, b.v); }
+template <bool MUL> XD_HD bool operator!=(const XD<MUL>& a, const XD<MUL>& b) { return !xeq(a.v, b.v); }
+template <bool MUL> XD_HD bool operator<(const XD<MUL>& a, double c) { return xlt_c(a.v, c); }
+template <bool MUL> XD_HD bool operator>(const XD<MUL>& a, double c) { return xgt_c(a.v, c); }
+template <bool MUL> XD_HD bool operator<=(const XD<MUL>& a, double c) { return xle_c(a.v, c); }
+template <bool MUL> XD_HD bool operator>=(const XD<MUL>& a, double c) { return xle(c, a.v); }
+template <bool MUL> XD_HD bool operator==(const XD<MUL>& a, double c) { return xeq(a.v, c); }
+template <bool MUL> XD_HD bool operator!=(const XD<MUL>& a, double c) {
+  return xbits(c) == 0 ? !xzero(a.v) : !xeq(a.v, c);
+}
+template <bool MUL> XD_HD bool operator<(double c, const XD<MUL>& a) { return xgt_c(a.v, c); }
+template <bool MUL> XD_HD bool operator>(double c, const XD<MUL>& a) { return xlt_c(a.v, c); }
+template <bool MUL> XD_HD bool operator<=(double c, const XD<MUL>& a) { return xle(c, a.v); }
+template <bool MUL> XD_HD bool operator>=(double c, const XD<MUL>& a) { return xle_c(a.v, c); }
 
-template <bool MUL, bool OC> XD_HD XD<MUL, OC> sqrt(const XD<MUL, OC>& a) { return XD<MUL, OC>(MUL ? em_sqrt(a.v) : ::sqrt(a.v)); }
-template <bool MUL, bool OC> XD_HD XD<MUL, OC> rcbrt(const XD<MUL, OC>& a) { return XD<MUL, OC>(rcbrt(a.v)); }
-template <bool MUL, bool OC> XD_HD XD<MUL, OC> fabs(const XD<MUL, OC>& a) { return XD<MUL, OC>(xdbl(xbits(a.v) & 0x7fffffffffffffffull)); }
-template <bool MUL, bool OC> XD_HD XD<MUL, OC> sgnmul(const XD<MUL, OC>& x, const XD<MUL, OC>& y) {
-  return XD<MUL, OC>(xdbl(xbits(y.v) ^ (xbits(x.v) & 0x8000000000000000ull)));
+template <bool MUL> XD_HD bool lt_nonneg(const XD<MUL>& a, const XD<MUL>& b) { return xlt_nonneg(a.v, b.v); }
+template <bool MUL>
+struct ConstOps<XD<MUL>> {
+  static XD_HD double quot(double a, double d, double y) { return val(div_rn(XD<MUL>(a), d, y)); }
+  static XD_HD double half(double x) { return val(halve(XD<MUL>(x))); }
+  static XD_HD double dbl(double x) { return val(twice(XD<MUL>(x))); }
+};
+
+/* max(0, x) with dmax's results: x where 0 < x, else +0 (-0, negative and NaN x) */
+template <bool MUL> XD_HD XD<MUL> dmax0(const XD<MUL>& x) { return xgt_c(x.v, 0.0) ? x : XD<MUL>(0.0); }
+
+template <bool MUL> XD_HD XD<MUL> sqrt(const XD<MUL>& a) { return XD<MUL>(MUL ? em_sqrt(a.v) : ::sqrt(a.v)); }
+template <bool MUL> XD_HD XD<MUL> rcbrt(const XD<MUL>& a) { return XD<MUL>(rcbrt(a.v)); }
+template <bool MUL> XD_HD XD<MUL> fabs(const XD<MUL>& a) {
+  uint32_t lo, hi;
+  xwords(a.v, lo, hi);
+  return XD<MUL>(xjoin(lo, hi & 0x7fffffffu));
+}
+template <bool MUL> XD_HD XD<MUL> sgnmul(const XD<MUL>& x, const XD<MUL>& y) {
+  return XD<MUL>(xhi_xor(y.v, xhi(x.v) & 0x80000000u));
 }
 
 /* x * 2^K (K = -2, -1, 1) by a change of the exponent field, for a normal x whose result is
@@ -330,30 +451,33 @@ template <bool MUL, bool OC> XD_HD XD<MUL, OC> sgnmul(const XD<MUL, OC>& x, cons
  * infinite and NaN operands and results out of the normal range take the FP64 product. */
 template <int K>
 XD_HD double xscale(double x) {
-  const uint64_t b = xbits(x);
-  const uint32_t e = (uint32_t)(b >> 52) & 0x7ffu;
+  uint32_t l, h;
+  xwords(x, l, h);
   const uint32_t lo = (K < 0) ? (uint32_t)(1 - K) : 1u;          /* lowest exponent field handled */
   const uint32_t n = (K < 0) ? (uint32_t)(2046 + K) : (uint32_t)(2046 - K);  /* fields handled */
-  if (e - lo < n) return xdbl(b + ((uint64_t)(int64_t)K << 52));
-  if (zero_u(b)) return x;
-  return xmul_slow(x, (K == -2) ? 0.25 : ((K == -1) ? 0.5 : 2.0));
+  const bool ok = h * 2u - (lo << 21) < (n << 21);
+  if (!ok && ((h << 1) | l) != 0) return xmul_slow(x, (K == -2) ? 0.25 : ((K == -1) ? 0.5 : 2.0));
+  return xjoin(l, ok ? h + ((uint32_t)K << 20) : h);
 }
-template <bool MUL, bool OC> XD_HD XD<MUL, OC> halve(const XD<MUL, OC>& x) { return XD<MUL, OC>(MUL ? xscale<-1>(x.v) : x.v * 0.5); }
-template <bool MUL, bool OC> XD_HD XD<MUL, OC> quarter(const XD<MUL, OC>& x) { return XD<MUL, OC>(MUL ? xscale<-2>(x.v) : x.v * 0.25); }
-template <bool MUL, bool OC> XD_HD XD<MUL, OC> twice(const XD<MUL, OC>& x) { return XD<MUL, OC>(MUL ? xscale<1>(x.v) : x.v * 2.0); }
+template <bool MUL> XD_HD XD<MUL> halve(const XD<MUL>& x) { return XD<MUL>(MUL ? xscale<-1>(x.v) : x.v * 0.5); }
+template <bool MUL> XD_HD XD<MUL> quarter(const XD<MUL>& x) { return XD<MUL>(MUL ? xscale<-2>(x.v) : x.v * 0.25); }
+template <bool MUL> XD_HD XD<MUL> twice(const XD<MUL>& x) { return XD<MUL>(MUL ? xscale<1>(x.v) : x.v * 2.0); }
+
+/* RN(1/d) for the quotients of div_rn: not needed where the quotient is formed directly */
+template <bool MUL> XD_HD XD<MUL> recip(const XD<MUL>& d) { return MUL ? XD<MUL>(0.0) : XD<MUL>(1.0 / d.v); }
 
 /* The quotient a / d that div_rn in cf_flux.h forms from y = RN(1/d) by Markstein's step: on the
  * integer path the division itself (the same bits, y unused), otherwise Markstein's step. */
-template <bool MUL, bool OC>
-XD_HD XD<MUL, OC> div_rn(const XD<MUL, OC>& a, double d, double y) {
-  if (MUL) return XD<MUL, OC>(em_div(a.v, d));
+template <bool MUL>
+XD_HD XD<MUL> div_rn(const XD<MUL>& a, double d, double y) {
+  if (MUL) return XD<MUL>(em_div(a.v, d));
   const double q = a.v * y;
   const double r = fma(-d, q, a.v);
   const double q1 = fma(r, y, q);
-  return XD<MUL, OC>(zero_u(xbits(a.v)) ? q : q1);
+  return XD<MUL>(zero_u(xbits(a.v)) ? q : q1);
 }
-template <bool MUL, bool OC>
-XD_HD XD<MUL, OC> div_rn(const XD<MUL, OC>& a, const XD<MUL, OC>& d, const XD<MUL, OC>& y) {
+template <bool MUL>
+XD_HD XD<MUL> div_rn(const XD<MUL>& a, const XD<MUL>& d, const XD<MUL>& y) {
   return div_rn(a, d.v, y.v);
 }
 
