@@ -26,7 +26,7 @@
  * is linear in the sums and is transposed by hand around a Dual<4> friction block.
  *
  * Replay kernels (k_rep_edges, k_rep_cells) advance a state with a recorded dt / time
- * sequence; they run the step's own edge_body / element_update, so a replayed trajectory is
+ * sequence; they run the step's own edge_lanes / element_update, so a replayed trajectory is
  * bit-identical to the recorded one.
  */
 #include <cuda_runtime.h>
@@ -34,6 +34,7 @@
 #include <algorithm>
 
 #include "cf_dual.h"
+#include "cf_edge_kernel.cuh"
 #include "cf_xd.h"
 
 namespace cf {
@@ -64,20 +65,13 @@ __device__ __forceinline__ size_t hidx(int n, int m, int nm) { return (size_t)n 
 /* The replays keep the forward kernels' occupancy: eight edge blocks and four element blocks per SM
  * (64 registers), where the latency of the integer-pipe chains is hidden by more warps. */
 template <int IFLUX>
-__global__ void __launch_bounds__(TILE_E, 8) k_rep_edges(StepArgs a, const double* dt_hist, const double* t_hist, int n) {
+__global__ void __launch_bounds__(2 * TILE_E, 4) k_rep_edges(StepArgs a, const double* dt_hist, const double* t_hist, int n) {
   const int tile = blockIdx.x;
   const int m = __ldg(a.etile_mem + tile);
   const MemberDev& M = a.mdev[m];
-  const int e = tile * TILE_E + threadIdx.x;
-  if (e >= M.edge_end) return;
+  const int e = tile * TILE_E + (threadIdx.x >> 1);
   const size_t h = hidx(n, m, a.nmembers);
-  const double dt = __ldg(dt_hist + h), t = __ldg(t_hist + h);
-  if (a.xd_cmp) {   /* the context's integer-pipe setting, as the step's edge kernel (same results) */
-    if ((a.xd_mul_mask >> (threadIdx.x >> 5)) & 1) edge_body<IFLUX, XD<true>>(a, M, e, dt, t);
-    else edge_body<IFLUX, XD<false>>(a, M, e, dt, t);
-  } else {
-    edge_body<IFLUX>(a, M, e, dt, t);
-  }
+  edge_lanes<IFLUX>(a, M, e, threadIdx.x & 1, e < M.edge_end, __ldg(dt_hist + h), __ldg(t_hist + h), nullptr);
 }
 
 __global__ void __launch_bounds__(TILE_C, 4) k_rep_cells(StepArgs a, const double* dt_hist, int n, uint32_t* flag,
@@ -449,9 +443,9 @@ int launch_replay_step(const StepArgs& a, const double* dt_hist, const double* t
                        Slot* sums, stream_t s) {
   cudaStream_t st = reinterpret_cast<cudaStream_t>(s);
   switch (a.iflux) {
-    case 1: k_rep_edges<1><<<a.n_etiles, TILE_E, 0, st>>>(a, dt_hist, t_hist, n); break;
-    case 2: k_rep_edges<2><<<a.n_etiles, TILE_E, 0, st>>>(a, dt_hist, t_hist, n); break;
-    case 3: k_rep_edges<3><<<a.n_etiles, TILE_E, 0, st>>>(a, dt_hist, t_hist, n); break;
+    case 1: k_rep_edges<1><<<a.n_etiles, 2 * TILE_E, 0, st>>>(a, dt_hist, t_hist, n); break;
+    case 2: k_rep_edges<2><<<a.n_etiles, 2 * TILE_E, 0, st>>>(a, dt_hist, t_hist, n); break;
+    case 3: k_rep_edges<3><<<a.n_etiles, 2 * TILE_E, 0, st>>>(a, dt_hist, t_hist, n); break;
     default: return CF_ENOTSUP;
   }
   k_rep_cells<<<a.n_ctiles, TILE_C, 0, st>>>(a, dt_hist, n, flag, sums);

@@ -2,19 +2,21 @@
  * cf_edge_kernel.cuh -- the edge kernel of the step (included by one small translation unit per
  * scheme, cf_edges_<IFLUX>.cu, so that the launch shapes of the four schemes compile in parallel).
  *
- * k_edges<IFLUX, BE, EPT>: blocks of BE threads, each thread evaluating EPT edges (e, e + BE, ...
- * of its block's BE * EPT consecutive edges).  Edges keep their layout of tiles of TILE_E = 128
- * edges, each owned by one member, whatever the shape: a thread looks up its edge's member, and
- * the integer-pipe warp mask bit w applies to the edges (e mod 128) / 32 = w of a tile.  Every
+ * k_edges<IFLUX, BE, EPT>: blocks of BE threads, two neighbouring lanes per edge, one for each of its
+ * sides (EdgeSide in cf_flux.h: what the sides share goes through shuffles), each lane evaluating EPT
+ * sides (i, i + BE, ... of its block's BE * EPT consecutive ones).  Edges keep their layout of tiles of
+ * TILE_E = 128 edges, each owned by one member, whatever the shape: a lane looks up its edge's member,
+ * and the integer-pipe warp mask bit w applies to the edges (e mod 128) / 32 = w of a tile.  Every
  * shape evaluates the same edges with the same arithmetic, so results do not depend on it (the
  * autotuner chooses one).
  *
- * Register budget: every IFLUX 1-3 shape keeps 1024 threads per SM (at most 64 registers; with
- * spills to L1): the tuned edge is chains of dependent integer-pipe products and quotients between
- * its FP64 sums and the warps hide their latency (1M WAF, tuned, 128-thread blocks: 0.462 ms at
- * four blocks per SM, 0.434 at five, 0.421 at six, 0.408 at eight; HLLC 0.266 -> 0.215 ms).
- * MUSCL-Hancock keeps 512 threads per SM (128 registers): at 1024 its spills cost more than the
- * warps gain (1.39 ms), at 384 (138 registers) it takes 1.32 ms, at 512 1.21 ms.
+ * What bounds it: a wet WAF side is ~4,100 instructions of which 55 are FP64 ones (76 cycles each on
+ * their pipe): issue slots 58 %, FP64 pipe 65 %, the two integer pipes 56 and 41 % busy, waits on
+ * fixed latencies and on instruction fetch between them (WAF 201k triangles, fully wet).
+ *
+ * Register budget: every IFLUX 1-3 shape keeps 1024 threads per SM (at most 64 registers); 768, 1280
+ * and 1536 threads measured the same within 3 % or slower (WAF 201k: 168 us per step at 1024; 172, 175,
+ * 181).  MUSCL-Hancock keeps 512 threads per SM (128 registers); 640 and 768 measured the same.
  */
 #ifndef CF_EDGE_KERNEL_CUH
 #define CF_EDGE_KERNEL_CUH
@@ -50,59 +52,118 @@ __device__ __forceinline__ void step_start(const MemberDev& M, MemberState* S, i
   }
 }
 
-/* The edge of index e of a step (member M, state S, parity p), in the context's arithmetic type. */
+/* One side of an edge on this lane, the other one on the neighbouring lane (lane ^ 1); mask holds the
+ * lanes whose edges are being evaluated. */
+template <int IFLUX, class T_>
+struct LanePair {
+  using T = T_;
+  using Side = EdgeSide<IFLUX, T>;
+  Side s;
+  T out[5];
+  unsigned mask;
+  template <class F>
+  __device__ __forceinline__ void each(F&& f) { f(s, out); }
+  __device__ __forceinline__ void exchange(int n) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+      if (k < n) s.y[k] = T(__shfl_xor_sync(mask, val(s.x[k]), 1));
+  }
+};
+
+/* This lane's side of the interior edge e (element state U), by every lane of mask at once */
+template <int IFLUX, class T>
+__device__ __forceinline__ void edge_side(const StepArgs& a, const MemberDev& M, unsigned mask, int e, int side,
+                                          const double4& geo, const double4& U, double dt) {
+  LanePair<IFLUX, T> p;
+  p.mask = mask;
+  side_load(a, M, e, side, geo, U, dt, p.s);
+  double4 dk = make_double4(0.0, 0.0, 0.0, 0.0);
+  if (IFLUX == 4) dk = ld4(a.edk + e);
+  side_stages<IFLUX>(p, a.ilimiteur, dk.x, dk.z, dk.y, dk.w);
+  if (a.flux_mode == 1) {   /* side B: side A's flux, negated */
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const T f = T(__shfl_xor_sync(mask, val(p.out[k]), 1));
+      if (side) p.out[k] = -f;
+    }
+  }
+  store_side(a.slots + 2 * (size_t)e + side, p.out, geo.z);
+}
+
+/* Edge e of a step on the lanes of its two sides, in the context's arithmetic type.  Every lane of the
+ * warp comes here; live: the lane's edge is one to evaluate (the 16 edges of a warp belong to one
+ * tile, so to one member and one setting of the integer-pipe mask). */
 template <int IFLUX>
-__device__ __forceinline__ void edge_in_step(const StepArgs& a, const MemberDev& M, MemberState* S, int e, double dt,
-                                             double t) {
-  if (a.xd_cmp) {
-    /* the same arithmetic with exact integer comparisons and, in the warps of xd_mul_mask,
-     * exact integer products: the FP64 pipe and the integer pipes share the work.  */
-    if ((a.xd_mul_mask >> ((e % TILE_E) >> 5)) & 1) edge_body<IFLUX, XD<true>>(a, M, e, dt, t, S->surf);
-    else edge_body<IFLUX, XD<false>>(a, M, e, dt, t, S->surf);
-  } else {
-    edge_body<IFLUX>(a, M, e, dt, t, S->surf);
+__device__ __forceinline__ void edge_lanes(const StepArgs& a, const MemberDev& M, int e, int side, bool live, double dt,
+                                           double t, const double* surf) {
+  int2 ab = make_int2(0, -3);
+  double4 geo = make_double4(0.0, 0.0, 0.0, 0.0), U = geo;
+  if (live) {
+    /* the normal and length, which every path needs, load beside the element's state */
+    ab = ldro(a.ecell + e);
+    geo = ld4(a.egeo + e);
+    U = ld4(a.Uin + ((side && ab.y >= 0) ? ab.y : ab.x));   /* {h, hu, hv, RN(1/h)} */
+  }
+  const double hp = __shfl_xor_sync(0xffffffffu, U.x, 1);
+  bool run = live && ab.y >= 0;
+  if (run && (dbits_hd(U.x) | dbits_hd(hp)) == 0 && dry_edge_ok<IFLUX>(M.gp, geo, dt)) {
+    /* an edge between two dry elements (most of a flood plain that the water has not reached) needs
+     * neither its beds nor its upwind states */
+    dry_slot<IFLUX>(M.gp, a.flux_mode, geo, side, a.slots + 2 * (size_t)e + side);
+    run = false;
+  }
+  const unsigned mask = __ballot_sync(0xffffffffu, run);
+  if (run) {
+    if (a.xd_cmp) {
+      /* the same arithmetic with exact integer comparisons and, in the warps of xd_mul_mask, exact
+       * integer products, quotients and roots: the FP64 pipe and the integer pipes share the work */
+      if ((a.xd_mul_mask >> ((e % TILE_E) >> 5)) & 1) edge_side<IFLUX, XD<true>>(a, M, mask, e, side, geo, U, dt);
+      else edge_side<IFLUX, XD<false>>(a, M, mask, e, side, geo, U, dt);
+    } else {
+      edge_side<IFLUX, double>(a, M, mask, e, side, geo, U, dt);
+    }
+  } else if (live && ab.y < 0 && side == 0) {
+    boundary_slot<IFLUX>(a, M, e, ab, geo, U, t, surf);
   }
 }
 
 template <int IFLUX, int BE, int EPT>
 __global__ void __launch_bounds__(BE, ((IFLUX == 4) ? 512 : 1024) / BE) k_edges(StepArgs a) {
   const int p = a.parity;
-  const int nedge = a.n_etiles * TILE_E;
+  const int nside = 2 * a.n_etiles * TILE_E;
 #pragma unroll 1
   for (int j = 0; j < EPT; ++j) {
-    const int e = (blockIdx.x * EPT + j) * BE + threadIdx.x;
-    if (e >= nedge) return;
+    const int i = (blockIdx.x * EPT + j) * BE + threadIdx.x;
+    if (i >= nside) return;
+    const int e = i >> 1;
     const int m = __ldg(a.etile_mem + e / TILE_E);
     const MemberDev& M = a.mdev[m];
     MemberState* S = a.mst + m;
     if (S->status) continue;
     const double dt = S->dt[p];
     const double t = S->t[p];
-    if (e == M.edge_begin) step_start(M, S, p);
-    if (e >= M.edge_end) continue;
-    edge_in_step<IFLUX>(a, M, S, e, dt, t);
+    if (i == 2 * M.edge_begin) step_start(M, S, p);
+    edge_lanes<IFLUX>(a, M, e, i & 1, e < M.edge_end, dt, t, S->surf);
   }
 }
 
-/* The edges of a list (a part's phase of its step): 128-thread blocks, one edge per thread; the
- * step's start is made by k_begin_step before the first phase. */
+/* The edges of a list (a part's phase of its step; a part is a context of one member): TILE_E lanes per
+ * block; the step's start is made by k_begin_step before the first phase. */
 template <int IFLUX>
 __global__ void __launch_bounds__(TILE_E, (IFLUX == 4) ? 4 : 8) k_edges_list(StepArgs a, const int32_t* list, int n) {
-  const int i = blockIdx.x * TILE_E + threadIdx.x;
-  if (i >= n) return;
-  const int e = list[i];
-  const int m = __ldg(a.etile_mem + e / TILE_E);
-  const MemberDev& M = a.mdev[m];
-  MemberState* S = a.mst + m;
-  if (S->status || e >= M.edge_end) return;
-  edge_in_step<IFLUX>(a, M, S, e, S->dt[a.parity], S->t[a.parity]);
+  const int i = (blockIdx.x * TILE_E + threadIdx.x) >> 1;
+  const MemberDev& M = a.mdev[0];
+  MemberState* S = a.mst;
+  if (S->status) return;
+  const int e = i < n ? list[i] : 0;
+  edge_lanes<IFLUX>(a, M, e, threadIdx.x & 1, i < n && e < M.edge_end, S->dt[a.parity], S->t[a.parity], S->surf);
 }
 
 template <int IFLUX, int BE, int EPT>
 void launch_edges_shape(const StepArgs& a, cudaStream_t st) {
-  const int nedge = a.n_etiles * TILE_E;
+  const int nside = 2 * a.n_etiles * TILE_E;
   const int per = BE * EPT;
-  k_edges<IFLUX, BE, EPT><<<(nedge + per - 1) / per, BE, 0, st>>>(a);
+  k_edges<IFLUX, BE, EPT><<<(nside + per - 1) / per, BE, 0, st>>>(a);
 }
 
 }  // namespace
@@ -110,7 +171,7 @@ void launch_edges_shape(const StepArgs& a, cudaStream_t st) {
 template <int IFLUX>
 int launch_edges_list_iflux(const StepArgs& a, const int32_t* list, int32_t n, cudaStream_t st) {
   if (n <= 0) return CF_OK;
-  k_edges_list<IFLUX><<<(n + TILE_E - 1) / TILE_E, TILE_E, 0, st>>>(a, list, n);
+  k_edges_list<IFLUX><<<(2 * n + TILE_E - 1) / TILE_E, TILE_E, 0, st>>>(a, list, n);
   return cudaGetLastError() == cudaSuccess ? CF_OK : CF_ECUDA;
 }
 

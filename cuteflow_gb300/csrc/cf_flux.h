@@ -353,7 +353,8 @@ CF_HD CF_INLINE void first_order_flux(double g, double nx, double ny, T hl, T ul
     const int rb = (-sr > 0.) ? 1 : ((-sl < 0.) ? 0 : 2);
     T h1 = T(0.0), h2 = T(0.0);
     if (ra == 2 || rb == 2) {
-      const T den = sr - sl + eps, yden = recip(den);
+      const T den = sr - sl + eps;
+    const auto yden = recip(den);
       h1 = div_rn(sr * fl1 - sl * fr1 + sl * sr * (hr - hl), den, yden);
       h2 = div_rn(sr * fl2 - sl * fr2 + sl * sr * (hr * ur - hl * ul), den, yden);
     }
@@ -464,7 +465,8 @@ CF_HD CF_INLINE void waf_flux(double g, int ilim, double nx, double ny, double d
   const int rb = (-sr > 0.) ? 1 : ((-sl < 0.) ? 0 : 2);
   T h1 = T(0.0), h2 = T(0.0);
   if (ra == 2 || rb == 2) {
-    const T den = sr - sl + eps, yden = recip(den);
+    const T den = sr - sl + eps;
+    const auto yden = recip(den);
     h1 = div_rn(sr * fl1 - sl * fr1 + sl * sr * (hr - hl), den, yden);
     h2 = div_rn(sr * fl2 - sl * fr2 + sl * sr * (hr * ur - hl * ul), den, yden);
   }
@@ -485,7 +487,8 @@ CF_HD CF_INLINE void waf_flux(double g, int ilim, double nx, double ny, double d
 
   /* side A (:854-899) */
   {
-    const T den = dloc + eps, yd = recip(den);
+    const T den = dloc + eps;
+    const auto yd = recip(den);
     const T rl = held(div_rn((sl > 0.) ? upl : upr, den, yd), freeze_r);
     const T rr = held(div_rn((sr > 0.) ? upl : upr, den, yd), freeze_r);
     const T ll = waf_limiter(ilim, rl, cl);
@@ -507,7 +510,8 @@ CF_HD CF_INLINE void waf_flux(double g, int ilim, double nx, double ny, double d
    * (hl - hr)/d = -dloc, its upwind differences are minus A's (for the wave it tests), the
    * tangential ones coincide; its Courant numbers are -cr, -cl, -cet. */
   {
-    const T den = -dloc + eps, yd = recip(den);
+    const T den = -dloc + eps;
+    const auto yd = recip(den);
     const T rl = held(div_rn((-sr > 0.) ? -upr : -upl, den, yd), freeze_r);
     const T rr = held(div_rn((-sl > 0.) ? -upr : -upl, den, yd), freeze_r);
     /* B's tangential ratio differs from A's only when s* == 0 (or is NaN) */
@@ -621,7 +625,8 @@ CF_HD CF_INLINE void muscl_side(double g, double tolisec, int ilim, double dtove
   } else {
     const T fl1 = h1 * u1, fl2 = h1 * (u1 * u1) + halve(g * h1 * h1);
     const T fr1 = h2 * u2, fr2 = h2 * (u2 * u2) + halve(g * h2 * h2);
-    const T den = sr - sl + eps, yden = recip(den);
+    const T den = sr - sl + eps;
+    const auto yden = recip(den);
     x1 = div_rn(sr * fl1 - sl * fr1 + sl * sr * (h2 - h1), den, yden);
     x2 = div_rn(sr * fl2 - sl * fr2 + sl * sr * (h2 * u2 - h1 * u1), den, yden);
     x3 = (set > 0.) ? x1 * v1 : x1 * v2;
@@ -735,7 +740,8 @@ CF_HD CF_INLINE double upwind_bed(double z1, double z2, double d1, double d2, do
 }
 
 /* The same, loading the elements' states (w = RN(1/h)), in the edge's arithmetic type T; ds = d1 + d2
- * of a pair (twice its d_mkvol, which the preprocessing forms as (d1 + d2) / 2). */
+ * and
+ * ysum = RN(1/ds) of a pair. */
 template <class T>
 CF_HD CF_INLINE void upwind_state(const double4* U, int i1, int i2, double d1, double d2, double ds, double ysum,
                                   double nx, double ny, double tolisec, T& hu_, T& vu_) {
@@ -925,6 +931,334 @@ CF_HD CF_INLINE void interior_edge_muscl(const MemberDev& M, int ilim, int flux_
   out[9] = -(tb * ny);
 }
 
+/* ---- one side of an edge ---------------------------------------------------------------- */
+
+/* The limiter of one wave, out of line: a side evaluates three, and its code has to stay in the
+ * instruction cache (WAF 1M: 250 us per step with the three in place, 248 called). */
+#ifdef __CUDACC__
+template <class T>
+static __host__ __device__ __noinline__ T side_limiter(int ilim, T r, T c) { return waf_limiter(ilim, r, c); }
+#else
+template <class T>
+inline T side_limiter(int ilim, T r, T c) { return waf_limiter(ilim, r, c); }
+#endif
+
+/* The flux of a side with the reconstructed state (h, u, v) towards a nearly dry other side at rest of
+ * depth hr (IFLUX 1, 2): rare, out of line, in plain doubles (the same bits). */
+#ifdef __CUDACC__
+template <int IFLUX>
+static __host__ __device__ __noinline__ void nearly_dry_flux(double g, double nx, double ny, double h, double u,
+                                                             double v, double hr, double o[3]) {
+#else
+template <int IFLUX>
+static void nearly_dry_flux(double g, double nx, double ny, double h, double u, double v, double hr, double o[3]) {
+#endif
+  TwoFluxT<double> F;
+  first_order_flux<IFLUX>(g, nx, ny, h, u, v, hr, 0.0, 0.0, F);
+  o[0] = F.a1;
+  o[1] = F.a2;
+  o[2] = F.a3;
+}
+
+/* Both sides of an interior edge, evaluated in lockstep, each in its own frame (normal out of its own
+ * element) exactly as the reference evaluates the edge from each of its elements
+ * (flux_riemann.cuf:33-426).  On the GPU the two sides are two neighbouring lanes; on the host two
+ * objects.  What one side computes the other one needs mirrored (depths equal, normal and tangential
+ * velocities negated, s_L' = -s_R, the mass flux negated: all exact), so every quantity of one side is
+ * computed once, by its side, and offered to the other in x[]; after an exchange y[] holds the other
+ * side's x[].  A value that both need in the same form (a sum of the two depths, the HLL quotients, the
+ * contact speed's numerator and denominator) is computed by one side while the other computes a second
+ * such value with the same instruction.  The stages are
+ *
+ *   frame      own frame state, hydrostatic reconstruction          x: h, u, v (first order: and the
+ *                                                                      raw depth's reconstruction;
+ *                                                                      MUSCL: the upwind h, u, v)
+ *   speeds1    celerity; h + h' on side 0, u' - u on side 1         x: a, sum
+ *   speeds2    s_L, the own term of s*'s denominator, own flux      x: s_L, d, f1, f2
+ *   hll        own term of s*'s numerator, one HLL quotient per side;
+ *              WAF: one local slope per side, both upwind slopes    x: t2, q, slope, up_h, up_v
+ *   contact1   s*'s numerator on side 0, denominator on side 1      x: it
+ *   contact2   s*; IFLUX 2: the own star flux                       x: its three components
+ *   finish     the side's flux and bed source in the global frame
+ *
+ * A lane has half the code, half the live values and half the dependent chain of a thread that
+ * evaluates a whole edge, for the ~6 FP64 sums per edge that both sides repeat: WAF 201k triangles
+ * (fully wet), the edge kernel: 141 us with 608 local memory instructions per 32 edges -> 120 us with
+ * 232 (117 with the quotients by known reciprocals). */
+template <int IFLUX, class T>
+struct EdgeSide {
+  int side;                      /* 0: the edge's first element (its normal points out of it), 1: the second */
+  double g, tolisec, nx, ny, len;
+  T x[6], y[6];
+  T h0, hw;                      /* own raw depth; the raw depth's reconstruction */
+  T h, u, v;                     /* reconstructed, masked state, own frame */
+  T hr, ur, vr;                  /* the other side's, in the own frame */
+  T gh, a, s, as_, sl, sr, d0, f1, f2, fr1, fr2;
+  T t2, d, q1, q2, set;          /* q1, q2: HLL mass and momentum flux */
+  T hup, uup, vup, sloc, sloct, up_h, up_v, upr_h, upr_v;   /* WAF */
+  T e1, e2, e3;                  /* IFLUX 2 */
+  double dt, d_mrl, y_mrl, d_up, y_up;
+  bool dry;                      /* both reconstructed depths below eps: zero flux */
+  T hraw;                        /* first order: the other side's reconstruction from its raw depth */
+
+  static constexpr double eps() { return IFLUX == 1 ? EPS_HLLC : IFLUX == 2 ? EPS_RIADH : EPS_SECOND; }
+
+  /* U: own state; z, zo: beds of the own and of the other element */
+  CF_HD CF_INLINE void frame(const MemberDev& M, int side_, double nx_, double ny_, double len_, const double4& U,
+                             double z, double zo) {
+    side = side_;
+    g = M.gp;
+    tolisec = M.tolisec;
+    nx = nx_;
+    ny = ny_;
+    len = len_;
+    h0 = T(U.x);
+    T hm;
+    to_frame(h0, T(U.y), T(U.z), U.w, nx, ny, tolisec, hm, u, v);
+    const bool wet = h0 > tolisec;
+    const double zij = val(dmax(T(z), T(zo)));
+    hw = dmax0(h0 + z - zij);     /* a masked depth reconstructs to +0 (see interior_edge) */
+    h = wet ? hw : T(0.0);
+    if (h < tolisec) { h = T(0.); u = T(0.); v = T(0.); }
+    x[0] = h;
+    x[1] = u;
+    x[2] = v;
+    /* the other side reconstructs this one from its raw depth (:176-181), with the masked velocities */
+    if (IFLUX <= 2) x[3] = hw < tolisec ? T(0.) : hw;
+  }
+  /* second order: the side's upwind reconstruction from its upwind elements i1, i2 (distances d1, d2;
+   * d1 < 0: a copy of i1; bed zu), the time step and the distances to the other element and to the
+   * upwind reconstruction */
+  CF_HD CF_INLINE void upwind(const double4* U, int i1, int i2, double d1, double d2, double zu, double z, double zo,
+                              double dt_, double d_mrl_, double y_mrl_, double d_up_, double y_up_) {
+    dt = dt_;
+    d_mrl = d_mrl_;
+    y_mrl = y_mrl_;
+    d_up = d_up_;
+    y_up = y_up_;
+    /* of a pair d_up = (d1 + d2) / 2, so d1 + d2 and its reciprocal are exact scalings */
+    const double ds = ConstOps<T>::dbl(d_up), ysum = ConstOps<T>::half(y_up);
+    T hu_;
+    if (IFLUX == 4) upwind_state3(U, i1, i2, d1, d2, ds, ysum, nx, ny, tolisec, hu_, uup, vup);
+    else upwind_state(U, i1, i2, d1, d2, ds, ysum, nx, ny, tolisec, hu_, vup);
+    hup = dmax0(hu_ + zu - val(dmax(T(z), T(zo))));
+    if (hup < tolisec) { hup = T(0.); vup = T(0.); uup = T(0.); }
+    if (IFLUX == 4) {
+      x[3] = hup;
+      x[4] = uup;
+      x[5] = vup;
+    }
+  }
+  CF_HD CF_INLINE void speeds1() {
+    hr = y[0];
+    ur = -y[1];
+    vr = -y[2];
+    if (IFLUX <= 2) hraw = y[3];
+    dry = h < eps() && hr < eps();
+    gh = g * h;
+    a = sqrt(gh);
+    s = (side ? ur : h) + (side ? -u : hr);
+    x[0] = a;
+    x[1] = s;
+  }
+  CF_HD CF_INLINE void speeds2() {
+    const T ar = y[0];
+    const T hs = side ? y[1] : s, du = side ? s : y[1];
+    as_ = a + ar;
+    const T het = halve(hs) - quarter(du * hs / as_);
+    const bool wl = h > eps(), wr = hr > eps();
+    T pq;
+    if (lt_nonneg(het, h)) pq = T(1.);
+    else pq = wl ? sqrt(halve(het + h) * het / (h * h)) : T(0.);
+    const T sub = wl ? (wr ? a * pq : a) : twice(ar);
+    sl = (wl ? u : ur) - sub;
+    d0 = u - sl;
+    f1 = h * u;
+    f2 = h * (u * u) + halve(gh * h);
+    d = h * d0;
+    x[0] = sl;
+    x[1] = d;
+    x[2] = f1;
+    x[3] = f2;
+  }
+  CF_HD CF_INLINE void hll() {
+    sr = -y[0];
+    s = y[1];                      /* the other side's denominator term, negated in the own frame */
+    fr1 = -y[2];
+    fr2 = y[3];
+    t2 = sr * h * d0;
+    const T den = sr - sl + eps();
+    const T diff = (side ? fr1 : hr) - (side ? f1 : h);
+    const T num = sr * (side ? f2 : f1) - sl * (side ? fr2 : fr1) + sl * sr * diff;
+    q1 = num / den;
+    x[0] = t2;
+    x[1] = q1;
+    if (IFLUX == 3) {
+      sloc = div_rn((side ? vr : hr) - (side ? v : h), d_mrl, y_mrl);
+      up_h = div_rn(h - hup, d_up, y_up);
+      up_v = div_rn(v - vup, d_up, y_up);
+      x[2] = sloc;
+      x[3] = up_h;
+      x[4] = up_v;
+    }
+  }
+  CF_HD CF_INLINE void contact1() {
+    q2 = side ? q1 : y[1];
+    q1 = side ? -y[1] : q1;
+    if (IFLUX == 3) {
+      sloct = side ? sloc : y[2];
+      sloc = side ? -y[2] : sloc;
+      upr_h = -y[3];
+      upr_v = y[4];
+    }
+    /* side 0: (s_L h' (u' - s_R)) - (s_R h (u - s_L)); side 1: h' (u' - s_R) - h (u - s_L) of side 0 */
+    t2 = (side ? -d : y[0]) - (side ? s : t2);
+    x[0] = t2;
+  }
+  CF_HD CF_INLINE void contact2() {
+    const T num = side ? -y[0] : t2, denom = side ? t2 : y[0];
+    if (fabs(denom) < eps()) set = halve(u + ur) - (hr - h) * as_ / (h + hr);
+    else set = num / denom;
+    if (IFLUX == 2) {
+      const T f3 = f1 * v;
+      const T p = (fabs(sl - set) > eps()) ? h * (-d0) / (sl - set) : T(0.0);
+      e1 = f1 + sl * (p - h);
+      e2 = f2 + sl * (p * set - f1);
+      e3 = f3 + sl * (p * v - h * v);
+      x[0] = e1;
+      x[1] = e2;
+      x[2] = e3;
+    }
+  }
+  /* the side's flux (times the length) and bed source, global frame */
+  CF_HD CF_INLINE void finish(int ilim, T out[5]) {
+    T x1, x2, x3;
+    const int r = (sl > 0.) ? 0 : ((sr < 0.) ? 1 : 2);
+    if (IFLUX == 1) {
+      x1 = r == 0 ? f1 : (r == 1 ? fr1 : q1);
+      x2 = r == 0 ? f2 : (r == 1 ? fr2 : q2);
+      x3 = x1 * (r == 0 ? v : (r == 1 ? vr : (set > 0.) ? v : vr));
+    } else if (IFLUX == 2) {
+      /* 0 < s_L: F_L; 0 < s* and 0 > s_L: star left; 0 > s* and 0 < s_R: star right; else F_R */
+      const int k = (0. < sl) ? 0 : ((0. < set && 0. > sl) ? 2 : ((0. > set && 0. < sr) ? 3 : 1));
+      x1 = k == 0 ? f1 : (k == 1 ? fr1 : (k == 2 ? e1 : -y[0]));
+      x2 = k == 0 ? f2 : (k == 1 ? fr2 : (k == 2 ? e2 : y[1]));
+      x3 = k == 2 ? e3 : (k == 3 ? y[2] : (k == 0 ? f1 * v : fr1 * vr));
+    } else {
+      const T m1 = r == 0 ? f1 : (r == 1 ? fr1 : q1);
+      const T m2 = r == 0 ? f2 : (r == 1 ? fr2 : q2);
+      const double dtoverdx = ConstOps<T>::quot(dt, d_mrl, y_mrl);
+      const T den = sloc + eps();
+      const auto yd = recip(den);
+      const T rl = div_rn((sl > 0.) ? up_h : upr_h, den, yd);
+      const T rr = div_rn((sr > 0.) ? up_h : upr_h, den, yd);
+      const T re = ((set > 0.) ? up_v : upr_v) / (sloct + eps());
+      const T ll = sgnmul(sl, side_limiter(ilim, rl, sl * dtoverdx));
+      const T lr = sgnmul(sr, side_limiter(ilim, rr, sr * dtoverdx));
+      const T le = sgnmul(set, side_limiter(ilim, re, set * dtoverdx));
+      const T wl = halve(1. + ll), wlr = halve(lr - ll), wr = halve(1. - lr);
+      x1 = wl * f1 + wlr * m1 + wr * fr1;
+      x2 = wl * f2 + wlr * m2 + wr * fr2;
+      x3 = (halve(1. + le) * v + halve(1. - le) * vr) * x1;
+    }
+    out[0] = x1;
+    out[1] = nx * x2 - ny * x3;
+    out[2] = ny * x2 + nx * x3;
+    if (dry) out[0] = out[1] = out[2] = T(0.0);
+    if (IFLUX <= 2 && hraw != hr) {
+      /* a nearly dry other side (0 < h <= tolisec), whose raw depth reaches the higher bed */
+      double o[3];
+      nearly_dry_flux<IFLUX>(g, nx, ny, val(h), val(u), val(v), val(hraw), o);
+      out[0] = T(o[0]);
+      out[1] = T(o[1]);
+      out[2] = T(o[2]);
+    }
+  }
+  /* MUSCL-Hancock: the flux of this side from the exchanged states; d_upr, y_upr: the other side's
+   * upwind distance */
+  CF_HD CF_INLINE void muscl(int ilim, double d_upr, double y_upr, T out[5]) {
+    T x1, x2, x3;
+    muscl_side(g, tolisec, ilim, ConstOps<T>::quot(dt, d_mrl, y_mrl), d_mrl, y_mrl, d_up, y_up, d_upr, y_upr, h, u, v,
+               y[0], -y[1], -y[2], hup, uup, vup, y[3], -y[4], -y[5], x1, x2, x3);
+    out[0] = x1;
+    out[1] = nx * x2 - ny * x3;
+    out[2] = ny * x2 + nx * x3;
+  }
+  CF_HD CF_INLINE void bed(T out[5]) {
+    const T t = ConstOps<T>::half(g) * (hw * hw - h0 * h0) * len;
+    out[3] = t * nx;
+    out[4] = t * ny;
+  }
+};
+
+/* The stages of both sides of an edge.  P holds the sides at hand: the lane's own one on the GPU
+ * (exchange: shuffles with the neighbouring lane), both on the host. */
+template <int IFLUX, class P>
+CF_HD CF_INLINE void side_stages(P& p, int ilim, double d_up0, double y_up0, double d_up1, double y_up1) {
+  using S = typename P::Side;
+  if (IFLUX == 4) {
+    p.exchange(6);
+    p.each([&](S& s, typename P::T* out) {
+      s.muscl(ilim, s.side ? d_up0 : d_up1, s.side ? y_up0 : y_up1, out);
+      s.bed(out);
+    });
+  } else {
+    p.exchange(IFLUX == 3 ? 3 : 4);
+    p.each([&](S& s, typename P::T*) { s.speeds1(); });
+    p.exchange(2);
+    p.each([&](S& s, typename P::T*) { s.speeds2(); });
+    p.exchange(4);
+    p.each([&](S& s, typename P::T*) { s.hll(); });
+    p.exchange(IFLUX == 3 ? 5 : 2);
+    p.each([&](S& s, typename P::T*) { s.contact1(); });
+    p.exchange(1);
+    p.each([&](S& s, typename P::T*) { s.contact2(); });
+    if (IFLUX == 2) p.exchange(3);
+    p.each([&](S& s, typename P::T* out) {
+      s.finish(ilim, out);
+      s.bed(out);
+    });
+  }
+}
+
+/* The inputs of one side of interior edge e: its element's state U, normal out of that element */
+template <int IFLUX, class T>
+CF_HD CF_INLINE void side_load(const StepArgs& a, const MemberDev& M, int e, int side, const double4& geo,
+                               const double4& U, double dt, EdgeSide<IFLUX, T>& s) {
+  const double2 z = ldro(reinterpret_cast<const double2*>(a.ez + e));        /* bed of A, of B */
+  const double zo = side ? z.x : z.y, zs = side ? z.y : z.x;
+  const double nx = side ? -geo.x : geo.x, ny = side ? -geo.y : geo.y;
+  s.frame(M, side, nx, ny, geo.z, U, zs, zo);
+  if (IFLUX >= 3) {
+    const double zu = ldro(reinterpret_cast<const double*>(a.ez + e) + 2 + side);
+    const int2 up = ldro(reinterpret_cast<const int2*>(a.eupw + e) + side);
+    const double2 dw = ldro(reinterpret_cast<const double2*>(a.ewts + e) + side);
+    const double4 dk = ld4(a.edk + e);
+    const double yi = ldro(reinterpret_cast<const double*>(a.einv + e));
+    s.upwind(a.Uin, up.x, up.y, dw.x, dw.y, zu, zs, zo, dt, geo.w, yi, side ? dk.y : dk.x, side ? dk.w : dk.z);
+  }
+}
+
+/* Both sides of an edge, one after another (host) */
+template <int IFLUX, class T_>
+struct HostPair {
+  using T = T_;
+  using Side = EdgeSide<IFLUX, T>;
+  Side s[2];
+  T out[2][5];
+  template <class F>
+  CF_HD void each(F&& f) {
+    f(s[0], out[0]);
+    f(s[1], out[1]);
+  }
+  CF_HD void exchange(int n) {
+    for (int k = 0; k < n; ++k) {
+      s[0].y[k] = s[1].x[k];
+      s[1].y[k] = s[0].x[k];
+    }
+  }
+};
+
 /* Static data of edge e in the form interior_edge takes. */
 CF_HD CF_INLINE EdgeGeo edge_geo(const StepArgs& a, int e, bool second, const double4& geo) {
   EdgeGeo G;
@@ -967,12 +1301,6 @@ CF_HD CF_INLINE void store_slot(Slot* p, double f1, double f2, double f3, double
 #endif
 }
 
-/* The two slots of an interior edge from interior_edge's out[10]. */
-CF_HD CF_INLINE void write_slots(Slot* sa, const double o[10]) {
-  store_slot(sa, o[0], o[1], o[2], o[3], o[4], 0.0);
-  store_slot(sa + 1, o[5], o[6], o[7], o[8], o[9], 0.0);
-}
-
 /* ---- dry regions ------------------------------------------------------------------------ */
 
 CF_HD CF_INLINE uint64_t dbits_hd(double x) {
@@ -1006,31 +1334,35 @@ CF_HD CF_INLINE double dbl_hd(uint64_t b) {
  * slots are these signed zeros whenever g, len, nx and ny are finite; otherwise (returns false)
  * the caller evaluates the edge. */
 template <int IFLUX>
-CF_HD CF_INLINE bool dry_edge_slots(double g, int flux_mode, const double4& geo, Slot* sa, double dt = 0.0) {
+CF_HD CF_INLINE bool dry_edge_ok(double g, const double4& geo, double dt) {
+  return finite_u(dbits_hd(g)) & finite_u(dbits_hd(geo.x)) & finite_u(dbits_hd(geo.y)) & finite_u(dbits_hd(geo.z)) &
+         (IFLUX != 4 || finite_u(dbits_hd(dt)));
+}
+/* the slot of one side (0 or 1) when dry_edge_ok holds */
+template <int IFLUX>
+CF_HD CF_INLINE void dry_slot(double g, int flux_mode, const double4& geo, int side, Slot* p) {
   const uint64_t S = 0x8000000000000000ull;
   const uint64_t bg = dbits_hd(g), bnx = dbits_hd(geo.x), bny = dbits_hd(geo.y), bl = dbits_hd(geo.z);
-  if (!(finite_u(bg) & finite_u(bnx) & finite_u(bny) & finite_u(bl))) return false;
-  if (IFLUX == 4 && !finite_u(dbits_hd(dt))) return false;
   const uint64_t sl = bl & S;                              /* the sign of len */
-  const uint64_t st = (bg & S) ^ sl;                       /* ta = tb = (g/2 * +0) * len */
-  /* the flux vectors (before * len): side A's frame flux rotated by n, side B's by -n */
-  uint64_t a1 = 0, a2 = 0, a3 = 0, b1 = 0, b2 = 0, b3 = 0;
+  const uint64_t st = (bg & S) ^ sl ^ (side ? S : 0);      /* ta = tb = (g/2 * +0) * len, side B negated */
+  /* the flux vector (before * len): the frame flux rotated by n, side B's by -n */
+  uint64_t f1 = 0, f2 = 0, f3 = 0;
+  const bool neg = side && flux_mode == 1;                 /* minus side A's */
   if (IFLUX == 4) {
-    const double x = geo.x * 0.0, y = geo.y * 0.0, mx = (-geo.x) * 0.0, my = (-geo.y) * 0.0;
-    a2 = dbits_hd(x - y);
-    a3 = dbits_hd(y + x);
-    b2 = dbits_hd(mx - my);
-    b3 = dbits_hd(my + mx);
+    const bool mirror = side && !neg;
+    const double x = (mirror ? -geo.x : geo.x) * 0.0, y = (mirror ? -geo.y : geo.y) * 0.0;
+    f2 = dbits_hd(x - y);
+    f3 = dbits_hd(y + x);
   }
-  if (flux_mode == 1) {
-    b1 = a1 ^ S;
-    b2 = a2 ^ S;
-    b3 = a3 ^ S;
-  }
-  store_slot(sa, dbl_hd((a1 & S) ^ sl), dbl_hd((a2 & S) ^ sl), dbl_hd((a3 & S) ^ sl), dbl_hd(st ^ (bnx & S)),
+  const uint64_t sf = sl ^ (neg ? S : 0);
+  store_slot(p, dbl_hd((f1 & S) ^ sf), dbl_hd((f2 & S) ^ sf), dbl_hd((f3 & S) ^ sf), dbl_hd(st ^ (bnx & S)),
              dbl_hd(st ^ (bny & S)), 0.0);
-  store_slot(sa + 1, dbl_hd((b1 & S) ^ sl), dbl_hd((b2 & S) ^ sl), dbl_hd((b3 & S) ^ sl),
-             dbl_hd(st ^ (bnx & S) ^ S), dbl_hd(st ^ (bny & S) ^ S), 0.0);
+}
+template <int IFLUX>
+CF_HD CF_INLINE bool dry_edge_slots(double g, int flux_mode, const double4& geo, Slot* sa, double dt = 0.0) {
+  if (!dry_edge_ok<IFLUX>(g, geo, dt)) return false;
+  dry_slot<IFLUX>(g, flux_mode, geo, 0, sa);
+  dry_slot<IFLUX>(g, flux_mode, geo, 1, sa + 1);
   return true;
 }
 
@@ -1084,66 +1416,48 @@ CF_HD CF_INLINE bool dry_neighbourhood(const MemberDev& M, const int4& nb, const
   return (dbits_hd(h_of(nb.x)) | dbits_hd(h_of(nb.y)) | dbits_hd(h_of(nb.z))) == 0;
 }
 
-/* Fluxes (times the edge length) and bed sources of edge e into its two slots, from the
- * state U of step n: the body of the edge kernel. */
-template <int IFLUX, class S = double>
-CF_HD CF_INLINE void edge_body(const StepArgs& a, const MemberDev& M, int e, double dt, double t,
-                               const double* surf = nullptr) {
-  const int2 ab = ldro(a.ecell + e);
-  /* the normal and length, which every path needs, load beside the element states (a dry edge
-   * then waits for two memory round trips, not three) */
-  const double4 geo = ld4(a.egeo + e);
-  const double4 UA = ld4(a.Uin + ab.x);   /* {h, hu, hv, RN(1/h)} */
-  Slot* sa = a.slots + 2 * (size_t)e;
+/* The slot of boundary edge e (kind ab.y < 0) */
+template <int IFLUX>
+CF_HD CF_INLINE void boundary_slot(const StepArgs& a, const MemberDev& M, int e, int2 ab, const double4& geo,
+                                   const double4& UA, double t, const double* surf) {
+  const double len = geo.z;
+  const int id = ldro(a.ebid + e);
+  const double sf = (surf && ab.y == -1 && M.inlet == 3 && id >= 1 && id <= M.nin) ? surf[id - 1] : 0.0;
+  double f1, f2, f3, q;
+  boundary_flux(IFLUX, M, ab.y, id, t, geo.x, geo.y, UA.x, UA.y, UA.z, UA.w, ldro(reinterpret_cast<const double*>(a.ez + e)),
+                f1, f2, f3, q, sf);
+  store_slot(a.slots + 2 * (size_t)e, f1 * len, f2 * len, f3 * len, 0.0, 0.0, q * len);
+}
 
-  if (ab.y >= 0) {
-    /* an edge between two dry elements (most of a flood plain that the water has not reached)
-     * needs neither its geometry beyond the normal nor its upwind states */
-    const double hB = ldro(reinterpret_cast<const double*>(a.Uin + ab.y));
-    if ((dbits_hd(UA.x) | dbits_hd(hB)) == 0 && dry_edge_slots<IFLUX>(M.gp, a.flux_mode, geo, sa, dt)) return;
-  }
-  const double4 ez = ld4(a.ez + e);       /* bed of A, of B, of A's and B's upwind reconstructions */
+/* A side's flux times the length, and its bed source, into its slot */
+template <class T>
+CF_HD CF_INLINE void store_side(Slot* p, const T out[5], double len) {
+  store_slot(p, val(out[0] * len), val(out[1] * len), val(out[2] * len), val(out[3]), val(out[4]), 0.0);
+}
 
+/* Fluxes (times the edge length) and bed sources of edge e into its two slots, from the state U of step
+ * n, on the host: the stages that the edge kernel runs on two lanes. */
+template <int IFLUX, class T = double>
+inline void edge_body(const StepArgs& a, const MemberDev& M, int e, double dt, double t, const double* surf = nullptr) {
+  const int2 ab = a.ecell[e];
+  const double4 geo = a.egeo[e], UA = a.Uin[ab.x];
   if (ab.y < 0) {
-    const double len = geo.z;
-    const int id = ldro(a.ebid + e);
-    const double sf = (surf && ab.y == -1 && M.inlet == 3 && id >= 1 && id <= M.nin) ? surf[id - 1] : 0.0;
-    double f1, f2, f3, q;
-    boundary_flux(IFLUX, M, ab.y, id, t, geo.x, geo.y, UA.x, UA.y, UA.z, UA.w, ez.x, f1, f2, f3, q, sf);
-    store_slot(sa, f1 * len, f2 * len, f3 * len, 0.0, 0.0, q * len);
+    boundary_slot<IFLUX>(a, M, e, ab, geo, UA, t, surf);
     return;
   }
-
-  const EdgeGeo G = edge_geo(a, e, IFLUX >= 3, geo);
-  const double4 UB = ld4(a.Uin + ab.y);
-  double o[10];
-  if (IFLUX == 4) {
-    const int4 up = ldro(a.eupw + e);
-    const double4 dw = ld4(a.ewts + e);
-    S upA[3], upB[3], om[10];
-    upwind_state3(a.Uin, up.x, up.y, dw.x, dw.y, ConstOps<S>::dbl(G.d_mkvol), G.ysum_a, G.nx, G.ny, M.tolisec, upA[0], upA[1], upA[2]);
-    upwind_state3(a.Uin, up.z, up.w, dw.z, dw.w, ConstOps<S>::dbl(G.d_mkvoisin), G.ysum_b, G.nx, G.ny, M.tolisec, upB[0], upB[1], upB[2]);
-    interior_edge_muscl(M, a.ilimiteur, a.flux_mode, G, dt, S(UA.x), S(UA.y), S(UA.z), ez.x, UA.w, S(UB.x), S(UB.y),
-                        S(UB.z), ez.y, UB.w, upA, ez.z, upB, ez.w, om);
-#pragma unroll
-    for (int i = 0; i < 10; ++i) o[i] = val(om[i]);
-    write_slots(sa, o);
-    return;
-  }
-  S hl_upw = S(0.0), vl_upw = S(0.0), hr_upw = S(0.0), vr_upw = S(0.0);
-  if (IFLUX == 3) {
-    const int4 up = ldro(a.eupw + e);
-    const double4 dw = ld4(a.ewts + e);   /* d1, d2 of side A, d1, d2 of side B */
-    upwind_state(a.Uin, up.x, up.y, dw.x, dw.y, ConstOps<S>::dbl(G.d_mkvol), G.ysum_a, G.nx, G.ny, M.tolisec, hl_upw, vl_upw);
-    upwind_state(a.Uin, up.z, up.w, dw.z, dw.w, ConstOps<S>::dbl(G.d_mkvoisin), G.ysum_b, G.nx, G.ny, M.tolisec, hr_upw, vr_upw);
-  }
-  S os[10];
-  interior_edge<(IFLUX == 4 ? 3 : IFLUX)>(M, a.ilimiteur, a.flux_mode, G, dt, S(UA.x), S(UA.y), S(UA.z), ez.x,
-                                          UA.w, S(UB.x), S(UB.y), S(UB.z), ez.y, UB.w, hl_upw, vl_upw, ez.z, hr_upw,
-                                          vr_upw, ez.w, os);
-#pragma unroll
-  for (int i = 0; i < 10; ++i) o[i] = val(os[i]);
-  write_slots(sa, o);
+  Slot* sa = a.slots + 2 * (size_t)e;
+  const double4 UB = a.Uin[ab.y];
+  /* an edge between two dry elements (most of a flood plain that the water has not reached) */
+  if ((dbits_hd(UA.x) | dbits_hd(UB.x)) == 0 && dry_edge_slots<IFLUX>(M.gp, a.flux_mode, geo, sa, dt)) return;
+  HostPair<IFLUX, T> p;
+  side_load(a, M, e, 0, geo, UA, dt, p.s[0]);
+  side_load(a, M, e, 1, geo, UB, dt, p.s[1]);
+  const double4 dk = IFLUX >= 3 ? a.edk[e] : make_double4(0.0, 0.0, 0.0, 0.0);
+  side_stages<IFLUX>(p, a.ilimiteur, dk.x, dk.z, dk.y, dk.w);
+  if (a.flux_mode == 1)
+    for (int k = 0; k < 3; ++k) p.out[1][k] = -p.out[0][k];
+  store_side(sa, p.out[0], geo.z);
+  store_side(sa + 1, p.out[1], geo.z);
 }
 
 /* ---- one element ------------------------------------------------------------------------ */
@@ -1183,7 +1497,7 @@ CF_HD CF_INLINE void friction_terms(const MemberDev& M, double area, double dt, 
     if (normvit > tol) {
       const T p43 = div_rn(p13, q1, yq);     /* q1**(-4/3) */
       if (M.fricimplic == 1) {
-        const T yn = recip(normvit);
+        const auto yn = recip(normvit);
         const T dtgn2h = dt / 2.0 * gp * manning * manning * p43;
         const T af21 = -(7.0 / 3.0 * dtgn2h * vitu * normvit);
         const T af22 = 1.0 + div_rn(dtgn2h * (twice(vitu * vitu) + vitv * vitv), normvit, yn);
@@ -1192,7 +1506,7 @@ CF_HD CF_INLINE void friction_terms(const MemberDev& M, double area, double dt, 
         const T af32 = af23;
         const T af33 = 1.0 + div_rn(dtgn2h * (vitu * vitu + twice(vitv * vitv)), normvit, yn);
         const T detaf = af22 * af33 - af23 * af32;
-        const T yd = recip(detaf);
+        const auto yd = recip(detaf);
         m[0] = div_rn(-(af21 * af33 - af23 * af31), detaf, yd);
         m[1] = div_rn(af33, detaf, yd);
         m[2] = div_rn(-af23, detaf, yd);

@@ -554,6 +554,23 @@ __global__ void __launch_bounds__(256) k_selftest_xd(long long n, unsigned long 
       const unsigned long long r = st_next(s);
       a = xdbl(((r >> 63) << 63) | ((1000ull + (r >> 8) % 40u) << 52) | (A & ((1ull << 52) - 1)));
       b = xdbl((((r >> 62) & 1) << 63) | ((1000ull + (r >> 20) % 40u) << 52) | (B & ((1ull << 52) - 1)));
+      if (r & 0x1000u) {
+        /* a / b within d / (2^55 B) of a midpoint, d odd and small: B odd, 2N + 1 = d / B modulo 2^54
+         * (the inverse by Newton's iteration), so (2N + 1) B = A 2^54 + d */
+        const unsigned long long Bo = B | 1u, d = 2 * ((r >> 13) & 0x3ffu) + 1;
+        unsigned long long inv = Bo;   /* 3 bits */
+        for (int k = 0; k < 5; ++k) inv *= 2 - Bo * inv;
+        const long long sd = (r & 0x800u) ? (long long)d : -(long long)d;
+        const unsigned long long M = (inv * (unsigned long long)sd) & ((1ull << 54) - 1);
+        const unsigned long long l = M * Bo, h = __umul64hi(M, Bo);
+        const unsigned long long ll = l - (unsigned long long)sd;
+        const unsigned long long hh = h - (sd > 0 ? (l < (unsigned long long)sd) : 0u) + (sd < 0 ? (ll < l) : 0u);
+        const unsigned long long A2 = (hh << 10) | (ll >> 54);
+        if (A2 >= (1ull << 52) && A2 < (1ull << 53)) {
+          a = xdbl((1010ull << 52) | (A2 & ((1ull << 52) - 1)));
+          b = xdbl((1005ull << 52) | (Bo & ((1ull << 52) - 1)));
+        }
+      }
     }
     if (mode == 4 && (st_next(s) & 1)) {
       /* sqrt(a) close to a rounding midpoint: the significand of RN((N + 1/2)^2 / 2^(52 + p)),
