@@ -204,95 +204,192 @@ CFD_HD Dual<N> rcbrt(const Dual<N>& x) {
   return r;
 }
 
+/* a b + c in one FP64 instruction (derivatives only: values round every operation) */
+CFD_HD XD<true> xfma(const XD<true>& a, const XD<true>& b, const XD<true>& c) { return XD<true>(fma(a.v, b.v, c.v)); }
+
 /* The transposed edge stage of an interior first-order HLLC edge (IFLUX 1, flux_mode 0): given the
  * adjoint weights w[10] of its two slots (side A: flux 1-3, bed x, y; then side B), the
  * contributions lamA, lamB to the adjoints of (h, hu, hv) of its two elements, i.e. J^T w for the
- * edge's Jacobian J, at a fraction of the cost of differentiating the whole edge in six lanes:
- *   - the change to the edge frame and the hydrostatic reconstruction have closed-form
- *     derivatives (u_n = (hu nx + hv ny) / h, u_t = (hv nx - hu ny) / h; reconstructed depths pass
- *     or are clamped to 0);
- *   - the flux core depends on (hl, ul, hr, ur) and on the tangential velocities only through its
- *     tangential components, which are x1 vl or x1 vr (side A) and y1 vl or y1 vr (side B) with
- *     the region telling which (first_order_flux reports it): the core runs on Dual<4> numbers over
- *     (hl, ul, hr, ur), and the tangential derivatives are x1, y1;
- *   - the bed sources g/2 (ha^2 - h^2) len have closed-form derivatives.
- * The value lanes repeat the step's IEEE operations, so every branch is the forward's.  Returns
- * false, and the caller differentiates the edge in full, where a side's raw and masked depths
- * differ (0 < h <= tolisec; the reference then evaluates the two sides differently). */
+ * edge's Jacobian J, by the chain rule backwards through the flux's own formulas:
+ *   - the rotation of both sides' frame fluxes (x1, x2, x3), with x3 = x1 v in every region, v the
+ *     tangential velocity the region takes;
+ *   - the HLL fluxes N / (s_R - s_L + eps) or the physical flux the region takes;
+ *   - the speeds s_L = u_l - a_l p_l, s_R = u_r + a_r p_r with p = 1 or sqrt((h* + h) h* / 2) / h, and
+ *     the depth h* = (h_l + h_r) / 2 - (u_r - u_l) (h_l + h_r) / (a_l + a_r) / 4; next to a dry side
+ *     s = u -+ a and u +- 2 a of the wet one;
+ *   - the hydrostatic reconstruction (depths pass or are clamped to 0), the change to the edge frame
+ *     (u_n = (hu nx + hv ny) / h, u_t = (hv nx - hu ny) / h) and the bed sources g/2 (ha^2 - h^2) len.
+ * The values repeat the step's IEEE operations (so every branch is the forward's), their products,
+ * quotients and roots on the integer pipes; of the derivatives the multiply-adds are FP64
+ * instructions and the products integer ones.  Returns false, and the caller differentiates the edge
+ * in full, where a side's raw and masked depths differ (0 < h <= tolisec; the reference then evaluates
+ * the two sides differently). */
 CFD_HD bool adj_edge_hllc(const MemberDev& M, const EdgeGeo& G, const double4& UA, const double4& UB, double zml,
                           double zmr, const double w[10], double lamA[3], double lamB[3]) {
-  const double g = M.gp, tolisec = M.tolisec, nx = G.nx, ny = G.ny, len = G.len;
-  /* the comparisons on integer keys (xlt, xeq, and XD<false> for the frame change: the same IEEE
-   * results and the same double arithmetic) keep them off the FP64 pipe that bounds this kernel */
-  const auto kmax = [](double a, double b) { return xlt(a, b) ? b : a; };   /* Fortran max */
-  const double zij = kmax(zml, zmr);
-  XD<false> hl_, ul_, vl_, hr_, ur_, vr_;
-  to_frame(XD<false>(UA.x), XD<false>(UA.y), XD<false>(UA.z), UA.w, nx, ny, tolisec, hl_, ul_, vl_);
-  to_frame(XD<false>(UB.x), XD<false>(UB.y), XD<false>(UB.z), UB.w, nx, ny, tolisec, hr_, ur_, vr_);
-  const double hautl = val(hl_), vitul = val(ul_), vitvl = val(vl_);
-  const double hautr = val(hr_), vitur = val(ur_), vitvr = val(vr_);
-  if (!xeq(hautl, UA.x) || !xeq(hautr, UB.x)) return false;
+  typedef XD<true> X;
+  const double g = M.gp, tolisec = M.tolisec, nx = G.nx, ny = G.ny, eps = EPS_HLLC;
+  const X hA(UA.x), hB(UB.x);
+  const bool wa = hA > tolisec, wb = hB > tolisec;   /* frame velocities differentiable */
+  if ((!wa && hA != 0.0) || (!wb && hB != 0.0)) return false;
+  const double zij = val(dmax(X(zml), X(zmr)));
+  X hm, ul, vl, ur, vr;
+  to_frame(hA, X(UA.y), X(UA.z), UA.w, nx, ny, tolisec, hm, ul, vl);
+  to_frame(hB, X(UB.y), X(UB.z), UB.w, nx, ny, tolisec, hm, ur, vr);
+  const X ul0 = ul, vl0 = vl, ur0 = ur, vr0 = vr;
   /* hydrostatic reconstruction (flux_riemann.cuf:176-181, :200-210); which variables carry a
    * derivative (a clamped or masked one is a constant of the inputs) */
-  const double el = hautl + zml - zij, er = UB.x + zmr - zij;
-  double hl = kmax(0.0, el), hr = kmax(0.0, er);
-  double ul = vitul, vl = vitvl, ur = vitur, vr = vitvr;
-  const bool pl = !xlt(hl, tolisec), pr = !xlt(hr, tolisec);
-  if (!pl) { hl = 0.; ul = 0.; vl = 0.; }
-  if (!pr) { hr = 0.; ur = 0.; vr = 0.; }
-  const bool wa = xlt(tolisec, UA.x), wb = xlt(tolisec, UB.x);   /* frame velocities differentiable */
-  const bool s_hl = pl && xlt(0.0, el), s_ul = pl && wa, s_hr = pr && xlt(0.0, er), s_ur = pr && wb;
-  const Dual<4> Hl = s_hl ? Dual<4>::var(hl, 0) : Dual<4>(hl), Ul = s_ul ? Dual<4>::var(ul, 1) : Dual<4>(ul);
-  const Dual<4> Hr = s_hr ? Dual<4>::var(hr, 2) : Dual<4>(hr), Ur = s_ur ? Dual<4>::var(ur, 3) : Dual<4>(ur);
-  TwoFluxT<Dual<4>> F;
-  HllcRegions rg;
-  first_order_flux<1>(g, nx, ny, Hl, Ul, Dual<4>(vl), Hr, Ur, Dual<4>(vr), F, &rg);
-  /* w^T d(slot fluxes)/d(hl, ul, hr, ur): the slots hold F * len */
-  double gc[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-    gc[i] = len * (w[0] * F.a1.d[i] + w[1] * F.a2.d[i] + w[2] * F.a3.d[i] + w[5] * F.b1.d[i] + w[6] * F.b2.d[i] +
-                   w[7] * F.b3.d[i]);
-  /* tangential velocities: a2 = nx x2 - ny x3, a3 = ny x2 + nx x3 with x3 = x1 v (x1 = a1);
-   * b2 = -(nx y2 - ny y3), b3 = -(ny y2 + nx y3) with y3 = y1 v (y1 = -b1) */
-  double gvl = 0.0, gvr = 0.0;
-  if (rg.valid) {
-    const double ga = len * (w[2] * nx - w[1] * ny) * F.a1.v;
-    const double gb = len * (w[7] * nx - w[6] * ny) * F.b1.v;   /* (ny w6 - nx w7) y1 with y1 = -b1 */
-    if (rg.a_vr) gvr += ga; else gvl += ga;
-    if (rg.b_vr) gvr += gb; else gvl += gb;
+  const X ea = hA + zml - zij, eb = hB + zmr - zij;
+  const X ha = dmax0(ea), hb = dmax0(eb);
+  X hl = wa ? ha : X(0.0), hr = hb;
+  const bool pl = !(hl < tolisec), pr = !(hr < tolisec);
+  if (!pl) { hl = X(0.); ul = X(0.); vl = X(0.); }
+  if (!pr) { hr = X(0.); ur = X(0.); vr = X(0.); }
+  const bool s_hl = pl && wa && ea > 0., s_ul = pl && wa, s_hr = pr && eb > 0., s_ur = pr && wb;
+  X ghl(0.0), gul(0.0), gvl(0.0), ghr(0.0), gur(0.0), gvr(0.0);   /* adjoints (without the factor len) */
+  if (!(hl < eps && hr < eps)) {
+    /* the flux's values, as wave_speeds and first_order_flux<1> form them */
+    const X gl = g * hl, gr = g * hr, al = sqrt(gl), ar = sqrt(gr);
+    const X hs = hl + hr, du = ur - ul, as = al + ar;
+    const X qd = du * hs / as;
+    const X het = halve(hs) - quarter(qd);
+    const bool wl = hl > eps, wr = hr > eps, both = wl && wr;
+    const bool kl = both && !lt_nonneg(het, hl), kr = both && !lt_nonneg(het, hr);
+    const X hll2 = hl * hl, hrr2 = hr * hr;
+    const X pql = kl ? sqrt(halve(het + hl) * het / hll2) : X(1.), pqr = kr ? sqrt(halve(het + hr) * het / hrr2) : X(1.);
+    X sl, sr;
+    if (wl) {
+      sl = ul - (both ? al * pql : al);
+      sr = wr ? ur + ar * pqr : ul + twice(al);
+    } else {
+      sl = ur - twice(ar);
+      sr = ur + ar;
+    }
+    const X fl1 = hl * ul, fl2 = hl * (ul * ul) + halve(gl * hl);
+    const X fr1 = hr * ur, fr2 = hr * (ur * ur) + halve(gr * hr);
+    const int ra = (sl > 0.) ? 0 : ((sr < 0.) ? 1 : 2);
+    const int rb = (sr < 0.) ? 1 : ((sl > 0.) ? 0 : 2);
+    /* s* decides which tangential velocity the HLL region carries */
+    bool right_a = ra == 1, right_b = rb == 1;
+    if (ra == 2 || rb == 2) {
+      const X d1 = hr * (ur - sr), d0 = hl * (ul - sl), denom = d1 - d0;
+      X set;
+      if (fabs(denom) < eps) set = halve(ul + ur) - (hr - hl) * as / hs;
+      else set = (sl * hr * (ur - sr) - sr * hl * (ul - sl)) / denom;
+      if (ra == 2) right_a = !(set > 0.);
+      if (rb == 2) right_b = set < 0.;
+    }
+    /* adjoints of x1, x2 (side A) and y1, y2 (side B, whose frame flux is (-y1, y2, y1 v) mirrored) */
+    const X ta = xfma(X(w[2]), X(nx), -(X(w[1]) * ny)), tb = xfma(X(w[7]), X(nx), -(X(w[6]) * ny));
+    const X ga2 = xfma(X(w[1]), X(nx), X(w[2]) * ny), gb2 = -xfma(X(w[6]), X(nx), X(w[7]) * ny);
+    const X ga1 = xfma(right_a ? vr : vl, ta, X(w[0])), gb1 = -xfma(right_b ? vr : vl, tb, X(w[5]));
+    X gfl1(0.0), gfl2(0.0), gfr1(0.0), gfr2(0.0), gsl(0.0), gsr(0.0), m1(0.0);
+    if (ra == 2 || rb == 2) {
+      const X gh1 = (ra == 2 && rb == 2) ? ga1 + gb1 : (ra == 2 ? ga1 : gb1);
+      const X gh2 = (ra == 2 && rb == 2) ? ga2 + gb2 : (ra == 2 ? ga2 : gb2);
+      const X y = 1.0 / (sr - sl + eps);
+      const X dh = hr - hl, df = fr1 - fl1, ss = sl * sr;
+      const X c1 = xfma(sl, dh, fl1), c2 = xfma(sl, df, fl2), e1 = xfma(sr, dh, -fr1), e2 = xfma(sr, df, -fr2);
+      m1 = xfma(sr, c1, -(sl * fr1)) * y;
+      const X m2 = xfma(sr, c2, -(sl * fr2)) * y;
+      const X n1 = gh1 * y, n2 = gh2 * y;
+      const X gd = -xfma(n1, m1, n2 * m2);
+      gsr = xfma(n1, c1, xfma(n2, c2, gd));
+      gsl = xfma(n1, e1, xfma(n2, e2, -gd));
+      const X q1 = n1 * ss, q2 = n2 * ss;
+      gfl1 = xfma(n1, sr, -q2);
+      gfr1 = xfma(-n1, sl, q2);
+      gfl2 = n2 * sr;
+      gfr2 = -(n2 * sl);
+      ghl = -q1;
+      ghr = q1;
+    }
+    if (ra == 0) { gfl1 = gfl1 + ga1; gfl2 = gfl2 + ga2; }
+    if (ra == 1) { gfr1 = gfr1 + ga1; gfr2 = gfr2 + ga2; }
+    if (rb == 0) { gfl1 = gfl1 + gb1; gfl2 = gfl2 + gb2; }
+    if (rb == 1) { gfr1 = gfr1 + gb1; gfr2 = gfr2 + gb2; }
+    /* tangential velocities: x1 ta on side A, -y1 tb on side B */
+    const X va = (ra == 0 ? fl1 : (ra == 1 ? fr1 : m1)) * ta, vb = -((rb == 0 ? fl1 : (rb == 1 ? fr1 : m1)) * tb);
+    if (right_a == right_b) (right_a ? gvr : gvl) = va + vb;
+    else { gvl = right_a ? vb : va; gvr = right_a ? va : vb; }
+    /* physical fluxes: f1 = h u, f2 = h u^2 + g h^2 / 2 */
+    ghl = xfma(gfl1, ul, xfma(gfl2, xfma(ul, ul, gl), ghl));
+    gul = xfma(gfl1, hl, twice(gfl2 * fl1));
+    ghr = xfma(gfr1, ur, xfma(gfr2, xfma(ur, ur, gr), ghr));
+    gur = xfma(gfr1, hr, twice(gfr2 * fr1));
+    /* speeds */
+    X gal(0.0), gar(0.0);
+    if (both) {
+      gul = gul + gsl;
+      gur = gur + gsr;
+      gal = -(gsl * pql);
+      gar = gsr * pqr;
+      if (kl || kr) {
+        /* p^2 = P = (h* + h) h* / 2 / h^2: dP/dh* = (h* + h / 2) / h^2, dP/dh = (h* / 2 - 2 P h) / h^2 */
+        X ghet(0.0);
+        if (kl) {
+          const X gp = -(gsl * al) / (twice(pql) * hll2);
+          ghet = gp * (het + halve(hl));
+          ghl = xfma(gp, xfma(-twice(pql * pql), hl, halve(het)), ghl);
+        }
+        if (kr) {
+          const X gp = gsr * ar / (twice(pqr) * hrr2);
+          ghet = xfma(gp, het + halve(hr), ghet);
+          ghr = xfma(gp, xfma(-twice(pqr * pqr), hr, halve(het)), ghr);
+        }
+        /* h* */
+        const X q = quarter(ghet) / as;
+        const X dq = q * du, uq = q * hs, aq = q * qd;
+        const X gh = halve(ghet) - dq;
+        ghl = ghl + gh;
+        ghr = ghr + gh;
+        gul = gul + uq;
+        gur = gur - uq;
+        gal = gal + aq;
+        gar = gar + aq;
+      }
+    } else if (wl) {
+      gul = gul + gsl + gsr;
+      gal = twice(gsr) - gsl;
+    } else {
+      gur = gur + gsl + gsr;
+      gar = gsr - twice(gsl);
+    }
+    /* celerities a = sqrt(g h): da/dh = g / (2 a) */
+    const double hg = ConstOps<X>::half(g);
+    if (wl) ghl = ghl + gal * hg / al;
+    if (wr) ghr = ghr + gar * hg / ar;
   }
-  /* to the conserved variables: d(h_m, u_n, u_t)/d(h, hu, hv) with y = RN(1/h) */
-  lamA[0] = lamA[1] = lamA[2] = 0.0;
-  lamB[0] = lamB[1] = lamB[2] = 0.0;
+  /* to the conserved variables: d(h_m, u_n, u_t)/d(h, hu, hv) with y = RN(1/h); the bed sources
+   * (source_terms.cuf:90-97): ta = g/2 (ha^2 - hA^2) len into (ta nx, ta ny) of side A, tb likewise
+   * into -(tb nx, tb ny) of side B */
+  const double len = G.len;
   {
-    const double gh = s_hl ? gc[0] : 0.0, gu = s_ul ? gc[1] : 0.0, gv = s_ul ? gvl : 0.0;
+    const X gu = s_ul ? gul : X(0.0), gv = s_ul ? gvl : X(0.0);
+    X gh = s_hl ? ghl : X(0.0);
+    gh = xfma(xfma(X(w[3]), X(nx), X(w[4]) * ny) * g, (ea > 0. ? ha : X(0.0)) - hA, gh);
+    const X y = len * X(UA.w);
+    lamA[0] = lamA[1] = lamA[2] = 0.0;
     if (wa) {
-      const double y = UA.w;
-      lamA[0] = gh - (gu * vitul + gv * vitvl) * y;
-      lamA[1] = (gu * nx - gv * ny) * y;
-      lamA[2] = (gu * ny + gv * nx) * y;
+      lamA[0] = val(xfma(gh, X(len), -(xfma(gu, ul0, gv * vl0) * y)));
+      lamA[1] = val(xfma(gu, X(nx), -(gv * ny)) * y);
+      lamA[2] = val(xfma(gu, X(ny), gv * nx) * y);
+    } else {
+      lamA[0] = val(gh * len);
     }
   }
   {
-    const double gh = s_hr ? gc[2] : 0.0, gu = s_ur ? gc[3] : 0.0, gv = s_ur ? gvr : 0.0;
-    lamB[0] = gh;   /* the B side reconstructs from the raw depth */
+    const X gu = s_ur ? gur : X(0.0), gv = s_ur ? gvr : X(0.0);
+    X gh = s_hr ? ghr : X(0.0);   /* the B side reconstructs from the raw depth */
+    gh = xfma(-(xfma(X(w[8]), X(nx), X(w[9]) * ny) * g), (eb > 0. ? hb : X(0.0)) - hB, gh);
+    const X y = len * X(UB.w);
+    lamB[0] = lamB[1] = lamB[2] = 0.0;
     if (wb) {
-      const double y = UB.w;
-      lamB[0] -= (gu * vitur + gv * vitvr) * y;
-      lamB[1] = (gu * nx - gv * ny) * y;
-      lamB[2] = (gu * ny + gv * nx) * y;
+      lamB[0] = val(xfma(gh, X(len), -(xfma(gu, ur0, gv * vr0) * y)));
+      lamB[1] = val(xfma(gu, X(nx), -(gv * ny)) * y);
+      lamB[2] = val(xfma(gu, X(ny), gv * nx) * y);
+    } else {
+      lamB[0] = val(gh * len);
     }
-  }
-  /* bed sources (source_terms.cuf:90-97): ta = g/2 (ha^2 - hA^2) len into (ta nx, ta ny) of
-   * side A, tb likewise into -(tb nx, tb ny) of side B */
-  {
-    const double ea = UA.x + zml - zij, eb = UB.x + zmr - zij;
-    const double ha = kmax(0.0, ea), hb = kmax(0.0, eb);
-    const double dta = g / 2.0 * (2.0 * (xlt(0.0, ea) ? ha : 0.0) - 2.0 * UA.x) * len;
-    const double dtb = g / 2.0 * (2.0 * (xlt(0.0, eb) ? hb : 0.0) - 2.0 * UB.x) * len;
-    lamA[0] += (w[3] * nx + w[4] * ny) * dta;
-    lamB[0] -= (w[8] * nx + w[9] * ny) * dtb;
   }
   return true;
 }
