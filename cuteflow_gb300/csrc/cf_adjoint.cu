@@ -23,7 +23,7 @@
  * floors, the wet/dry clamp of the update) is the one the forward took.  For an edge the D
  * derivative lanes run in chunks over its 6 (first order) or 10 (WAF: + the upwind
  * reconstructions) inputs; D trades registers for repeated value lanes.  The element stage
- * is linear in the sums and is transposed by hand around a Dual<4> friction block.
+ * is transposed by hand (adj_element), and so is the first-order HLLC edge (adj_edge_hllc).
  *
  * Replay kernels (k_rep_edges, k_rep_cells) advance a state with a recorded dt / time
  * sequence; they run the step's own edge_lanes / element_update, so a replayed trajectory is
@@ -145,14 +145,13 @@ __device__ __forceinline__ double4 gather_lambda(const AdjArgs& A, int c, const 
   return L;
 }
 
-/* The element update is linear in its flux and bed sums: U^{n+1} = q + dt R (S + sf(q, n) - rc)
- * / area (R = I, or the semi-implicit matrix of rows (1, 0, 0), (m4, m5, m6), (m7, m8, m9)),
- * then the wet/dry clamp.  Its transpose is applied by hand; only the friction block
- * (q1, q2, q3, n) -> (sf2, sf3, m4..m9) is differentiated with Dual<4> numbers of the step's own
- * friction_terms.  128-thread blocks capped at 168 registers: three blocks per SM (a 256-thread
- * block at its 170 registers left room for one). */
+/* The transposed element stage (adj_element) of every element, with lambda gathered first.  Its values
+ * and lone products run on the integer pipes, its sums and multiply-adds on the FP64 pipe: ~60 FP64
+ * instructions per element, 243 while the friction ran on four dual lanes (51k triangles, with the
+ * reverse edge at its own four blocks: backward and forward of 50 steps 5.9 -> 4.8 ms).  Five, six and
+ * eight blocks per SM measure the same within 3 %. */
 constexpr int ADJ_CELLS_BLOCK = 128;
-__global__ void __launch_bounds__(ADJ_CELLS_BLOCK, 3) k_adj_cells(AdjArgs A) {
+__global__ void __launch_bounds__(ADJ_CELLS_BLOCK, 6) k_adj_cells(AdjArgs A) {
   const StepArgs& a = A.s;
   const int c = blockIdx.x * ADJ_CELLS_BLOCK + threadIdx.x;
   const int mem = __ldg(a.ctile_mem + c / TILE_C);
@@ -160,69 +159,13 @@ __global__ void __launch_bounds__(ADJ_CELLS_BLOCK, 3) k_adj_cells(AdjArgs A) {
   if (c >= M.cell_end) return;
   const double4 L = A.gather ? gather_lambda(A, c, A.gw) : ld4(A.lam_init + c);
   const double dt = __ldg(A.dt_hist + hidx(A.n, mem, a.nmembers));
-  const double4 U = ld4(a.Uin + c);
-  const double4 st = ld4(a.cstat + c);
-  const double2* sp = reinterpret_cast<const double2*>(A.sums + c);
-  const double2 sa = __ldg(sp), sb = __ldg(sp + 1), sc = __ldg(sp + 2);
-  const double rc1 = sa.x, rc2 = sa.y, rc3 = sb.x, sb2 = sb.y, sb3 = sc.x;
-  const double area = st.x, y = st.w;
-  const bool fric = M.friction == 1;
-  const bool impl = fric && (M.fricimplic == 1 || M.fricimplic == 2);
-  Dual<4> sf2(0.0), sf3(0.0), m[6];
-  double r1, ri1, ri2, ri3;
-  if (fric) {
-    friction_terms(M, area, dt, Dual<4>::var(st.y, 3), Dual<4>::var(U.x, 0), Dual<4>::var(U.y, 1),
-                   Dual<4>::var(U.z, 2), sf2, sf3, m, U.w);
-    ri1 = div_rn(0. + 0. - rc1, area, y);
-    ri2 = div_rn(sb2 + sf2.v - rc2, area, y);
-    ri3 = div_rn(sb3 + sf3.v - rc3, area, y);
-    r1 = impl ? 1. * ri1 + 0. * ri2 + 0. * ri3 : ri1;
-  } else {
-    ri1 = div_rn(0. - rc1, area, y);
-    ri2 = div_rn(sb2 - rc2, area, y);
-    ri3 = div_rn(sb3 - rc3, area, y);
-    r1 = ri1;
-  }
-  const double h = U.x + dt * r1;
-  double4 own = make_double4(0.0, 0.0, 0.0, 0.0);
+  const Slot sums = load_slot_adj(A.sums + c);
+  double4 own;
   Slot w;
-  w.f1 = w.f2 = w.f3 = w.bx = w.by = w.q = 0.0;
-  double nb = 0.0;
-  if (!(h <= M.tolisec)) {   /* a clamped element is a constant of its inputs */
-    own = make_double4(L.x, L.y, L.z, 0.0);
-    const double r1b = dt * L.x, r2b = dt * L.y, r3b = dt * L.z;
-    double ri1b = r1b, ri2b = r2b, ri3b = r3b;
-    if (impl) {
-      ri1b = r1b + r2b * m[0].v + r3b * m[3].v;
-      ri2b = r2b * m[1].v + r3b * m[4].v;
-      ri3b = r2b * m[2].v + r3b * m[5].v;
-    }
-    w.f1 = -ri1b * y;
-    w.f2 = -ri2b * y;
-    w.f3 = -ri3b * y;
-    w.bx = ri2b * y;
-    w.by = ri3b * y;
-    if (fric) {
-      const double sf2b = ri2b * y, sf3b = ri3b * y;
-      const double mb[6] = {r2b * ri1, r2b * ri2, r2b * ri3, r3b * ri1, r3b * ri2, r3b * ri3};
-      double g[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        double v = sf2b * sf2.d[k] + sf3b * sf3.d[k];
-        if (impl) {
-#pragma unroll
-          for (int j = 0; j < 6; ++j) v = fma(mb[j], m[j].d[k], v);
-        }
-        g[k] = v;
-      }
-      own.x += g[0];
-      own.y += g[1];
-      own.z += g[2];
-      nb = g[3];
-    }
-  }
+  double nb;
+  adj_element(M, ld4(a.Uin + c), ld4(a.cstat + c), sums, L, dt, own, w, nb);
   A.lam_own[c] = own;
-  A.cadj[c] = w;
+  store_slot(A.cadj + c, w.f1, w.f2, w.f3, w.bx, w.by, w.q);
   A.gman[c] += nb;
 }
 
@@ -332,11 +275,12 @@ __global__ void __launch_bounds__(TILE_E) k_adj_edges(AdjArgs A) {
   else adj_interior_edge<IFLUX, D>(A, M, e, ab, dt);
 }
 
-/* First-order HLLC (flux_mode 0): the closed-form reverse edge (adj_edge_hllc: frame change,
- * reconstruction, tangential velocities and bed sources by hand around a Dual<4> flux core) for
- * every interior edge it covers, at three blocks per SM; the edges it leaves (a nearly dry side
- * whose raw and masked depths differ) are queued for k_adj_edges_rest. */
-__global__ void __launch_bounds__(TILE_E, 3) k_adj_edges_hllc(AdjArgs A) {
+/* First-order HLLC (flux_mode 0): the closed-form reverse edge (adj_edge_hllc) for every interior edge
+ * it covers; the edges it leaves (a nearly dry side whose raw and masked depths differ) are queued for
+ * k_adj_edges_rest.  Four blocks per SM (128 registers): 51k triangles, 51.6 us at three, 38.2 at four,
+ * 39.7 at five, 40.0 at six; 339 us per reverse step of 200k triangles while the flux ran on four dual
+ * lanes. */
+__global__ void __launch_bounds__(TILE_E, 4) k_adj_edges_hllc(AdjArgs A) {
   const StepArgs& a = A.s;
   const int tile = blockIdx.x;
   const int m = __ldg(a.etile_mem + tile);

@@ -394,6 +394,98 @@ CFD_HD bool adj_edge_hllc(const MemberDev& M, const EdgeGeo& G, const double4& U
   return true;
 }
 
+/* The transposed element stage (element_core): given the adjoint L of an element's new state, its old
+ * state U, its statics st = {area, n, -, RN(1/area)} and its flux and bed sums s, the adjoint own of
+ * its old state (besides what comes through its edges), w of its sums and nb of its Manning n, by the
+ * chain rule backwards through the formulas of friction_terms and element_core:
+ *   - the update q + dt r and the clamp (a clamped element is a constant of its inputs);
+ *   - r = R ri with ri = (S + sf - rc) / area, R = I or the semi-implicit matrix.  With fricimplic 1
+ *     (r2, r3) solves A (r2, r3) = (ri2, ri3) - (a21, a31) ri1 with the symmetric A of entries 1 + A22,
+ *     a23, 1 + A33, so with (s2, s3) = A^-1 (r2', r3') the adjoint of an entry a_ij is -s_i r_j;
+ *   - all of a21, a31 are n^2 q1^(-4/3) |v| times a velocity, A22, A33, a23 the same over |v| times a
+ *     product of two, sf = -g n^2 area q1^(-1/3) |v| v: their logarithmic derivatives are the same
+ *     sums S, W, Z, F for every factor.
+ * Only the clamp depends on a value to the last bit; that value (h = q1 + dt ri1) is the step's. */
+CFD_HD void adj_element(const MemberDev& M, const double4& U, const double4& st, const Slot& s, const double4& L,
+                        double dt, double4& own, Slot& w, double& nb) {
+  typedef XD<true> X;
+  const double area = st.x, ya = st.w;
+  own = make_double4(0.0, 0.0, 0.0, 0.0);
+  w.f1 = w.f2 = w.f3 = w.bx = w.by = w.q = 0.0;
+  nb = 0.0;
+  const bool fric = M.friction == 1;
+  const X ri1 = div_rn(fric ? 0. + 0. - X(s.f1) : 0. - X(s.f1), area, ya);
+  if (X(U.x) + dt * ri1 <= M.tolisec) return;
+  const X q1(U.x), n(st.y), r1b = dt * X(L.x), r2b = dt * X(L.y), r3b = dt * X(L.z);
+  const bool wet = fric && q1 > M.tolisec;
+  X u(0.0), v(0.0), nv(0.0), iv(0.0), sf2(0.0), sf3(0.0), c(0.0), p13(0.0);
+  bool fast = false;   /* |v| > tol: the matrix differs from the identity */
+  if (wet) {
+    u = div_rn(X(U.y), q1, X(U.w));
+    v = div_rn(X(U.z), q1, X(U.w));
+    nv = sqrt(u * u + v * v);
+    const bool held = nv < M.tol;   /* a constant of the inputs then, as where it is 0 */
+    if (held) nv = X(M.tol);
+    else if (nv > 0.) iv = 1.0 / nv;
+    fast = nv > M.tol;
+    p13 = rcbrt(q1);
+    c = M.gp * n * n * nv * area * p13;
+    sf2 = -(c * u);
+    sf3 = -(c * v);
+  }
+  X s2 = r2b, s3 = r3b, ri1b = r1b, ub(0.0), vb(0.0), nvb(0.0), S(0.0);
+  if (fast && (M.fricimplic == 1 || M.fricimplic == 2)) {
+    const X ri2 = div_rn(s.bx + sf2 - s.f2, area, ya), ri3 = div_rn(s.by + sf3 - s.f3, area, ya);
+    const X d = ConstOps<X>::half(dt) * M.gp * n * n * p13 * U.w;
+    if (M.fricimplic == 1) {
+      const X e = d * iv, dn = (7.0 / 3.0) * d * nv;
+      const X uu = u * u, vv = v * v;
+      const X A22 = e * xfma(u, u, uu + vv), A33 = e * xfma(v, v, uu + vv), a23 = e * (u * v);
+      const X a22 = 1. + A22, a33 = 1. + A33;
+      const X id = 1.0 / xfma(a22, a33, -(a23 * a23));
+      s2 = xfma(a33, r2b, -(a23 * r3b)) * id;
+      s3 = xfma(a22, r3b, -(a23 * r2b)) * id;
+      const X m1 = dn * ri1, t2 = xfma(m1, u, ri2), t3 = xfma(m1, v, ri3);
+      const X r2 = xfma(a33, t2, -(a23 * t3)) * id, r3 = xfma(a22, t3, -(a23 * t2)) * id;
+      const X us = xfma(u, s2, v * s3);
+      ri1b = xfma(dn, us, r1b);
+      const X b22 = -(s2 * r2), b33 = -(s3 * r3), b23 = -xfma(s2, r3, s3 * r2);
+      /* b21 a21 + b31 a31 = ri1 dn (u s2 + v s3) */
+      const X Z = m1 * us, W = xfma(b22, A22, xfma(b33, A33, b23 * a23));
+      S = Z + W;
+      nvb = (Z - W) * iv;
+      ub = xfma(m1, s2, e * xfma(twice(u), twice(b22) + b33, v * b23));
+      vb = xfma(m1, s3, e * xfma(twice(v), twice(b33) + b22, u * b23));
+    } else {
+      const X beta = -(twice(d) * nv), im = 1.0 / (1. - beta);
+      s2 = r2b * im;
+      s3 = r3b * im;
+      S = xfma(s2, ri2, s3 * ri3) * beta * im;
+      nvb = S * iv;
+    }
+  }
+  const X s2y = s2 * ya, s3y = s3 * ya;
+  w.f1 = val(-(ri1b * ya));
+  w.f2 = val(-s2y);
+  w.f3 = val(-s3y);
+  w.bx = val(s2y);
+  w.by = val(s3y);
+  own = L;
+  own.w = 0.0;
+  if (wet) {
+    const X F = xfma(sf2, s2y, sf3 * s3y);
+    const X g = xfma(F, iv, nvb) * iv;   /* adjoint of |v| over |v| */
+    ub = xfma(-c, s2y, xfma(g, u, ub));
+    vb = xfma(-c, s3y, xfma(g, v, vb));
+    const X k = xfma(ub, u, xfma(vb, v, xfma(X(4.0), S, F) * (1.0 / 3.0)));
+    const X y(U.w);
+    own.x = val(xfma(-k, y, X(L.x)));
+    own.y = val(xfma(ub, y, X(L.y)));
+    own.z = val(xfma(vb, y, X(L.z)));
+    nb = n != 0.0 ? val(twice(F + S) / n) : 0.0;
+  }
+}
+
 }  // namespace cf
 
 #endif

@@ -1,0 +1,53 @@
+/*
+ * element_harness.cpp -- TEST INFRASTRUCTURE.  The transposed element stage of the reverse sweep
+ * (adj_element in cf_dual.h) against the element stage differentiated in nine Dual lanes, on the CPU.
+ */
+#include "../cuteflow_gb300/csrc/cf_dual.h"
+
+#include <cmath>
+
+using namespace cf;
+
+/* The largest difference relative to the element's largest contribution, over n random elements of one
+ * friction option: depths around the dry threshold and up, velocities at rest, around the floor tol and
+ * up, clamped and free updates, a zero Manning n. */
+extern "C" double harness_adj_element(long long n, unsigned long long seed, int friction, int fricimplic) {
+  unsigned long long s = seed | 1;
+  auto rnd = [&]() { s ^= s << 13; s ^= s >> 7; s ^= s << 17; return s; };
+  auto unif = [&]() { return (double)(rnd() >> 11) * (1.0 / 9007199254740992.0); };
+  auto sym = [&]() { return 2.0 * unif() - 1.0; };
+  typedef Dual<9> D;
+  double worst = 0.0;
+  for (long long i = 0; i < n; ++i) {
+    MemberDev M;
+    std::memset(&M, 0, sizeof(M));
+    M.gp = 9.81; M.tolisec = 1e-4; M.tol = (double)1e-6f; M.friction = friction; M.fricimplic = fricimplic;
+    const double h = rnd() % 5 == 0 ? 2e-4 * unif() : 0.01 + 3.0 * unif();
+    const double vel = rnd() % 4 == 0 ? 0.0 : (rnd() % 4 == 0 ? 3e-6 : 2.0);
+    const double4 U = make_double4(h, h * vel * sym(), h * vel * sym(), h > 0.0 ? 1.0 / h : 0.0);
+    const double area = 0.5 + 3.0 * unif();
+    const double4 st = make_double4(area, rnd() % 16 == 0 ? 0.0 : 0.01 + 0.05 * unif(), 0.0, 1.0 / area);
+    Slot q;
+    q.f1 = sym() * (rnd() % 3 == 0 ? 10.0 : 0.5); q.f2 = sym(); q.f3 = sym(); q.bx = sym(); q.by = sym(); q.q = 0.0;
+    const double4 L = make_double4(sym(), sym(), sym(), 0.0);
+    const double dt = 0.2 * unif();
+    double4 own;
+    Slot w;
+    double nb;
+    adj_element(M, U, st, q, L, dt, own, w, nb);
+    D H, HU, HV;
+    bool nf;
+    element_core(M, area, st.w, D::var(st.y, 8), D::var(U.x, 0), D::var(U.y, 1), D::var(U.z, 2), D::var(q.f1, 3),
+                 D::var(q.f2, 4), D::var(q.f3, 5), D::var(q.bx, 6), D::var(q.by, 7), dt, H, HU, HV, nf, U.w);
+    const double got[9] = {own.x, own.y, own.z, w.f1, w.f2, w.f3, w.bx, w.by, nb};
+    double err = 0.0, top = 1e-30;
+    for (int k = 0; k < 9; ++k) {
+      const double want = L.x * H.d[k] + L.y * HU.d[k] + L.z * HV.d[k];
+      err = std::fmax(err, std::fabs(got[k] - want));
+      top = std::fmax(top, std::fabs(want));
+      if (!(got[k] == got[k])) return INFINITY;
+    }
+    worst = std::fmax(worst, err / top);
+  }
+  return worst;
+}
