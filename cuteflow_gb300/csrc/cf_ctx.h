@@ -65,8 +65,12 @@ struct cf_ctx {
   bool any_phys_inflow = false;        /* some member has inlet 3 */
   bool any_steady = false;             /* some member tests for steady state */
   int32_t* ids = nullptr;              /* max_n element ids (cf_get_elements / cf_set_elements) */
-  int32_t xd_cmp = 0;                  /* edge kernel: integer comparisons (cf_set_tuning) */
-  int32_t xd_mul_mask = 0;             /* edge kernel: warps multiplying on the integer pipes */
+  /* how the FP64 work is shared (cf_set_tuning): from the start everything but the sums on the integer
+   * pipes, in every edge warp and in the element kernel.  It is the faster setting at every size and
+   * scheme (all on the FP64 pipe / this, us per step: 1.4k triangles 28.0 / 24.9, dam break 80k 111 /
+   * 46, WAF 25k 51 / 35, descent of 22k 191 / 160), so that a caller who does not tune has it too. */
+  int32_t xd_cmp = 1;                  /* integer comparisons */
+  int32_t xd_mul_mask = 0x1f;          /* warps multiplying on the integer pipes, XD_CELLS */
   /* launch shape (cf_set_launch_shape): the autotuner's usual choice on the 1M WAF step, 2-3 %
    * faster there than (128, 1, 256) */
   int32_t eblock = 256, ept = 1;       /* edge kernel: threads per block, edges per thread */
