@@ -127,6 +127,13 @@ struct ConstOps {
   static CF_HD CF_INLINE double dbl(double x) { return x * 2.0; }
 };
 
+/* 0 - x, and the first row (1, 0, 0) of the semi-implicit matrix applied to (a, b, c); cf_xd.h forms
+ * them for its type without the arithmetic where that does not change the value */
+template <class T>
+CF_HD CF_INLINE T zero_minus(const T& x) { return 0. - x; }
+template <class T>
+CF_HD CF_INLINE T first_row(const T& a, const T& b, const T& c) { return 1. * a + 0. * b + 0. * c; }
+
 /* RN(1/d) of a denominator that several quotients share (div_rn) */
 template <class T>
 CF_HD CF_INLINE T recip(const T& d) { return 1.0 / d; }
@@ -177,6 +184,10 @@ CF_HD CF_INLINE double ConstOps<T>::quot(double a, double d, double y) { return 
  * reaches y; then the final rounding); measured within 1 ulp of the exact value (tests).  Seven
  * FP64-pipe instructions.  Zero, subnormal, infinite, negative and NaN x (never reached by the
  * step, whose depths here exceed tolisec > 0) take rcbrt_special. */
+struct MulFp64 {
+  static CF_HD CF_INLINE double mul(double a, double b) { return a * b; }
+};
+template <class P = MulFp64>
 CF_HD CF_INLINE double rcbrt_core(uint64_t b) {
   const uint32_t ex = (uint32_t)(b >> 52);
   const uint32_t ep = ex + 177u;            /* unbiased exponent + 1200 */
@@ -196,8 +207,8 @@ CF_HD CF_INLINE double rcbrt_core(uint64_t b) {
   const float e32 = fmaf(-mf, y * y * y, 1.0f);
   y = fmaf(y, e32 * 0x1.555556p-2f, y);
   const double yd = (double)y;
-  const double e = fma(-m, yd * yd * yd, 1.0);
-  const double c = e * fma(e, 2.0 / 9.0, 1.0 / 3.0);
+  const double e = fma(-m, P::mul(P::mul(yd, yd), yd), 1.0);
+  const double c = P::mul(e, fma(e, 2.0 / 9.0, 1.0 / 3.0));
   const double res = fma(yd, c, yd);
   uint64_t rb;
   memcpy(&rb, &res, sizeof(rb));
@@ -225,12 +236,14 @@ CF_HD CF_INLINE double rcbrt_special(double x) {
   return rcbrt_core(b) * 0x1p18;
 }
 
-CF_HD CF_INLINE double rcbrt(double x) {
+template <class P = MulFp64>
+CF_HD CF_INLINE double rcbrt_of(double x) {
   uint64_t b;
   memcpy(&b, &x, sizeof(b));
   if ((uint32_t)(b >> 52) - 1u >= 2046u) return rcbrt_special(x);
-  return rcbrt_core(b);
+  return rcbrt_core<P>(b);
 }
+CF_HD CF_INLINE double rcbrt(double x) { return rcbrt_of(x); }
 
 /* ---- edge-frame states ------------------------------------------------------------------ */
 
@@ -1498,7 +1511,7 @@ CF_HD CF_INLINE void friction_terms(const MemberDev& M, double area, double dt, 
       const T p43 = div_rn(p13, q1, yq);     /* q1**(-4/3) */
       if (M.fricimplic == 1) {
         const auto yn = recip(normvit);
-        const T dtgn2h = dt / 2.0 * gp * manning * manning * p43;
+        const T dtgn2h = T(ConstOps<T>::half(dt)) * gp * manning * manning * p43;
         const T af21 = -(7.0 / 3.0 * dtgn2h * vitu * normvit);
         const T af22 = 1.0 + div_rn(dtgn2h * (twice(vitu * vitu) + vitv * vitv), normvit, yn);
         const T af23 = div_rn(dtgn2h * vitu * vitv, normvit, yn);
@@ -1535,11 +1548,11 @@ CF_HD CF_INLINE void element_core(const MemberDev& M, double area, double yarea,
   if (M.friction == 1) {
     T sf2, sf3, m[6];
     friction_terms(M, area, dt, manning, q1, q2, q3, sf2, sf3, m, yq1);
-    const T ri1 = div_rn(0. + 0. - rc1, area, yarea);
+    const T ri1 = div_rn(zero_minus(rc1), area, yarea);   /* 0 + 0 - rc1 */
     const T ri2 = div_rn(sb2 + sf2 - rc2, area, yarea);
     const T ri3 = div_rn(sb3 + sf3 - rc3, area, yarea);
     if (M.fricimplic == 1 || M.fricimplic == 2) {
-      r1 = 1. * ri1 + 0. * ri2 + 0. * ri3;
+      r1 = first_row(ri1, ri2, ri3);
       r2 = m[0] * ri1 + m[1] * ri2 + m[2] * ri3;
       r3 = m[3] * ri1 + m[4] * ri2 + m[5] * ri3;
     } else {
@@ -1548,7 +1561,7 @@ CF_HD CF_INLINE void element_core(const MemberDev& M, double area, double yarea,
       r3 = ri3;
     }
   } else {
-    r1 = div_rn(0. - rc1, area, yarea);
+    r1 = div_rn(zero_minus(rc1), area, yarea);
     r2 = div_rn(sb2 - rc2, area, yarea);
     r3 = div_rn(sb3 - rc3, area, yarea);
   }

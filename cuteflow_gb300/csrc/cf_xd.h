@@ -482,7 +482,18 @@ struct ConstOps<XD<MUL>> {
 template <bool MUL> XD_HD XD<MUL> dmax0(const XD<MUL>& x) { return xgt_c(x.v, 0.0) ? x : XD<MUL>(0.0); }
 
 template <bool MUL> XD_HD XD<MUL> sqrt(const XD<MUL>& a) { return XD<MUL>(MUL ? em_sqrt(a.v) : ::sqrt(a.v)); }
-template <bool MUL> XD_HD XD<MUL> rcbrt(const XD<MUL>& a) { return XD<MUL>(rcbrt(a.v)); }
+struct MulInt {
+  static XD_HD double mul(double a, double b) { return em_mul(a, b); }
+};
+XD_HD XD<false> rcbrt(const XD<false>& a) { return XD<false>(rcbrt(a.v)); }
+XD_HD XD<true> rcbrt(const XD<true>& a) { return XD<true>(rcbrt_of<MulInt>(a.v)); }
+/* 0 - x but for the sign of a zero, which the update adds to a depth */
+template <bool MUL> XD_HD XD<MUL> zero_minus(const XD<MUL>& x) { return -x; }
+/* a where b and c are finite (0 b and 0 c are zeros then) */
+template <bool MUL> XD_HD XD<MUL> first_row(const XD<MUL>& a, const XD<MUL>& b, const XD<MUL>& c) {
+  const bool fin = ((~xhi(b.v) & 0x7ff00000u) != 0) & ((~xhi(c.v) & 0x7ff00000u) != 0);
+  return fin ? a : XD<MUL>(xdbl(0x7ff8000000000000ull));
+}
 template <bool MUL> XD_HD XD<MUL> fabs(const XD<MUL>& a) {
   uint32_t lo, hi;
   xwords(a.v, lo, hi);
