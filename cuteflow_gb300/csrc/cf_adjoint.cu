@@ -275,48 +275,61 @@ __global__ void __launch_bounds__(TILE_E) k_adj_edges(AdjArgs A) {
   else adj_interior_edge<IFLUX, D>(A, M, e, ab, dt);
 }
 
-/* First-order HLLC (flux_mode 0): the closed-form reverse edge (adj_edge_hllc) for every interior edge
- * it covers; the edges it leaves (a nearly dry side whose raw and masked depths differ) are queued for
- * k_adj_edges_rest.  Four blocks per SM (128 registers): 51k triangles, 51.6 us at three, 38.2 at four,
- * 39.7 at five, 40.0 at six; 339 us per reverse step of 200k triangles while the flux ran on four dual
- * lanes. */
-__global__ void __launch_bounds__(TILE_E, 4) k_adj_edges_hllc(AdjArgs A) {
+/* One side of a reverse HLLC edge on this lane, the other one on lane ^ 1; mask: the lanes at work */
+struct AdjLanePair {
+  AdjSide s;
+  double lam[3];
+  unsigned mask;
+  template <class F>
+  __device__ __forceinline__ void each(F&& f) { f(s, lam); }
+  __device__ __forceinline__ void exchange(int n) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (k < n) s.y[k] = XD<true>(__shfl_xor_sync(mask, val(s.x[k]), 1));
+  }
+  __device__ __forceinline__ void finish() {
+    if (__any_sync(mask, s.odd)) {
+      const bool odd = s.odd | __shfl_xor_sync(mask, (int)s.odd, 1);
+      double o[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, q[6], one[3];
+      if (odd) s.one_side(o);
+#pragma unroll
+      for (int k = 0; k < 6; ++k) q[k] = __shfl_xor_sync(mask, o[k], 1);
+      s.join(o, q, one);
+      s.reverse3(odd ? one : nullptr, lam);
+    } else {
+      s.reverse3(nullptr, lam);
+    }
+  }
+};
+
+/* First-order HLLC (flux_mode 0): the closed-form reverse edge (AdjSide), two lanes per edge as in the
+ * edge kernel: ~3,000 instructions a lane, 59 of them FP64 ones.  Us per reverse step, 22k / 51k
+ * triangles: 25 / 33 (one thread per edge: 39, latency-bound / 38; on four dual lanes 339 at 200k).
+ * 24 warps per SM at 80 registers; 16 at 128 and 20 at 102 measured the same. */
+__global__ void __launch_bounds__(2 * TILE_E, 3) k_adj_edges_hllc(AdjArgs A) {
   const StepArgs& a = A.s;
   const int tile = blockIdx.x;
   const int m = __ldg(a.etile_mem + tile);
   const MemberDev& M = a.mdev[m];
-  const int e = tile * TILE_E + threadIdx.x;
-  if (e >= M.edge_end) return;
-  const int2 ab = ldro(a.ecell + e);
-  if (ab.y < 0) {
+  const int e = tile * TILE_E + (threadIdx.x >> 1), side = threadIdx.x & 1;
+  const bool live = e < M.edge_end;
+  int2 ab = make_int2(0, -3);
+  if (live) ab = ldro(a.ecell + e);
+  const bool run = live && ab.y >= 0;
+  const unsigned mask = __ballot_sync(0xffffffffu, run);
+  if (run) {
+    const int c = side ? ab.y : ab.x;
+    const double4 geo = ld4(a.egeo + e), U = ld4(a.Uin + c);
+    const double2 z = ldro(reinterpret_cast<const double2*>(a.ez + e));
+    const Slot wc = load_slot_adj(A.cadj + c);
+    const double w[5] = {wc.f1, wc.f2, wc.f3, wc.bx, wc.by};
+    AdjLanePair p;
+    p.mask = mask;
+    p.s.begin(M, side, geo, U, side ? z.y : z.x, side ? z.x : z.y, w);
+    adj_stages(p);
+    A.eadj[2 * (size_t)e + side] = make_double4(p.lam[0], p.lam[1], p.lam[2], 0.0);
+  } else if (live && side == 0) {
     adj_boundary_edge<1>(A, M, e, ab, __ldg(A.t_hist + hidx(A.n, m, a.nmembers)));
-    return;
-  }
-  const double4 UA = ld4(a.Uin + ab.x), UB = ld4(a.Uin + ab.y);
-  const double4 ez = ld4(a.ez + e);
-  const Slot wa = A.cadj[ab.x], wb = A.cadj[ab.y];
-  const EdgeGeo G = edge_geo(a, e, false);
-  const double w[10] = {wa.f1, wa.f2, wa.f3, wa.bx, wa.by, wb.f1, wb.f2, wb.f3, wb.bx, wb.by};
-  double la[3], lb[3];
-  if (adj_edge_hllc(M, G, UA, UB, ez.x, ez.y, w, la, lb)) {
-    A.eadj[2 * (size_t)e] = make_double4(la[0], la[1], la[2], 0.0);
-    A.eadj[2 * (size_t)e + 1] = make_double4(lb[0], lb[1], lb[2], 0.0);
-  } else {
-    A.pend[atomicAdd(A.npend, 1)] = e;
-  }
-}
-
-/* The queued interior edges of k_adj_edges_hllc, differentiated in six Dual lanes (grid-stride
- * over the queue; the queue's order does not matter, every edge writes only its own entries). */
-__global__ void __launch_bounds__(TILE_E) k_adj_edges_rest(AdjArgs A) {
-  const StepArgs& a = A.s;
-  const int n = *A.npend;
-  for (int i = blockIdx.x * TILE_E + threadIdx.x; i < n; i += gridDim.x * TILE_E) {
-    const int e = A.pend[i];
-    const int m = __ldg(a.etile_mem + e / TILE_E);
-    const MemberDev& M = a.mdev[m];
-    const double dt = __ldg(A.dt_hist + hidx(A.n, m, a.nmembers));
-    adj_interior_edge<1, 6>(A, M, e, ldro(a.ecell + e), dt);
   }
 }
 
@@ -408,13 +421,8 @@ int launch_adjoint_step(const AdjArgs& A, stream_t s) {
   k_adj_cells<<<a.n_ctiles * (TILE_C / ADJ_CELLS_BLOCK), ADJ_CELLS_BLOCK, 0, st>>>(A);
   switch (a.iflux) {
     case 1:
-      if (a.flux_mode == 0 && A.pend && A.npend) {
-        cudaMemsetAsync(A.npend, 0, sizeof(int32_t), st);
-        k_adj_edges_hllc<<<a.n_etiles, TILE_E, 0, st>>>(A);
-        k_adj_edges_rest<<<std::min(a.n_etiles, 304), TILE_E, 0, st>>>(A);
-      } else {
-        k_adj_edges<1, 6><<<a.n_etiles, TILE_E, 0, st>>>(A);
-      }
+      if (a.flux_mode == 0) k_adj_edges_hllc<<<a.n_etiles, 2 * TILE_E, 0, st>>>(A);
+      else k_adj_edges<1, 6><<<a.n_etiles, TILE_E, 0, st>>>(A);
       break;
     case 2: k_adj_edges<2, 3><<<a.n_etiles, TILE_E, 0, st>>>(A); break;
     case 3: k_adj_edges<3, 2><<<a.n_etiles, TILE_E, 0, st>>>(A); break;

@@ -207,189 +207,260 @@ CFD_HD Dual<N> rcbrt(const Dual<N>& x) {
 /* a b + c in one FP64 instruction (derivatives only: values round every operation) */
 CFD_HD XD<true> xfma(const XD<true>& a, const XD<true>& b, const XD<true>& c) { return XD<true>(fma(a.v, b.v, c.v)); }
 
-/* The transposed edge stage of an interior first-order HLLC edge (IFLUX 1, flux_mode 0): given the
- * adjoint weights w[10] of its two slots (side A: flux 1-3, bed x, y; then side B), the
- * contributions lamA, lamB to the adjoints of (h, hu, hv) of its two elements, i.e. J^T w for the
- * edge's Jacobian J, by the chain rule backwards through the flux's own formulas:
- *   - the rotation of both sides' frame fluxes (x1, x2, x3), with x3 = x1 v in every region, v the
- *     tangential velocity the region takes;
+/* J^T w of one side's first-order HLLC flux (weights w of its three global components) towards a
+ * differing right state, for the edges with a nearly dry side (0 < h <= tolisec, whose raw and masked
+ * depths differ, so that the two sides see different states): rare, out of line, on dual numbers.
+ * out: the adjoints of the left (h, u, v) and of the right one. */
+#ifdef __CUDACC__
+static __host__ __device__ __noinline__
+#else
+static inline
+#endif
+void adj_one_side(double g, double nx, double ny, const double l[3], const double r[3], const double w[3],
+                  double out[6]) {
+  typedef Dual<6> D;
+  TwoFluxT<D> F;
+  first_order_flux<1>(g, nx, ny, D::var(l[0], 0), D::var(l[1], 1), D::var(l[2], 2), D::var(r[0], 3), D::var(r[1], 4),
+                      D::var(r[2], 5), F);
+  for (int i = 0; i < 6; ++i) out[i] = fma(w[0], F.a1.d[i], fma(w[1], F.a2.d[i], w[2] * F.a3.d[i]));
+}
+
+/* One side of the transposed edge stage of an interior first-order HLLC edge (IFLUX 1, flux_mode 0):
+ * given the adjoint weights w[5] of this side's slot (flux 1-3, bed x, y), and the other side running
+ * beside it (EdgeSide: two lanes of the GPU), the contribution lam to the adjoint of (h, hu, hv) of
+ * this side's element, by the chain rule backwards through the flux's own formulas:
+ *   - the rotation of the frame flux (x1, x2, x3), with x3 = x1 v in every region, v the tangential
+ *     velocity the region takes;
  *   - the HLL fluxes N / (s_R - s_L + eps) or the physical flux the region takes;
- *   - the speeds s_L = u_l - a_l p_l, s_R = u_r + a_r p_r with p = 1 or sqrt((h* + h) h* / 2) / h, and
- *     the depth h* = (h_l + h_r) / 2 - (u_r - u_l) (h_l + h_r) / (a_l + a_r) / 4; next to a dry side
- *     s = u -+ a and u +- 2 a of the wet one;
+ *   - the speed s_L = u - a p with p = 1 or sqrt((h* + h) h* / 2) / h, and the depth
+ *     h* = (h + h') / 2 - (u' - u) (h + h') / (a + a') / 4; next to a dry side s = u - a and u + 2 a of
+ *     the wet one;
  *   - the hydrostatic reconstruction (depths pass or are clamped to 0), the change to the edge frame
- *     (u_n = (hu nx + hv ny) / h, u_t = (hv nx - hu ny) / h) and the bed sources g/2 (ha^2 - h^2) len.
- * The values repeat the step's IEEE operations (so every branch is the forward's), their products,
- * quotients and roots on the integer pipes; of the derivatives the multiply-adds are FP64
- * instructions and the products integer ones.  Returns false, and the caller differentiates the edge
- * in full, where a side's raw and masked depths differ (0 < h <= tolisec; the reference then evaluates
- * the two sides differently). */
-CFD_HD bool adj_edge_hllc(const MemberDev& M, const EdgeGeo& G, const double4& UA, const double4& UB, double zml,
-                          double zmr, const double w[10], double lamA[3], double lamB[3]) {
+ *     (u_n = (hu nx + hv ny) / h, u_t = (hv nx - hu ny) / h) and the bed source g/2 (hw^2 - h^2) len.
+ * The other side's flux is this one's mirrored, so the adjoints of the HLL fluxes are the difference
+ * and the sum of the two sides' weights, and what remains towards each side's own state is the same
+ * code on either.  The values repeat the step's IEEE operations (so every branch is the forward's),
+ * their products, quotients and roots on the integer pipes; of the derivatives the multiply-adds are
+ * FP64 instructions and the products integer ones. */
+struct AdjSide : EdgeSide<1, XD<true>> {
   typedef XD<true> X;
-  const double g = M.gp, tolisec = M.tolisec, nx = G.nx, ny = G.ny, eps = EPS_HLLC;
-  const X hA(UA.x), hB(UB.x);
-  const bool wa = hA > tolisec, wb = hB > tolisec;   /* frame velocities differentiable */
-  if ((!wa && hA != 0.0) || (!wb && hB != 0.0)) return false;
-  const double zij = val(dmax(X(zml), X(zmr)));
-  X hm, ul, vl, ur, vr;
-  to_frame(hA, X(UA.y), X(UA.z), UA.w, nx, ny, tolisec, hm, ul, vl);
-  to_frame(hB, X(UB.y), X(UB.z), UB.w, nx, ny, tolisec, hm, ur, vr);
-  const X ul0 = ul, vl0 = vl, ur0 = ur, vr0 = vr;
-  /* hydrostatic reconstruction (flux_riemann.cuf:176-181, :200-210); which variables carry a
-   * derivative (a clamped or masked one is a constant of the inputs) */
-  const X ea = hA + zml - zij, eb = hB + zmr - zij;
-  const X ha = dmax0(ea), hb = dmax0(eb);
-  X hl = wa ? ha : X(0.0), hr = hb;
-  const bool pl = !(hl < tolisec), pr = !(hr < tolisec);
-  if (!pl) { hl = X(0.); ul = X(0.); vl = X(0.); }
-  if (!pr) { hr = X(0.); ur = X(0.); vr = X(0.); }
-  const bool s_hl = pl && wa && ea > 0., s_ul = pl && wa, s_hr = pr && eb > 0., s_ur = pr && wb;
-  X ghl(0.0), gul(0.0), gvl(0.0), ghr(0.0), gur(0.0), gvr(0.0);   /* adjoints (without the factor len) */
-  if (!(hl < eps && hr < eps)) {
-    /* the flux's values, as wave_speeds and first_order_flux<1> form them */
-    const X gl = g * hl, gr = g * hr, al = sqrt(gl), ar = sqrt(gr);
-    const X hs = hl + hr, du = ur - ul, as = al + ar;
-    const X qd = du * hs / as;
-    const X het = halve(hs) - quarter(qd);
-    const bool wl = hl > eps, wr = hr > eps, both = wl && wr;
-    const bool kl = both && !lt_nonneg(het, hl), kr = both && !lt_nonneg(het, hr);
-    const X hll2 = hl * hl, hrr2 = hr * hr;
-    const X pql = kl ? sqrt(halve(het + hl) * het / hll2) : X(1.), pqr = kr ? sqrt(halve(het + hr) * het / hrr2) : X(1.);
-    X sl, sr;
-    if (wl) {
-      sl = ul - (both ? al * pql : al);
-      sr = wr ? ur + ar * pqr : ul + twice(al);
-    } else {
-      sl = ur - twice(ar);
-      sr = ur + ar;
+  double w[5];
+  double yh;                     /* RN(1/h) of the element */
+  X het, pq, hs, du, qd;
+  X fg1, fg2, t, y1, m1, m2, gh, gu, gv, ga, gsl;
+  bool wet, both, wl, strong, odd;
+  int r, rp;                     /* region of this side's flux, and of the other side's in its own frame */
+
+  CFD_HD void begin(const MemberDev& M, int side_, const double4& geo, const double4& U, double z, double zo,
+                    const double w_[5]) {
+    for (int i = 0; i < 5; ++i) w[i] = w_[i];
+    yh = U.w;
+    frame(M, side_, side_ ? -geo.x : geo.x, side_ ? -geo.y : geo.y, geo.z, U, z, zo);
+    wet = h0 > tolisec;
+  }
+  CFD_HD void values1() {
+    speeds1();
+    odd = hraw != hr;            /* the other side is nearly dry */
+  }
+  CFD_HD void values2() {
+    const X ar = y[0];
+    hs = side ? y[1] : s;
+    du = side ? s : y[1];
+    as_ = a + ar;
+    qd = du * hs / as_;
+    het = halve(hs) - quarter(qd);
+    wl = h > eps();
+    both = wl && hr > eps();
+    strong = both && !lt_nonneg(het, h);
+    pq = strong ? sqrt(halve(het + h) * het / (h * h)) : X(1.);
+    sl = (wl ? u : ur) - (wl ? (both ? a * pq : a) : twice(ar));
+    d0 = u - sl;
+    f1 = h * u;
+    f2 = h * (u * u) + halve(gh_() * h);
+    d = h * d0;
+    x[0] = sl;
+    x[1] = d;
+    x[2] = f1;
+    x[3] = f2;
+  }
+  CFD_HD const X& gh_() const { return EdgeSide<1, XD<true>>::gh; }
+  CFD_HD void values3() {
+    sr = -y[0];
+    s = y[1];
+    fr1 = -y[2];
+    fr2 = y[3];
+    t2 = sr * h * d0;
+    x[0] = t2;
+  }
+  CFD_HD void values4() {
+    t2 = (side ? -d : y[0]) - (side ? s : t2);   /* as contact1 */
+    x[0] = t2;
+  }
+  CFD_HD void reverse1() {
+    const X num = side ? -y[0] : t2, denom = side ? t2 : y[0];
+    if (fabs(denom) < eps()) set = halve(u + ur) - (hr - h) * as_ / hs;
+    else set = num / denom;
+    r = (sl > 0.) ? 0 : ((sr < 0.) ? 1 : 2);
+    rp = (sr < 0.) ? 0 : ((sl > 0.) ? 1 : 2);
+    const bool right = r == 1 || (r == 2 && !(set > 0.));
+    t = xfma(X(w[2]), X(nx), -(X(w[1]) * ny));
+    fg2 = xfma(X(w[1]), X(nx), X(w[2]) * ny);
+    fg1 = xfma(right ? vr : v, t, X(w[0]));
+    y1 = 1.0 / (sr - sl + eps());
+    const X c1 = xfma(sl, hr - h, f1), c2 = xfma(sl, fr1 - f1, f2);
+    m1 = xfma(sr, c1, -(sl * fr1)) * y1;
+    m2 = xfma(sr, c2, -(sl * fr2)) * y1;
+    const X c = t * (r == 0 ? f1 : (r == 1 ? fr1 : m1));
+    gv = right ? X(0.0) : c;
+    x[0] = fg1;
+    x[1] = fg2;
+    x[2] = c;
+  }
+  CFD_HD void reverse2() {
+    /* the other side's tangential flux carries this side's v */
+    if (rp == 1 || (rp == 2 && !(set < 0.))) gv = gv - y[2];
+    X gf1(0.0), gf2(0.0);
+    gh = X(0.0);
+    gsl = X(0.0);
+    if (r == 2 || rp == 2) {
+      const X n1 = (rp == 2 ? (r == 2 ? fg1 - y[0] : -y[0]) : fg1) * y1;
+      const X n2 = (rp == 2 ? (r == 2 ? fg2 + y[1] : y[1]) : fg2) * y1;
+      const X ss = sl * sr, q2 = n2 * ss;
+      gsl = xfma(n1, xfma(sr, hr - h, -fr1) + m1, n2 * (xfma(sr, fr1 - f1, -fr2) + m2));
+      gf1 = xfma(n1, sr, -q2);
+      gf2 = n2 * sr;
+      gh = -(n1 * ss);
     }
-    const X fl1 = hl * ul, fl2 = hl * (ul * ul) + halve(gl * hl);
-    const X fr1 = hr * ur, fr2 = hr * (ur * ur) + halve(gr * hr);
-    const int ra = (sl > 0.) ? 0 : ((sr < 0.) ? 1 : 2);
-    const int rb = (sr < 0.) ? 1 : ((sl > 0.) ? 0 : 2);
-    /* s* decides which tangential velocity the HLL region carries */
-    bool right_a = ra == 1, right_b = rb == 1;
-    if (ra == 2 || rb == 2) {
-      const X d1 = hr * (ur - sr), d0 = hl * (ul - sl), denom = d1 - d0;
-      X set;
-      if (fabs(denom) < eps) set = halve(ul + ur) - (hr - hl) * as / hs;
-      else set = (sl * hr * (ur - sr) - sr * hl * (ul - sl)) / denom;
-      if (ra == 2) right_a = !(set > 0.);
-      if (rb == 2) right_b = set < 0.;
+    if (r == 0) { gf1 = gf1 + fg1; gf2 = gf2 + fg2; }
+    if (rp == 1) { gf1 = gf1 - y[0]; gf2 = gf2 + y[1]; }
+    /* physical flux: f1 = h u, f2 = h u^2 + g h^2 / 2 */
+    gh = xfma(gf1, u, xfma(gf2, xfma(u, u, gh_()), gh));
+    gu = xfma(gf1, h, twice(gf2 * f1));
+    ga = X(0.0);
+    X ghet(0.0);
+    if (strong) {
+      /* p^2 = P = (h* + h) h* / 2 / h^2: dP/dh* = (h* + h / 2) / h^2, dP/dh = (h* / 2 - 2 P h) / h^2 */
+      const X gp = -(gsl * a) / (twice(pq) * (h * h));
+      ghet = gp * (het + halve(h));
+      gh = xfma(gp, xfma(-twice(pq * pq), h, halve(het)), gh);
     }
-    /* adjoints of x1, x2 (side A) and y1, y2 (side B, whose frame flux is (-y1, y2, y1 v) mirrored) */
-    const X ta = xfma(X(w[2]), X(nx), -(X(w[1]) * ny)), tb = xfma(X(w[7]), X(nx), -(X(w[6]) * ny));
-    const X ga2 = xfma(X(w[1]), X(nx), X(w[2]) * ny), gb2 = -xfma(X(w[6]), X(nx), X(w[7]) * ny);
-    const X ga1 = xfma(right_a ? vr : vl, ta, X(w[0])), gb1 = -xfma(right_b ? vr : vl, tb, X(w[5]));
-    X gfl1(0.0), gfl2(0.0), gfr1(0.0), gfr2(0.0), gsl(0.0), gsr(0.0), m1(0.0);
-    if (ra == 2 || rb == 2) {
-      const X gh1 = (ra == 2 && rb == 2) ? ga1 + gb1 : (ra == 2 ? ga1 : gb1);
-      const X gh2 = (ra == 2 && rb == 2) ? ga2 + gb2 : (ra == 2 ? ga2 : gb2);
-      const X y = 1.0 / (sr - sl + eps);
-      const X dh = hr - hl, df = fr1 - fl1, ss = sl * sr;
-      const X c1 = xfma(sl, dh, fl1), c2 = xfma(sl, df, fl2), e1 = xfma(sr, dh, -fr1), e2 = xfma(sr, df, -fr2);
-      m1 = xfma(sr, c1, -(sl * fr1)) * y;
-      const X m2 = xfma(sr, c2, -(sl * fr2)) * y;
-      const X n1 = gh1 * y, n2 = gh2 * y;
-      const X gd = -xfma(n1, m1, n2 * m2);
-      gsr = xfma(n1, c1, xfma(n2, c2, gd));
-      gsl = xfma(n1, e1, xfma(n2, e2, -gd));
-      const X q1 = n1 * ss, q2 = n2 * ss;
-      gfl1 = xfma(n1, sr, -q2);
-      gfr1 = xfma(-n1, sl, q2);
-      gfl2 = n2 * sr;
-      gfr2 = -(n2 * sl);
-      ghl = -q1;
-      ghr = q1;
-    }
-    if (ra == 0) { gfl1 = gfl1 + ga1; gfl2 = gfl2 + ga2; }
-    if (ra == 1) { gfr1 = gfr1 + ga1; gfr2 = gfr2 + ga2; }
-    if (rb == 0) { gfl1 = gfl1 + gb1; gfl2 = gfl2 + gb2; }
-    if (rb == 1) { gfr1 = gfr1 + gb1; gfr2 = gfr2 + gb2; }
-    /* tangential velocities: x1 ta on side A, -y1 tb on side B */
-    const X va = (ra == 0 ? fl1 : (ra == 1 ? fr1 : m1)) * ta, vb = -((rb == 0 ? fl1 : (rb == 1 ? fr1 : m1)) * tb);
-    if (right_a == right_b) (right_a ? gvr : gvl) = va + vb;
-    else { gvl = right_a ? vb : va; gvr = right_a ? va : vb; }
-    /* physical fluxes: f1 = h u, f2 = h u^2 + g h^2 / 2 */
-    ghl = xfma(gfl1, ul, xfma(gfl2, xfma(ul, ul, gl), ghl));
-    gul = xfma(gfl1, hl, twice(gfl2 * fl1));
-    ghr = xfma(gfr1, ur, xfma(gfr2, xfma(ur, ur, gr), ghr));
-    gur = xfma(gfr1, hr, twice(gfr2 * fr1));
-    /* speeds */
-    X gal(0.0), gar(0.0);
+    x[0] = ghet;
+    x[1] = gsl;
+  }
+  /* this side's flux alone, from its masked state towards the other one's raw reconstruction: the
+   * adjoints of the two states, each in this side's frame */
+  CFD_HD void one_side(double o[6]) const {
+    const double l[3] = {val(h), val(u), val(v)};
+    const double rr[3] = {val(hraw), val(ur), val(vr)};
+    const double ww[3] = {w[0], w[1], w[2]};
+    double oo[6];
+    adj_one_side(g, nx, ny, l, rr, ww, oo);
+    for (int i = 0; i < 6; ++i) o[i] = oo[i];
+  }
+  /* the adjoints of this side's own state from both one-sided evaluations: the left state of its own (a
+   * constant where the depth is masked), the right state (mirrored velocities) of the other's */
+  CFD_HD void join(const double own[6], const double other[6], double one[3]) const {
+    one[0] = (wet ? own[0] : 0.0) + other[3];
+    one[1] = own[1] - other[4];
+    one[2] = own[2] - other[5];
+  }
+  /* one: the adjoints of this side's own state from a one-sided evaluation (adj_one_side) of both
+   * fluxes, in place of the above */
+  CFD_HD void reverse3(const double* one, double lam[3]) {
     if (both) {
-      gul = gul + gsl;
-      gur = gur + gsr;
-      gal = -(gsl * pql);
-      gar = gsr * pqr;
-      if (kl || kr) {
-        /* p^2 = P = (h* + h) h* / 2 / h^2: dP/dh* = (h* + h / 2) / h^2, dP/dh = (h* / 2 - 2 P h) / h^2 */
-        X ghet(0.0);
-        if (kl) {
-          const X gp = -(gsl * al) / (twice(pql) * hll2);
-          ghet = gp * (het + halve(hl));
-          ghl = xfma(gp, xfma(-twice(pql * pql), hl, halve(het)), ghl);
-        }
-        if (kr) {
-          const X gp = gsr * ar / (twice(pqr) * hrr2);
-          ghet = xfma(gp, het + halve(hr), ghet);
-          ghr = xfma(gp, xfma(-twice(pqr * pqr), hr, halve(het)), ghr);
-        }
-        /* h* */
-        const X q = quarter(ghet) / as;
-        const X dq = q * du, uq = q * hs, aq = q * qd;
-        const X gh = halve(ghet) - dq;
-        ghl = ghl + gh;
-        ghr = ghr + gh;
-        gul = gul + uq;
-        gur = gur - uq;
-        gal = gal + aq;
-        gar = gar + aq;
-      }
+      gu = gu + gsl;
+      ga = -(gsl * pq);
+      const X ghet = x[0] + y[0];
+      const X q = quarter(ghet) / as_;
+      gh = gh + (halve(ghet) - q * du);
+      gu = xfma(q, hs, gu);
+      ga = xfma(q, qd, ga);
     } else if (wl) {
-      gul = gul + gsl + gsr;
-      gal = twice(gsr) - gsl;
-    } else {
-      gur = gur + gsl + gsr;
-      gar = gsr - twice(gsl);
+      const X gsr = -y[1];       /* next to a dry side this one sets both speeds */
+      gu = gu + gsl + gsr;
+      ga = twice(gsr) - gsl;
     }
-    /* celerities a = sqrt(g h): da/dh = g / (2 a) */
-    const double hg = ConstOps<X>::half(g);
-    if (wl) ghl = ghl + gal * hg / al;
-    if (wr) ghr = ghr + gar * hg / ar;
-  }
-  /* to the conserved variables: d(h_m, u_n, u_t)/d(h, hu, hv) with y = RN(1/h); the bed sources
-   * (source_terms.cuf:90-97): ta = g/2 (ha^2 - hA^2) len into (ta nx, ta ny) of side A, tb likewise
-   * into -(tb nx, tb ny) of side B */
-  const double len = G.len;
-  {
-    const X gu = s_ul ? gul : X(0.0), gv = s_ul ? gvl : X(0.0);
-    X gh = s_hl ? ghl : X(0.0);
-    gh = xfma(xfma(X(w[3]), X(nx), X(w[4]) * ny) * g, (ea > 0. ? ha : X(0.0)) - hA, gh);
-    const X y = len * X(UA.w);
-    lamA[0] = lamA[1] = lamA[2] = 0.0;
-    if (wa) {
-      lamA[0] = val(xfma(gh, X(len), -(xfma(gu, ul0, gv * vl0) * y)));
-      lamA[1] = val(xfma(gu, X(nx), -(gv * ny)) * y);
-      lamA[2] = val(xfma(gu, X(ny), gv * nx) * y);
+    if (wl) gh = gh + ga * ConstOps<X>::half(g) / a;   /* a = sqrt(g h) */
+    if (dry) gh = gu = gv = X(0.0);
+    bool sh = wet && hw > 0. && !(h < tolisec), su = wet && !(h < tolisec);
+    if (one) {
+      gh = X(one[0]);
+      gu = X(one[1]);
+      gv = X(one[2]);
+      sh = hw > 0. && !(hw < tolisec);
+    }
+    if (!sh) gh = X(0.0);
+    if (!su) gu = gv = X(0.0);
+    gh = xfma(xfma(X(w[3]), X(nx), X(w[4]) * ny) * g, hw - h0, gh);
+    if (wet) {
+      const X yl = len * X(yh);
+      lam[0] = val(xfma(gh, X(len), -(xfma(gu, u, gv * v) * yl)));
+      lam[1] = val(xfma(gu, X(nx), -(gv * ny)) * yl);
+      lam[2] = val(xfma(gu, X(ny), gv * nx) * yl);
     } else {
-      lamA[0] = val(gh * len);
+      lam[0] = val(gh * len);
+      lam[1] = lam[2] = 0.0;
     }
   }
-  {
-    const X gu = s_ur ? gur : X(0.0), gv = s_ur ? gvr : X(0.0);
-    X gh = s_hr ? ghr : X(0.0);   /* the B side reconstructs from the raw depth */
-    gh = xfma(-(xfma(X(w[8]), X(nx), X(w[9]) * ny) * g), (eb > 0. ? hb : X(0.0)) - hB, gh);
-    const X y = len * X(UB.w);
-    lamB[0] = lamB[1] = lamB[2] = 0.0;
-    if (wb) {
-      lamB[0] = val(xfma(gh, X(len), -(xfma(gu, ur0, gv * vr0) * y)));
-      lamB[1] = val(xfma(gu, X(nx), -(gv * ny)) * y);
-      lamB[2] = val(xfma(gu, X(ny), gv * nx) * y);
-    } else {
-      lamB[0] = val(gh * len);
+};
+
+/* The stages of both sides (P as in side_stages; P::any: some pair at hand takes the one-sided
+ * evaluation) */
+template <class P>
+CFD_HD void adj_stages(P& p) {
+  p.exchange(4);
+  p.each([](AdjSide& s, double*) { s.values1(); });
+  p.exchange(2);
+  p.each([](AdjSide& s, double*) { s.values2(); });
+  p.exchange(4);
+  p.each([](AdjSide& s, double*) { s.values3(); });
+  p.exchange(1);
+  p.each([](AdjSide& s, double*) { s.values4(); });
+  p.exchange(1);
+  p.each([](AdjSide& s, double*) { s.reverse1(); });
+  p.exchange(3);
+  p.each([](AdjSide& s, double*) { s.reverse2(); });
+  p.exchange(2);
+  p.finish();
+}
+
+struct AdjHostPair {
+  AdjSide s[2];
+  double lam[2][3];
+  template <class F>
+  CFD_HD void each(F&& f) {
+    f(s[0], lam[0]);
+    f(s[1], lam[1]);
+  }
+  CFD_HD void exchange(int n) {
+    for (int k = 0; k < n; ++k) {
+      s[0].y[k] = s[1].x[k];
+      s[1].y[k] = s[0].x[k];
     }
+  }
+  void finish() {
+    double one[2][3];
+    const bool odd = s[0].odd || s[1].odd;
+    if (odd) {
+      double o[2][6];
+      for (int k = 0; k < 2; ++k) s[k].one_side(o[k]);
+      for (int k = 0; k < 2; ++k) s[k].join(o[k], o[1 - k], one[k]);
+    }
+    for (int k = 0; k < 2; ++k) s[k].reverse3(odd ? one[k] : nullptr, lam[k]);
+  }
+};
+
+/* Both sides on the host: lamA, lamB from the weights w[10] of the two slots */
+inline bool adj_edge_hllc(const MemberDev& M, const EdgeGeo& G, const double4& UA, const double4& UB, double zml,
+                          double zmr, const double w[10], double lamA[3], double lamB[3]) {
+  const double4 geo = make_double4(G.nx, G.ny, G.len, 0.0);
+  AdjHostPair p;
+  p.s[0].begin(M, 0, geo, UA, zml, zmr, w);
+  p.s[1].begin(M, 1, geo, UB, zmr, zml, w + 5);
+  adj_stages(p);
+  for (int k = 0; k < 3; ++k) {
+    lamA[k] = p.lam[0][k];
+    lamB[k] = p.lam[1][k];
   }
   return true;
 }

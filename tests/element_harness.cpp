@@ -51,3 +51,49 @@ extern "C" double harness_adj_element(long long n, unsigned long long seed, int 
   }
   return worst;
 }
+
+/* adj_edge_hllc against the edge differentiated in six Dual lanes, on edges with a side at the dry
+ * threshold (masked, with a raw depth that reconstructs to the threshold).  Relative to the largest sum
+ * of the magnitudes of a component's terms: a component itself may cancel to any degree (a bed source
+ * along the edge). */
+extern "C" double harness_adj_nearly_dry(long long n, unsigned long long seed) {
+  unsigned long long s = seed | 1;
+  auto rnd = [&]() { s ^= s << 13; s ^= s >> 7; s ^= s << 17; return s; };
+  auto unif = [&]() { return (double)(rnd() >> 11) * (1.0 / 9007199254740992.0); };
+  auto sym = [&]() { return 2.0 * unif() - 1.0; };
+  typedef Dual<6> D;
+  double worst = 0.0;
+  for (long long i = 0; i < n; ++i) {
+    MemberDev M;
+    std::memset(&M, 0, sizeof(M));
+    M.gp = 9.81; M.tolisec = 1e-3;
+    const double phi = 6.283 * unif();
+    EdgeGeo G = EdgeGeo();
+    G.nx = std::cos(phi); G.ny = std::sin(phi); G.len = 0.5 + unif();
+    const double zl = rnd() & 1 ? 0.0 : 0.1 * unif(), zr = rnd() % 3 ? zl : 0.1 * unif();
+    auto depth = [&](int k) { return k == 0 ? M.tolisec : (k == 1 ? 0.5 * M.tolisec : 0.002 + 2.0 * unif()); };
+    const int k = (int)(rnd() % 2);
+    double hl = depth(k ? 0 : (int)(rnd() % 3)), hr = depth(k ? (int)(rnd() % 3) : 0);
+    const double4 UA = make_double4(hl, hl * sym(), hl * sym(), 1.0 / hl), UB = make_double4(hr, hr * sym(), hr * sym(), 1.0 / hr);
+    double w[10], la[3], lb[3];
+    for (double& x : w) x = sym();
+    if (!adj_edge_hllc(M, G, UA, UB, zl, zr, w, la, lb)) return INFINITY;
+    D o[10];
+    interior_edge<1>(M, 1, 0, G, 0.01, D::var(UA.x, 0), D::var(UA.y, 1), D::var(UA.z, 2), zl, UA.w, D::var(UB.x, 3),
+                     D::var(UB.y, 4), D::var(UB.z, 5), zr, UB.w, D(0.0), D(0.0), 0.0, D(0.0), D(0.0), 0.0, o);
+    double err = 0.0, top = 1e-30;
+    for (int j = 0; j < 6; ++j) {
+      double want = 0.0, terms = 0.0;
+      for (int q = 0; q < 10; ++q) {
+        want += w[q] * o[q].d[j];
+        terms += std::fabs(w[q] * o[q].d[j]);
+      }
+      const double got = j < 3 ? la[j] : lb[j - 3];
+      if (!(got == got)) return INFINITY;
+      err = std::fmax(err, std::fabs(got - want));
+      top = std::fmax(top, terms);
+    }
+    worst = std::fmax(worst, err / top);
+  }
+  return worst;
+}

@@ -30,3 +30,9 @@ def test_transposed_element_is_the_dual_derivative(lib, friction, fricimplic):
     # ~30 operations on either side, each within 2^-53 of terms no larger than the largest contribution
     # but for cancellations of a factor ~100
     assert lib.harness_adj_element(200_000, 3, friction, fricimplic) < 1e-12
+
+
+def test_reverse_edge_with_a_nearly_dry_side_is_the_dual_derivative(lib):
+    lib.harness_adj_nearly_dry.argtypes = [C.c_longlong, C.c_ulonglong]
+    lib.harness_adj_nearly_dry.restype = C.c_double
+    assert lib.harness_adj_nearly_dry(200_000, 9) < 1e-12
