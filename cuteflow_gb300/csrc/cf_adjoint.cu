@@ -33,20 +33,13 @@
 
 #include <algorithm>
 
+#include "cf_cell_kernel.cuh"
 #include "cf_dual.h"
 #include "cf_edge_kernel.cuh"
 #include "cf_xd.h"
 
 namespace cf {
 namespace {
-
-__device__ __forceinline__ Slot load_slot_adj(const Slot* p) {
-  const double2* q = reinterpret_cast<const double2*>(p);
-  const double2 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2);
-  Slot s;
-  s.f1 = a.x; s.f2 = a.y; s.f3 = b.x; s.bx = b.y; s.by = c.x; s.q = c.y;
-  return s;
-}
 
 /* Dual<D> for input k of the lane chunk starting at base */
 template <int D>
@@ -62,8 +55,8 @@ __device__ __forceinline__ Dual<D> seed(double v, int k, int base) {
 /* The recorded dt and start time of step n of member m: histories are [N][members]. */
 __device__ __forceinline__ size_t hidx(int n, int m, int nm) { return (size_t)n * nm + m; }
 
-/* The replays keep the forward kernels' occupancy: eight edge blocks and four element blocks per SM
- * (64 registers), where the latency of the integer-pipe chains is hidden by more warps. */
+/* The replays keep the forward kernels' occupancy, 1024 threads per SM (64 registers), where the latency
+ * of the integer-pipe chains is hidden by more warps. */
 template <int IFLUX>
 __global__ void __launch_bounds__(2 * TILE_E, 4) k_rep_edges(StepArgs a, const double* dt_hist, const double* t_hist, int n) {
   const int tile = blockIdx.x;
@@ -74,34 +67,46 @@ __global__ void __launch_bounds__(2 * TILE_E, 4) k_rep_edges(StepArgs a, const d
   edge_lanes<IFLUX>(a, M, e, threadIdx.x & 1, e < M.edge_end, __ldg(dt_hist + h), __ldg(t_hist + h), nullptr);
 }
 
-__global__ void __launch_bounds__(TILE_C, 4) k_rep_cells(StepArgs a, const double* dt_hist, int n, uint32_t* flag,
-                                                         Slot* sums) {
-  const int tile = blockIdx.x;
-  const int m = __ldg(a.ctile_mem + tile);
+template <int LANES>
+__global__ void __launch_bounds__(128, 8) k_rep_cells(StepArgs a, const double* dt_hist, int n, uint32_t* flag,
+                                                      Slot* sums_out) {
+  const int c = (blockIdx.x * 128 + threadIdx.x) / LANES, comp = threadIdx.x % LANES;
+  const int m = __ldg(a.ctile_mem + c / TILE_C);
   const MemberDev& M = a.mdev[m];
-  const int c = tile * TILE_C + threadIdx.x;
-  if (c >= M.cell_end) return;
+  const bool active = c < M.cell_end;
   const double dt = __ldg(dt_hist + hidx(n, m, a.nmembers));
-  const double4 U = ld4(a.Uin + c);
-  const double4 st = ld4(a.cstat + c);
-  const int4 sl = __ldg(a.cslot + c);
-  const Slot s0 = load_slot_adj(a.slots + sl.x), s1 = load_slot_adj(a.slots + sl.y), s2 = load_slot_adj(a.slots + sl.z);
+  double4 U = make_double4(0.0, 0.0, 0.0, 0.0), st = U, V = U;
+  Slot s0, s1, s2;
+  CompSums sums = {0.0, 0.0, 0.0, false};
   bool nonfinite = false;
-  const double4 V = (a.xd_cmp && (a.xd_mul_mask & XD_CELLS))
-                        ? element_update<XD<true>>(M, U, st, s0, s1, s2, dt, nonfinite)
-                        : element_update(M, U, st, s0, s1, s2, dt, nonfinite);
-  if (nonfinite) atomicOr(flag, CF_STATUS_NONFINITE);
-  if (a.Uout) {
-    double4* o = a.Uout + c;
-    reinterpret_cast<double2*>(o)[0] = make_double2(V.x, V.y);
-    reinterpret_cast<double2*>(o)[1] = make_double2(V.z, V.w);
+  if (active) {
+    U = ld4(a.Uin + c);
+    st = ld4(a.cstat + c);
+    const int4 sl = __ldg(a.cslot + c);
+    if (LANES == 2) {
+      sums = comp_sums(a.slots, sl, comp);
+    } else {
+      s0 = load_slot(a.slots + sl.x);
+      s1 = load_slot(a.slots + sl.y);
+      s2 = load_slot(a.slots + sl.z);
+    }
   }
-  if (sums) {
-    /* the sums element_update forms (same expressions, same values) */
-    double2* q = reinterpret_cast<double2*>(sums + c);
-    q[0] = make_double2(s0.f1 + s1.f1 + s2.f1, s0.f2 + s1.f2 + s2.f2);
-    q[1] = make_double2(s0.f3 + s1.f3 + s2.f3, s0.bx + s1.bx + s2.bx);
-    q[2] = make_double2(s0.by + s1.by + s2.by, 0.0);
+  if (LANES == 2) V = cell_lanes(a, M, comp, active, U, st, sums, dt, nonfinite);
+  else if (active) V = cell_thread(a, M, U, st, s0, s1, s2, dt, nonfinite);
+  if (nonfinite) atomicOr(flag, CF_STATUS_NONFINITE);
+  if (!active) return;
+  if (a.Uout) {
+    double2* o = reinterpret_cast<double2*>(a.Uout + c);
+    if (LANES == 2) {
+      o[comp] = comp ? make_double2(V.z, V.w) : make_double2(V.x, V.y);
+    } else {
+      o[0] = make_double2(V.x, V.y);
+      o[1] = make_double2(V.z, V.w);
+    }
+  }
+  if (sums_out) {
+    if (LANES == 2) store_comp_sums(sums_out + c, sums, comp);
+    else store_sums(sums_out + c, s0, s1, s2);
   }
 }
 
@@ -159,7 +164,7 @@ __global__ void __launch_bounds__(ADJ_CELLS_BLOCK, 6) k_adj_cells(AdjArgs A) {
   if (c >= M.cell_end) return;
   const double4 L = A.gather ? gather_lambda(A, c, A.gw) : ld4(A.lam_init + c);
   const double dt = __ldg(A.dt_hist + hidx(A.n, mem, a.nmembers));
-  const Slot sums = load_slot_adj(A.sums + c);
+  const Slot sums = load_slot(A.sums + c);
   double4 own;
   Slot w;
   double nb;
@@ -321,7 +326,7 @@ __global__ void __launch_bounds__(2 * TILE_E, 3) k_adj_edges_hllc(AdjArgs A) {
     const int c = side ? ab.y : ab.x;
     const double4 geo = ld4(a.egeo + e), U = ld4(a.Uin + c);
     const double2 z = ldro(reinterpret_cast<const double2*>(a.ez + e));
-    const Slot wc = load_slot_adj(A.cadj + c);
+    const Slot wc = load_slot(A.cadj + c);
     const double w[5] = {wc.f1, wc.f2, wc.f3, wc.bx, wc.by};
     AdjLanePair p;
     p.mask = mask;
@@ -405,7 +410,9 @@ int launch_replay_step(const StepArgs& a, const double* dt_hist, const double* t
     case 3: k_rep_edges<3><<<a.n_etiles, 2 * TILE_E, 0, st>>>(a, dt_hist, t_hist, n); break;
     default: return CF_ENOTSUP;
   }
-  k_rep_cells<<<a.n_ctiles, TILE_C, 0, st>>>(a, dt_hist, n, flag, sums);
+  const int nc = a.n_ctiles * TILE_C;
+  if (two_lanes(a)) k_rep_cells<2><<<2 * nc / 128, 128, 0, st>>>(a, dt_hist, n, flag, sums);
+  else k_rep_cells<1><<<nc / 128, 128, 0, st>>>(a, dt_hist, n, flag, sums);
   return chk(cudaGetLastError());
 }
 

@@ -133,6 +133,9 @@ template <class T>
 CF_HD CF_INLINE T zero_minus(const T& x) { return 0. - x; }
 template <class T>
 CF_HD CF_INLINE T first_row(const T& a, const T& b, const T& c) { return 1. * a + 0. * b + 0. * c; }
+/* every component finite */
+template <class T>
+CF_HD CF_INLINE bool finite_val(const T& x) { return finite_bits(val(x)); }
 
 /* RN(1/d) of a denominator that several quotients share (div_rn) */
 template <class T>
@@ -1605,6 +1608,129 @@ CF_HD CF_INLINE double4 element_update(const MemberDev& M, const double4 U, cons
     return make_double4(0.0, 0.0, 0.0, 0.0);
   }
   return element_update_full<S>(M, U, st, s0, s1, s2, dt, nonfinite);
+}
+
+/* ---- one momentum component of an element ------------------------------------------------- */
+
+/* The update of an element (element_update_full) by two lanes in lockstep, one for each component of the
+ * momentum: comp 0 works on hu, comp 1 on hv, with the same formulas under the exchange of the two, and
+ * both carry the depth.  x[] is offered to the other lane, y[] is what it offers (as EdgeSide).
+ * Stages: velocity (x: u, u^2); friction (x: diagonal entry, first-column entry, ri); update. */
+template <class T>
+struct ElemSide {
+  int comp;
+  T x[3], y[3];
+  T q1, q, rc1, rcq, sb, vel, sq, ri, ri1, diag, a1, a23, h, qn;
+  bool wet, fast, impl;
+
+  /* U: the state; rc1_, rcq_, sb_: the sums of the depth flux, of this component's flux and bed source */
+  CF_HD CF_INLINE void velocity(const MemberDev& M, int comp_, const double4& U, double rc1_, double rcq_, double sb_) {
+    comp = comp_;
+    q1 = T(U.x);
+    q = T(comp ? U.z : U.y);
+    rc1 = T(rc1_);
+    rcq = T(rcq_);
+    sb = T(sb_);
+    wet = M.friction == 1 && q1 > M.tolisec;
+    vel = sq = T(0.0);
+    if (wet) {
+      vel = div_rn(q, q1, recip_h(q1, U.w));
+      sq = vel * vel;
+    }
+    x[0] = vel;
+    x[1] = sq;
+  }
+  CF_HD CF_INLINE void friction(const MemberDev& M, const double4& U, const double4& st, double dt) {
+    const double gp = M.gp, area = st.x, tol = M.tol;
+    T sf = T(0.0);
+    fast = false;
+    impl = M.friction == 1 && (M.fricimplic == 1 || M.fricimplic == 2);
+    diag = T(1.0);
+    a1 = T(0.0);
+    a23 = T(0.0);
+    if (wet) {
+      const T n = T(st.y), ot = y[0];
+      T nv = sqrt(sq + y[1]);
+      if (nv < tol) nv = T(tol);
+      const T p13 = rcbrt(q1);
+      sf = -(gp * n * n * vel * nv * area * p13);
+      fast = impl && nv > tol;
+      if (fast) {
+        const T p43 = div_rn(p13, q1, recip_h(q1, U.w));
+        if (M.fricimplic == 1) {
+          const auto yn = recip(nv);
+          const T d = T(ConstOps<T>::half(dt)) * gp * n * n * p43;
+          diag = 1.0 + div_rn(d * (twice(sq) + y[1]), nv, yn);
+          a1 = -(7.0 / 3.0 * d * vel * nv);
+          a23 = div_rn(d * (comp ? ot : vel) * (comp ? vel : ot), nv, yn);
+        } else {
+          const T beta = -(dt * gp * n * n * nv * p43);
+          diag = (1. - beta) / ((1. - beta) * (1. - beta));
+        }
+      }
+    }
+    if (M.friction == 1) {
+      ri1 = div_rn(zero_minus(rc1), area, st.w);
+      ri = div_rn(sb + sf - rcq, area, st.w);
+    } else {
+      ri1 = div_rn(zero_minus(rc1), area, st.w);
+      ri = div_rn(sb - rcq, area, st.w);
+    }
+    x[0] = diag;
+    x[1] = a1;
+    x[2] = ri;
+  }
+  /* the new depth and momentum component; false when one is not finite */
+  CF_HD CF_INLINE bool update(const MemberDev& M, double dt) {
+    const T ro = y[2];
+    T r1 = ri1, r = ri;
+    if (impl) {
+      r1 = first_row(ri1, ri, ro);
+      if (fast && M.fricimplic == 1) {
+        const T det = diag * y[0] - a23 * a23;
+        const auto yd = recip(det);
+        /* the other side's row is the same with the roles exchanged: -(a b - c) = c - a b */
+        const T ma = div_rn(a23 * y[1] - a1 * y[0], det, yd);
+        const T own = div_rn(y[0], det, yd) * ri, oth = div_rn(-a23, det, yd) * ro;
+        r = ma * ri1 + (comp ? oth : own) + (comp ? own : oth);
+      } else if (fast) {
+        r = first_row(diag * ri, ri1, ro);
+      } else {
+        r = first_row(ri, ri1, ro);
+      }
+    }
+    h = q1 + dt * r1;
+    qn = q + dt * r;
+    const bool ok = finite_val(h) && finite_val(qn);
+    if (h <= M.tolisec) {
+      h = T(0.);
+      qn = T(0.);
+    }
+    return ok;
+  }
+};
+
+/* element_update_full by its two components, on the host */
+template <class T>
+inline double4 element_update_pair(const MemberDev& M, const double4& U, const double4& st, const Slot& s0,
+                                   const Slot& s1, const Slot& s2, double dt, bool& nonfinite) {
+  ElemSide<T> e[2];
+  e[0].velocity(M, 0, U, s0.f1 + s1.f1 + s2.f1, s0.f2 + s1.f2 + s2.f2, s0.bx + s1.bx + s2.bx);
+  e[1].velocity(M, 1, U, s0.f1 + s1.f1 + s2.f1, s0.f3 + s1.f3 + s2.f3, s0.by + s1.by + s2.by);
+  auto swap = [&](int n) {
+    for (int k = 0; k < n; ++k) {
+      e[0].y[k] = e[1].x[k];
+      e[1].y[k] = e[0].x[k];
+    }
+  };
+  swap(2);
+  e[0].friction(M, U, st, dt);
+  e[1].friction(M, U, st, dt);
+  swap(3);
+  const bool ok0 = e[0].update(M, dt), ok1 = e[1].update(M, dt);
+  nonfinite = !(ok0 && ok1);
+  const double h = val(e[0].h);
+  return make_double4(h, val(e[0].qn), val(e[1].qn), h > 0.0 ? val(T(1.0) / e[0].h) : 0.0);
 }
 
 }  // namespace cf

@@ -28,6 +28,7 @@
 
 #include <cstdio>
 
+#include "cf_cell_kernel.cuh"
 #include "cf_edge_kernel.cuh"
 #include "cf_flux.h"
 #include "cf_xd.h"
@@ -65,14 +66,6 @@ __global__ void __launch_bounds__(32) k_surf(StepArgs a) {
 /* ---- the element kernel ----------------------------------------------------------------- */
 
 __device__ __forceinline__ unsigned long long dbits(double x) { return (unsigned long long)__double_as_longlong(x); }
-
-__device__ __forceinline__ Slot load_slot(const Slot* p) {
-  const double2* q = reinterpret_cast<const double2*>(p);
-  const double2 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2);
-  Slot s;
-  s.f1 = a.x; s.f2 = a.y; s.f3 = b.x; s.bx = b.y; s.by = c.x; s.q = c.y;
-  return s;
-}
 
 /* Minimum over the block, folded into *target with one atomic.  The values are positive (or
  * NaN, which the minimum ignores as fmin would), so they order like their bit patterns: the
@@ -167,19 +160,14 @@ __device__ __forceinline__ void block_cfl_min(const MemberDev& M, bool active, d
   block_min_atomic<BC>(dti, target);
 }
 
-/* 1024 threads per SM (at most 64 registers; 116 bytes spilled): the element update is a chain of
- * dependent integer-pipe quotients and products, and since the dry-region shortcuts most of the
- * kernel's time is memory latency, which more warps hide (1M WAF step, tuned, 256-thread blocks:
- * 0.152 -> 0.130 ms from two to three blocks per SM before the shortcuts; 0.088 -> 0.082 ms from
- * three to four after them).  A block of BC threads (128 or 256, the launch shape) lies within one
- * tile of TILE_C elements, so within one member; each block folds its dt minimum into the member's
- * with one atomic.  SUMS (the recording forward) also stores the element's slot sums; it is a
- * separate instantiation because the compiler shares those sums with the general update's and then
- * forms them ahead of the dry-element test, for every element (1M WAF step: 9 -> 19 FP64 sums per
- * element, 0.088 -> 0.098 ms). */
-template <int BC, bool SUMS>
+/* The element kernel: LANES lanes per element, 1024 threads per SM (at most 64 registers).  A block of BC
+ * threads (128 or 256, the launch shape) lies within one tile of TILE_C elements, so within one member;
+ * each block folds its dt minimum into the member's with one atomic.  SUMS (the recording forward) also
+ * stores the element's slot sums; it is a separate instantiation because it needs the slots of every
+ * element (and on one lane the compiler would form those sums ahead of the dry-element test). */
+template <int BC, bool SUMS, int LANES>
 __global__ void __launch_bounds__(BC, 1024 / BC) k_cells(StepArgs a) {
-  const int c0 = a.c_lo + blockIdx.x * BC;   /* the block's first element (c_lo: a part's phase) */
+  const int c0 = a.c_lo + blockIdx.x * (BC / LANES);   /* the block's first element (c_lo: a part's phase) */
   const int tile = c0 / TILE_C;
   const int m = __ldg(a.ctile_mem + tile);
   const MemberDev& M = a.mdev[m];
@@ -191,12 +179,14 @@ __global__ void __launch_bounds__(BC, 1024 / BC) k_cells(StepArgs a) {
   __syncthreads();
   if (s_stop) return;
   const double dt = S->dt[p];
-  const int c = c0 + threadIdx.x;
-  const int cend = min(M.cell_end, a.c_hi);
-  double4 V = make_double4(0.0, 0.0, 0.0, 0.0);
-  double cflL = 0.0;
-  if (c < cend) {
-    const double4 U = ld4(a.Uin + c);
+  const int c = c0 + threadIdx.x / LANES, comp = threadIdx.x % LANES;
+  const bool active = c < min(M.cell_end, a.c_hi);
+  double4 U = make_double4(0.0, 0.0, 0.0, 0.0), st = U, V = U;
+  Slot s0, s1, s2;
+  CompSums sums = {0.0, 0.0, 0.0, false};
+  bool run = false, nonfinite = false;
+  if (active) {
+    U = ld4(a.Uin + c);
     /* a dry element amid dry ones (most of an unflooded plain): its slots are signed zeros and
      * its update is +0, known from four depths and its neighbour entry, without its slots or its
      * statics (a dry element's CFL value does not use its length) */
@@ -207,30 +197,40 @@ __global__ void __launch_bounds__(BC, 1024 / BC) k_cells(StepArgs a) {
             dry_neighbourhood(M, nb, U, [&](int k) { return ldro(reinterpret_cast<const double*>(a.Uin + k)); });
     }
     if (!dry) {
-      const double4 st = ld4(a.cstat + c);   /* area, manning n, cfl L, - */
+      run = true;
+      st = ld4(a.cstat + c);   /* area, manning n, cfl L, 1/area */
       const int4 sl = __ldg(a.cslot + c);
-      const Slot s0 = load_slot(a.slots + sl.x);
-      const Slot s1 = load_slot(a.slots + sl.y);
-      const Slot s2 = load_slot(a.slots + sl.z);
-      if (SUMS) {
-        /* the sums element_update forms (same expressions, same values) */
-        double2* q = reinterpret_cast<double2*>(a.sums_out + c);
-        q[0] = make_double2(s0.f1 + s1.f1 + s2.f1, s0.f2 + s1.f2 + s2.f2);
-        q[1] = make_double2(s0.f3 + s1.f3 + s2.f3, s0.bx + s1.bx + s2.bx);
-        q[2] = make_double2(s0.by + s1.by + s2.by, 0.0);
+      if (LANES == 2) {
+        sums = comp_sums(a.slots, sl, comp);
+        if (SUMS) store_comp_sums(a.sums_out + c, sums, comp);
+      } else {
+        s0 = load_slot(a.slots + sl.x);
+        s1 = load_slot(a.slots + sl.y);
+        s2 = load_slot(a.slots + sl.z);
+        if (SUMS) store_sums(a.sums_out + c, s0, s1, s2);
       }
-      bool nonfinite = false;
-      /* bit 4 of xd_mul_mask: the element's arithmetic on the integer pipes (cf_xd.h) */
-      if (a.xd_cmp && (a.xd_mul_mask & XD_CELLS)) V = element_update<XD<true>>(M, U, st, s0, s1, s2, dt, nonfinite);
-      else V = element_update(M, U, st, s0, s1, s2, dt, nonfinite);
-      if (nonfinite) atomicOr(&S->status, CF_STATUS_NONFINITE);
-      cflL = st.z;
     }
-    double4* o = a.Uout + c;
-    reinterpret_cast<double2*>(o)[0] = make_double2(V.x, V.y);
-    reinterpret_cast<double2*>(o)[1] = make_double2(V.z, V.w);
   }
-  block_cfl_min<BC>(M, c < cend, cflL, V, &S->dt[1 - p]);
+  if (LANES == 2) V = cell_lanes(a, M, comp, run, U, st, sums, dt, nonfinite);
+  else if (run) V = cell_thread(a, M, U, st, s0, s1, s2, dt, nonfinite);
+  if (nonfinite) atomicOr(&S->status, CF_STATUS_NONFINITE);
+  if (active) {
+    double2* o = reinterpret_cast<double2*>(a.Uout + c);
+    if (LANES == 2) {
+      o[comp] = comp ? make_double2(V.z, V.w) : make_double2(V.x, V.y);
+    } else {
+      o[0] = make_double2(V.x, V.y);
+      o[1] = make_double2(V.z, V.w);
+    }
+  }
+  block_cfl_min<BC>(M, active && comp == 0, st.z, V, &S->dt[1 - p]);
+}
+
+/* n elements (whole tiles, or a part's range) in blocks of bc lanes */
+template <int BC, bool SUMS>
+void launch_cells(const StepArgs& a, int n, cudaStream_t st) {
+  if (two_lanes(a)) k_cells<BC, SUMS, 2><<<(2 * n + BC - 1) / BC, BC, 0, st>>>(a);
+  else k_cells<BC, SUMS, 1><<<(n + BC - 1) / BC, BC, 0, st>>>(a);
 }
 
 /* CFL of a state into mst[m].dt[slot] (the initial dt, finite_volumes_method.cuf:113-116). */
@@ -632,9 +632,10 @@ int launch_step(const StepArgs& a, stream_t s, void* ev_mid, void* ev_end) {
   }
   if (rc != CF_OK) return rc;
   if (ev_mid) cudaEventRecord(reinterpret_cast<cudaEvent_t>(ev_mid), st);
-  if (a.sums_out) k_cells<TILE_C, true><<<a.n_ctiles, TILE_C, 0, st>>>(a);
-  else if (a.cblock == 128) k_cells<128, false><<<a.n_ctiles * (TILE_C / 128), 128, 0, st>>>(a);
-  else k_cells<TILE_C, false><<<a.n_ctiles, TILE_C, 0, st>>>(a);
+  const int n = a.n_ctiles * TILE_C;
+  if (a.sums_out) launch_cells<128, true>(a, n, st);
+  else if (a.cblock == 128) launch_cells<128, false>(a, n, st);
+  else launch_cells<256, false>(a, n, st);
   if (a.steady) k_discharge<<<a.nmembers, 256, 0, st>>>(a.slots, a.ecell, a.bq, a.mdev, a.mst, 1);
   if (ev_end) cudaEventRecord(reinterpret_cast<cudaEvent_t>(ev_end), st);
   return check(cudaGetLastError());
@@ -693,9 +694,8 @@ int launch_part_phase(const StepArgs& a, int phase, const int32_t* elist, int32_
     StepArgs b = a;
     b.c_lo = c_lo;
     b.c_hi = c_hi;
-    const int nb = (c_hi - c_lo + TILE_C - 1) / TILE_C;
-    if (b.sums_out) k_cells<TILE_C, true><<<nb, TILE_C, 0, st>>>(b);
-    else k_cells<TILE_C, false><<<nb, TILE_C, 0, st>>>(b);
+    if (b.sums_out) launch_cells<128, true>(b, c_hi - c_lo, st);
+    else launch_cells<128, false>(b, c_hi - c_lo, st);
   }
   return check(cudaGetLastError());
 }

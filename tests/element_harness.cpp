@@ -97,3 +97,48 @@ extern "C" double harness_adj_nearly_dry(long long n, unsigned long long seed) {
   }
   return worst;
 }
+
+/* element_update_pair (the two lanes of the element kernel) against element_update_full on n random
+ * elements of every friction option and arithmetic type; the number of different results (zeros of
+ * either sign are equal). */
+extern "C" long long harness_element_pair(long long n, unsigned long long seed) {
+  unsigned long long s = seed | 1;
+  auto rnd = [&]() { s ^= s << 13; s ^= s >> 7; s ^= s << 17; return s; };
+  auto unif = [&]() { return (double)(rnd() >> 11) * (1.0 / 9007199254740992.0); };
+  auto sym = [&]() { return rnd() % 12 == 0 ? 0.0 : 2.0 * unif() - 1.0; };
+  auto same = [](double a, double b) { return a == b || (a != a && b != b); };
+  long long bad = 0;
+  for (long long i = 0; i < n; ++i) {
+    MemberDev M;
+    std::memset(&M, 0, sizeof(M));
+    M.gp = 9.81; M.tolisec = rnd() % 4 ? 1e-4 : 0.0; M.tol = (double)1e-6f;
+    M.friction = (int)(rnd() % 4 != 0); M.fricimplic = (int)(rnd() % 3);
+    const double h = rnd() % 5 == 0 ? (rnd() % 2 ? 2e-4 * unif() : 0.0) : 0.01 + 3.0 * unif();
+    const double vel = rnd() % 4 == 0 ? 0.0 : (rnd() % 4 == 0 ? 3e-6 : 2.0);
+    const double4 U = make_double4(h, h * vel * sym(), h * vel * sym(), h > 0.0 ? 1.0 / h : 0.0);
+    const double area = 0.5 + 3.0 * unif();
+    const double4 st = make_double4(area, rnd() % 16 == 0 ? 0.0 : 0.01 + 0.05 * unif(), 0.0, 1.0 / area);
+    Slot c[3];
+    for (int k = 0; k < 3; ++k) {
+      double* f = &c[k].f1;
+      for (int j = 0; j < 6; ++j) f[j] = sym();
+      if (rnd() % 50 == 0) f[rnd() % 5] = rnd() % 2 ? INFINITY : NAN;
+    }
+    const double dt = 0.3 * unif();
+    const int xd = (int)(rnd() % 3);
+    bool n0 = false, n1 = false;
+    double4 a, b;
+    if (xd == 0) {
+      a = element_update_full<double>(M, U, st, c[0], c[1], c[2], dt, n0);
+      b = element_update_pair<double>(M, U, st, c[0], c[1], c[2], dt, n1);
+    } else if (xd == 1) {
+      a = element_update_full<XD<false>>(M, U, st, c[0], c[1], c[2], dt, n0);
+      b = element_update_pair<XD<false>>(M, U, st, c[0], c[1], c[2], dt, n1);
+    } else {
+      a = element_update_full<XD<true>>(M, U, st, c[0], c[1], c[2], dt, n0);
+      b = element_update_pair<XD<true>>(M, U, st, c[0], c[1], c[2], dt, n1);
+    }
+    if (!(n0 == n1 && same(a.x, b.x) && same(a.y, b.y) && same(a.z, b.z) && same(a.w, b.w))) ++bad;
+  }
+  return bad;
+}

@@ -36,3 +36,9 @@ def test_reverse_edge_with_a_nearly_dry_side_is_the_dual_derivative(lib):
     lib.harness_adj_nearly_dry.argtypes = [C.c_longlong, C.c_ulonglong]
     lib.harness_adj_nearly_dry.restype = C.c_double
     assert lib.harness_adj_nearly_dry(200_000, 9) < 1e-12
+
+
+def test_element_by_two_lanes_is_the_element(lib):
+    lib.harness_element_pair.argtypes = [C.c_longlong, C.c_ulonglong]
+    lib.harness_element_pair.restype = C.c_longlong
+    assert lib.harness_element_pair(600_000, 17) == 0
