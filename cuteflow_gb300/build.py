@@ -25,7 +25,7 @@ CU_SOURCES = ["cf_kernels.cu", "cf_edges_1.cu", "cf_edges_2.cu", "cf_edges_3.cu"
               "cf_adjoint.cu"]
 CPP_SOURCES = ["cf_mesh.cpp", "cf_api.cpp", "cf_adjoint_api.cpp", "cf_io.cpp", "cf_cgns.cpp"]
 HEADERS = ["cf_internal.h", "cf_flux.h", "cf_dual.h", "cf_ctx.h", "cf_xd.h", "cf_edge_kernel.cuh",
-           "cf_cell_kernel.cuh"]
+           "cf_cell_kernel.cuh", "cf_launch.cuh"]
 
 
 def _sources():

@@ -63,8 +63,11 @@ __global__ void __launch_bounds__(2 * TILE_E, 4) k_rep_edges(StepArgs a, const d
   const int m = __ldg(a.etile_mem + tile);
   const MemberDev& M = a.mdev[m];
   const int e = tile * TILE_E + (threadIdx.x >> 1);
+  EdgeHead E;
+  E.load(a, e, e < M.edge_end);
+  pdl_begin();
   const size_t h = hidx(n, m, a.nmembers);
-  edge_lanes<IFLUX>(a, M, e, threadIdx.x & 1, e < M.edge_end, __ldg(dt_hist + h), __ldg(t_hist + h), nullptr);
+  edge_lanes<IFLUX>(a, M, E, e, threadIdx.x & 1, e < M.edge_end, dt_hist[h], t_hist[h], nullptr);
 }
 
 template <int LANES>
@@ -74,7 +77,8 @@ __global__ void __launch_bounds__(128, 8) k_rep_cells(StepArgs a, const double* 
   const int m = __ldg(a.ctile_mem + c / TILE_C);
   const MemberDev& M = a.mdev[m];
   const bool active = c < M.cell_end;
-  const double dt = __ldg(dt_hist + hidx(n, m, a.nmembers));
+  pdl_begin();
+  const double dt = dt_hist[hidx(n, m, a.nmembers)];
   double4 U = make_double4(0.0, 0.0, 0.0, 0.0), st = U, V = U;
   Slot s0, s1, s2;
   CompSums sums = {0.0, 0.0, 0.0, false};
@@ -114,6 +118,7 @@ __global__ void __launch_bounds__(128, 8) k_rep_cells(StepArgs a, const double* 
  * member's dt and start time of the step (read from its record of parity p). */
 __global__ void k_record(const double4* Unew, const double* zcell, const MemberState* S, int nm, int p, int n,
                          double* dt_hist, double* t_hist, const int32_t* gcell, int G, double* eta) {
+  pdl_begin();
   for (int g = threadIdx.x; g < G; g += blockDim.x) {
     const int c = gcell[g];
     eta[(size_t)n * G + g] = Unew[c].x + zcell[c];
@@ -146,7 +151,7 @@ __device__ __forceinline__ double4 gather_lambda(const AdjArgs& A, int c, const 
     }
   }
   if (gw)
-    for (int j = __ldg(A.goff + c), j1 = __ldg(A.goff + c + 1); j < j1; ++j) L.x += __ldg(gw + __ldg(A.gidx + j));
+    for (int j = __ldg(A.goff + c), j1 = __ldg(A.goff + c + 1); j < j1; ++j) L.x += gw[__ldg(A.gidx + j)];
   return L;
 }
 
@@ -161,9 +166,10 @@ __global__ void __launch_bounds__(ADJ_CELLS_BLOCK, 6) k_adj_cells(AdjArgs A) {
   const int c = blockIdx.x * ADJ_CELLS_BLOCK + threadIdx.x;
   const int mem = __ldg(a.ctile_mem + c / TILE_C);
   const MemberDev& M = a.mdev[mem];
+  pdl_begin();
   if (c >= M.cell_end) return;
   const double4 L = A.gather ? gather_lambda(A, c, A.gw) : ld4(A.lam_init + c);
-  const double dt = __ldg(A.dt_hist + hidx(A.n, mem, a.nmembers));
+  const double dt = A.dt_hist[hidx(A.n, mem, a.nmembers)];
   const Slot sums = load_slot(A.sums + c);
   double4 own;
   Slot w;
@@ -272,9 +278,10 @@ __global__ void __launch_bounds__(TILE_E) k_adj_edges(AdjArgs A) {
   const int m = __ldg(a.etile_mem + tile);
   const MemberDev& M = a.mdev[m];
   const int e = tile * TILE_E + threadIdx.x;
+  pdl_begin();
   if (e >= M.edge_end) return;
   const size_t h = hidx(A.n, m, a.nmembers);
-  const double dt = __ldg(A.dt_hist + h), t = __ldg(A.t_hist + h);
+  const double dt = A.dt_hist[h], t = A.t_hist[h];
   const int2 ab = ldro(a.ecell + e);
   if (ab.y < 0) adj_boundary_edge<IFLUX>(A, M, e, ab, t);
   else adj_interior_edge<IFLUX, D>(A, M, e, ab, dt);
@@ -317,6 +324,7 @@ __global__ void __launch_bounds__(2 * TILE_E, 3) k_adj_edges_hllc(AdjArgs A) {
   const int m = __ldg(a.etile_mem + tile);
   const MemberDev& M = a.mdev[m];
   const int e = tile * TILE_E + (threadIdx.x >> 1), side = threadIdx.x & 1;
+  pdl_begin();
   const bool live = e < M.edge_end;
   int2 ab = make_int2(0, -3);
   if (live) ab = ldro(a.ecell + e);
@@ -334,7 +342,7 @@ __global__ void __launch_bounds__(2 * TILE_E, 3) k_adj_edges_hllc(AdjArgs A) {
     adj_stages(p);
     A.eadj[2 * (size_t)e + side] = make_double4(p.lam[0], p.lam[1], p.lam[2], 0.0);
   } else if (live && side == 0) {
-    adj_boundary_edge<1>(A, M, e, ab, __ldg(A.t_hist + hidx(A.n, m, a.nmembers)));
+    adj_boundary_edge<1>(A, M, e, ab, A.t_hist[hidx(A.n, m, a.nmembers)]);
   }
 }
 
@@ -405,34 +413,34 @@ int launch_replay_step(const StepArgs& a, const double* dt_hist, const double* t
                        Slot* sums, stream_t s) {
   cudaStream_t st = reinterpret_cast<cudaStream_t>(s);
   switch (a.iflux) {
-    case 1: k_rep_edges<1><<<a.n_etiles, 2 * TILE_E, 0, st>>>(a, dt_hist, t_hist, n); break;
-    case 2: k_rep_edges<2><<<a.n_etiles, 2 * TILE_E, 0, st>>>(a, dt_hist, t_hist, n); break;
-    case 3: k_rep_edges<3><<<a.n_etiles, 2 * TILE_E, 0, st>>>(a, dt_hist, t_hist, n); break;
+    case 1: launch_pdl(k_rep_edges<1>, a.n_etiles, 2 * TILE_E, st, a, dt_hist, t_hist, n); break;
+    case 2: launch_pdl(k_rep_edges<2>, a.n_etiles, 2 * TILE_E, st, a, dt_hist, t_hist, n); break;
+    case 3: launch_pdl(k_rep_edges<3>, a.n_etiles, 2 * TILE_E, st, a, dt_hist, t_hist, n); break;
     default: return CF_ENOTSUP;
   }
   const int nc = a.n_ctiles * TILE_C;
-  if (two_lanes(a)) k_rep_cells<2><<<2 * nc / 128, 128, 0, st>>>(a, dt_hist, n, flag, sums);
-  else k_rep_cells<1><<<nc / 128, 128, 0, st>>>(a, dt_hist, n, flag, sums);
+  if (two_lanes(a)) launch_pdl(k_rep_cells<2>, 2 * nc / 128, 128, st, a, dt_hist, n, flag, sums);
+  else launch_pdl(k_rep_cells<1>, nc / 128, 128, st, a, dt_hist, n, flag, sums);
   return chk(cudaGetLastError());
 }
 
 int launch_record(const double4* Unew, const double* zcell, const MemberState* S, int nm, int p, int n, double* dt_hist,
                   double* t_hist, const int32_t* gcell, int G, double* eta, stream_t s) {
-  k_record<<<1, 256, 0, reinterpret_cast<cudaStream_t>(s)>>>(Unew, zcell, S, nm, p, n, dt_hist, t_hist, gcell, G, eta);
+  launch_pdl(k_record, 1, 256, reinterpret_cast<cudaStream_t>(s), Unew, zcell, S, nm, p, n, dt_hist, t_hist, gcell, G, eta);
   return chk(cudaGetLastError());
 }
 
 int launch_adjoint_step(const AdjArgs& A, stream_t s) {
   cudaStream_t st = reinterpret_cast<cudaStream_t>(s);
   const StepArgs& a = A.s;
-  k_adj_cells<<<a.n_ctiles * (TILE_C / ADJ_CELLS_BLOCK), ADJ_CELLS_BLOCK, 0, st>>>(A);
+  launch_pdl(k_adj_cells, a.n_ctiles * (TILE_C / ADJ_CELLS_BLOCK), ADJ_CELLS_BLOCK, st, A);
   switch (a.iflux) {
     case 1:
-      if (a.flux_mode == 0) k_adj_edges_hllc<<<a.n_etiles, 2 * TILE_E, 0, st>>>(A);
-      else k_adj_edges<1, 6><<<a.n_etiles, TILE_E, 0, st>>>(A);
+      if (a.flux_mode == 0) launch_pdl(k_adj_edges_hllc, a.n_etiles, 2 * TILE_E, st, A);
+      else launch_pdl(k_adj_edges<1, 6>, a.n_etiles, TILE_E, st, A);
       break;
-    case 2: k_adj_edges<2, 3><<<a.n_etiles, TILE_E, 0, st>>>(A); break;
-    case 3: k_adj_edges<3, 2><<<a.n_etiles, TILE_E, 0, st>>>(A); break;
+    case 2: launch_pdl(k_adj_edges<2, 3>, a.n_etiles, TILE_E, st, A); break;
+    case 3: launch_pdl(k_adj_edges<3, 2>, a.n_etiles, TILE_E, st, A); break;
     default: return CF_ENOTSUP;
   }
   return chk(cudaGetLastError());

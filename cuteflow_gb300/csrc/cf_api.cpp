@@ -10,8 +10,8 @@
  *
  * Stepping never returns to the host between steps: the next dt of every member is produced on
  * the device by the element kernel and read by the next edge kernel.  The host reads the small
- * per-member records once at the end of a cf_step call.  Runs of steps are replayed from a
- * captured CUDA graph of two steps (even and odd buffer parity).
+ * per-member records once at the end of a cf_step call.  Runs of steps are replayed from captured
+ * CUDA graphs of GRAPH_RUN and of two steps (even and odd buffer parity).
  */
 #include <cuda_runtime.h>
 
@@ -89,8 +89,16 @@ StepArgs step_args(const cf_ctx* c, int parity) {
   return a;
 }
 
+/* the captured steps (they hold the settings and launch shape of their capture) */
+void drop_graphs(cf_ctx* c) {
+  for (cudaGraphExec_t* g : {&c->graph2, &c->graph_run}) {
+    if (*g) cudaGraphExecDestroy(*g);
+    *g = nullptr;
+  }
+}
+
 void free_all(cf_ctx* c) {
-  if (c->graph2) cudaGraphExecDestroy(c->graph2);
+  drop_graphs(c);
   void* ptrs[] = {c->U[0], c->U[1], c->cslot, c->cnbr, c->cstat, c->zcell, c->perm, c->iperm, c->ecell, c->egeo, c->ez,
                   c->ebid, c->eupw, c->ewts, c->edk, c->einv, c->slots, c->etile_mem, c->ctile_mem, c->mdev,
                   c->mst, c->staging, c->inl_cell, c->inl_len, c->ids, c->bq, c->elist1, c->elist2,
@@ -138,18 +146,19 @@ int enqueue_step(cf_ctx* c, int parity, bool timed) {
   return CF_OK;
 }
 
-int build_graph(cf_ctx* c) {
+/* capture nsteps steps (an even number, from parity 0) into *out */
+int build_graph(cf_ctx* c, int nsteps, cudaGraphExec_t* out) {
   cudaGraph_t g = nullptr;
   CF_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-  int rc0 = enqueue_step(c, 0, false);
-  int rc1 = rc0 == CF_OK ? enqueue_step(c, 1, false) : rc0;
+  int rc = CF_OK;
+  for (int k = 0; k < nsteps && rc == CF_OK; ++k) rc = enqueue_step(c, k & 1, false);
   cudaError_t e = cudaStreamEndCapture(c->stream, &g);
-  if (rc1 != CF_OK) {
+  if (rc != CF_OK) {
     if (g) cudaGraphDestroy(g);
-    return rc1;
+    return rc;
   }
   if (e != cudaSuccess) return cuda_fail(c, e, "cudaStreamEndCapture");
-  e = cudaGraphInstantiate(&c->graph2, g, 0);
+  e = cudaGraphInstantiate(out, g, 0);
   cudaGraphDestroy(g);
   if (e != cudaSuccess) return cuda_fail(c, e, "cudaGraphInstantiate");
   return CF_OK;
@@ -575,8 +584,12 @@ int enqueue_steps(cf_ctx* c, int32_t nsteps) {
       if ((rc = enqueue_step(c, 1, false))) return rc;
       --left;
     }
+    if (c->use_graph && left >= GRAPH_RUN) {
+      if (!c->graph_run && (rc = build_graph(c, GRAPH_RUN, &c->graph_run))) return rc;
+      for (; left >= GRAPH_RUN; left -= GRAPH_RUN) CF_CUDA(c, cudaGraphLaunch(c->graph_run, c->stream));
+    }
     if (c->use_graph && left >= 2) {
-      if (!c->graph2 && (rc = build_graph(c))) return rc;
+      if (!c->graph2 && (rc = build_graph(c, 2, &c->graph2))) return rc;
       for (; left >= 2; left -= 2) CF_CUDA(c, cudaGraphLaunch(c->graph2, c->stream));
     }
     while (left > 0) {
@@ -728,10 +741,9 @@ int cf_set_tuning(cf_ctx* ctx, int32_t int_compare, int32_t int_mul_warps) {
   if (ctx->xd_cmp != int_compare || ctx->xd_mul_mask != int_mul_warps) {
     ctx->xd_cmp = int_compare;
     ctx->xd_mul_mask = int_mul_warps;
-    if (ctx->graph2) {   /* the captured steps hold the old arguments */
+    if (ctx->graph2 || ctx->graph_run) {   /* the captured steps hold the old arguments */
       CF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-      cudaGraphExecDestroy(ctx->graph2);
-      ctx->graph2 = nullptr;
+      drop_graphs(ctx);
     }
   }
   return CF_OK;
@@ -804,10 +816,9 @@ int cf_set_launch_shape(cf_ctx* ctx, int32_t edge_block, int32_t edges_per_threa
     ctx->eblock = edge_block;
     ctx->ept = edges_per_thread;
     ctx->cblock = cell_block;
-    if (ctx->graph2) {   /* the captured steps hold the old launch configuration */
+    if (ctx->graph2 || ctx->graph_run) {   /* the captured steps hold the old launch configuration */
       CF_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-      cudaGraphExecDestroy(ctx->graph2);
-      ctx->graph2 = nullptr;
+      drop_graphs(ctx);
     }
   }
   return CF_OK;

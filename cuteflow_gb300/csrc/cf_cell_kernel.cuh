@@ -26,7 +26,7 @@ inline bool two_lanes(const StepArgs& a) { return a.n_ctiles * TILE_C <= TWO_LAN
 
 __device__ __forceinline__ Slot load_slot(const Slot* p) {
   const double2* q = reinterpret_cast<const double2*>(p);
-  const double2 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2);
+  const double2 a = q[0], b = q[1], c = q[2];
   Slot s;
   s.f1 = a.x; s.f2 = a.y; s.f3 = b.x; s.bx = b.y; s.by = c.x; s.q = c.y;
   return s;
@@ -56,9 +56,9 @@ __device__ __forceinline__ CompSums comp_sums(const Slot* slots, const int4& sl,
   uint64_t z = 0;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    f[k] = __ldg(p[k]);
-    q[k] = __ldg(p[k] + 1 + comp);
-    b[k] = __ldg(p[k] + 3 + comp);
+    f[k] = p[k][0];
+    q[k] = p[k][1 + comp];
+    b[k] = p[k][3 + comp];
     z |= dbits_hd(f[k]) | dbits_hd(q[k]) | dbits_hd(b[k]);
   }
   CompSums s;

@@ -18,6 +18,8 @@
 
 namespace cf {
 
+constexpr int GRAPH_RUN = 16;   /* steps of the longer captured graph */
+
 /* One simulation of a context: its inputs, host tables and place in the flat space. */
 struct Member {
   cf_params params{};
@@ -93,6 +95,7 @@ struct cf_ctx {
   /* stepping */
   int64_t launched = 0;                /* steps launched since creation (buffer parity) */
   cudaGraphExec_t graph2 = nullptr;    /* two steps: parity 0 then 1 */
+  cudaGraphExec_t graph_run = nullptr; /* GRAPH_RUN steps */
   bool use_graph = true;
   /* timing */
   bool timing = false;

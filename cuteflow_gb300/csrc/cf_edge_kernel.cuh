@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 
 #include "cf_flux.h"
+#include "cf_launch.cuh"
 #include "cf_xd.h"
 
 namespace cf {
@@ -90,20 +91,33 @@ __device__ __forceinline__ void edge_side(const StepArgs& a, const MemberDev& M,
   store_side(a.slots + 2 * (size_t)e + side, p.out, geo.z);
 }
 
+/* What every path of an edge reads of the mesh's tables: loaded before the kernel waits for the one
+ * before it. */
+struct EdgeHead {
+  int2 ab;
+  double4 geo;
+  __device__ __forceinline__ void load(const StepArgs& a, int e, bool live) {
+    ab = make_int2(0, -3);
+    geo = make_double4(0.0, 0.0, 0.0, 0.0);
+    if (live) {
+      ab = ldro(a.ecell + e);
+      const double2* q = reinterpret_cast<const double2*>(a.egeo + e);
+      const double2 u = ldro(q), v = ldro(q + 1);
+      geo = make_double4(u.x, u.y, v.x, v.y);
+    }
+  }
+};
+
 /* Edge e of a step on the lanes of its two sides, in the context's arithmetic type.  Every lane of the
  * warp comes here; live: the lane's edge is one to evaluate (the 16 edges of a warp belong to one
  * tile, so to one member and one setting of the integer-pipe mask). */
 template <int IFLUX>
-__device__ __forceinline__ void edge_lanes(const StepArgs& a, const MemberDev& M, int e, int side, bool live, double dt,
-                                           double t, const double* surf) {
-  int2 ab = make_int2(0, -3);
-  double4 geo = make_double4(0.0, 0.0, 0.0, 0.0), U = geo;
-  if (live) {
-    /* the normal and length, which every path needs, load beside the element's state */
-    ab = ldro(a.ecell + e);
-    geo = ld4(a.egeo + e);
-    U = ld4(a.Uin + ((side && ab.y >= 0) ? ab.y : ab.x));   /* {h, hu, hv, RN(1/h)} */
-  }
+__device__ __forceinline__ void edge_lanes(const StepArgs& a, const MemberDev& M, const EdgeHead& E, int e, int side,
+                                           bool live, double dt, double t, const double* surf) {
+  const int2 ab = E.ab;
+  const double4 geo = E.geo;
+  double4 U = make_double4(0.0, 0.0, 0.0, 0.0);
+  if (live) U = ld4(a.Uin + ((side && ab.y >= 0) ? ab.y : ab.x));   /* {h, hu, hv, RN(1/h)} */
   const double hp = __shfl_xor_sync(0xffffffffu, U.x, 1);
   bool run = live && ab.y >= 0;
   if (run && (dbits_hd(U.x) | dbits_hd(hp)) == 0 && dry_edge_ok<IFLUX>(M.gp, geo, dt)) {
@@ -139,11 +153,14 @@ __global__ void __launch_bounds__(BE, ((IFLUX == 4) ? 512 : 1024) / BE) k_edges(
     const int m = __ldg(a.etile_mem + e / TILE_E);
     const MemberDev& M = a.mdev[m];
     MemberState* S = a.mst + m;
+    EdgeHead E;
+    E.load(a, e, e < M.edge_end);
+    if (j == 0) pdl_begin();
     if (S->status) continue;
     const double dt = S->dt[p];
     const double t = S->t[p];
     if (i == 2 * M.edge_begin) step_start(M, S, p);
-    edge_lanes<IFLUX>(a, M, e, i & 1, e < M.edge_end, dt, t, S->surf);
+    edge_lanes<IFLUX>(a, M, E, e, i & 1, e < M.edge_end, dt, t, S->surf);
   }
 }
 
@@ -156,14 +173,16 @@ __global__ void __launch_bounds__(TILE_E, (IFLUX == 4) ? 4 : 8) k_edges_list(Ste
   MemberState* S = a.mst;
   if (S->status) return;
   const int e = i < n ? list[i] : 0;
-  edge_lanes<IFLUX>(a, M, e, threadIdx.x & 1, i < n && e < M.edge_end, S->dt[a.parity], S->t[a.parity], S->surf);
+  EdgeHead E;
+  E.load(a, e, i < n && e < M.edge_end);
+  edge_lanes<IFLUX>(a, M, E, e, threadIdx.x & 1, i < n && e < M.edge_end, S->dt[a.parity], S->t[a.parity], S->surf);
 }
 
 template <int IFLUX, int BE, int EPT>
 void launch_edges_shape(const StepArgs& a, cudaStream_t st) {
   const int nside = 2 * a.n_etiles * TILE_E;
   const int per = BE * EPT;
-  k_edges<IFLUX, BE, EPT><<<(nside + per - 1) / per, BE, 0, st>>>(a);
+  launch_pdl(k_edges<IFLUX, BE, EPT>, (nside + per - 1) / per, BE, st, a);
 }
 
 }  // namespace

@@ -51,16 +51,19 @@ using std::sqrt;
 
 /* ---- loads --------------------------------------------------------------------------- */
 
+/* Two 16-byte loads.  Plain ones: states, statics and slots are written by kernels that may still run
+ * when a kernel that overlaps them begins (cf_launch.cuh), which the read-only path does not allow. */
 CF_HD CF_INLINE double4 ld4(const double4* p) {
 #ifdef __CUDA_ARCH__
   const double2* q = reinterpret_cast<const double2*>(p);
-  double2 a = __ldg(q), b = __ldg(q + 1);
+  const double2 a = q[0], b = q[1];
   return make_double4(a.x, a.y, b.x, b.y);
 #else
   return *p;
 #endif
 }
 
+/* the mesh's tables, which no kernel writes */
 template <class T>
 CF_HD CF_INLINE T ldro(const T* p) {
 #ifdef __CUDA_ARCH__

@@ -46,6 +46,7 @@ __global__ void __launch_bounds__(32) k_surf(StepArgs a) {
   const int m = blockIdx.x;
   const MemberDev& M = a.mdev[m];
   MemberState* S = a.mst + m;
+  pdl_begin();
   if (M.inlet != 3 || S->status) return;
   const int lane = threadIdx.x;
   for (int id = 0; id < M.nin; ++id) {
@@ -175,12 +176,20 @@ __global__ void __launch_bounds__(BC, 1024 / BC) k_cells(StepArgs a) {
   const int p = a.parity;
   /* the stop test must be uniform over the block (the dt reduction below synchronises it) */
   __shared__ uint32_t s_stop;
+  const int c = c0 + threadIdx.x / LANES, comp = threadIdx.x % LANES;
+  const bool active = c < min(M.cell_end, a.c_hi);
+  /* the mesh's tables before the wait for the kernel before this one (the slot numbers only on small
+   * meshes: on large ones it is traffic, 16 bytes of each element, that a dry element does not need) */
+  int4 nb = make_int4(0, 0, 0, 0), sl = nb;
+  if (active) {
+    if (!SUMS) nb = __ldg(a.cnbr + c);
+    if (SUMS || LANES == 2) sl = __ldg(a.cslot + c);
+  }
+  pdl_begin();
   if (threadIdx.x == 0) s_stop = *((volatile uint32_t*)&S->status);
   __syncthreads();
   if (s_stop) return;
   const double dt = S->dt[p];
-  const int c = c0 + threadIdx.x / LANES, comp = threadIdx.x % LANES;
-  const bool active = c < min(M.cell_end, a.c_hi);
   double4 U = make_double4(0.0, 0.0, 0.0, 0.0), st = U, V = U;
   Slot s0, s1, s2;
   CompSums sums = {0.0, 0.0, 0.0, false};
@@ -192,14 +201,13 @@ __global__ void __launch_bounds__(BC, 1024 / BC) k_cells(StepArgs a) {
      * statics (a dry element's CFL value does not use its length) */
     bool dry = false;
     if (!SUMS) {
-      const int4 nb = __ldg(a.cnbr + c);
       dry = dry_state_ok(M, U, dt) &&
-            dry_neighbourhood(M, nb, U, [&](int k) { return ldro(reinterpret_cast<const double*>(a.Uin + k)); });
+            dry_neighbourhood(M, nb, U, [&](int k) { return a.Uin[k].x; });
     }
     if (!dry) {
       run = true;
       st = ld4(a.cstat + c);   /* area, manning n, cfl L, 1/area */
-      const int4 sl = __ldg(a.cslot + c);
+      if (!SUMS && LANES == 1) sl = __ldg(a.cslot + c);
       if (LANES == 2) {
         sums = comp_sums(a.slots, sl, comp);
         if (SUMS) store_comp_sums(a.sums_out + c, sums, comp);
@@ -229,8 +237,8 @@ __global__ void __launch_bounds__(BC, 1024 / BC) k_cells(StepArgs a) {
 /* n elements (whole tiles, or a part's range) in blocks of bc lanes */
 template <int BC, bool SUMS>
 void launch_cells(const StepArgs& a, int n, cudaStream_t st) {
-  if (two_lanes(a)) k_cells<BC, SUMS, 2><<<(2 * n + BC - 1) / BC, BC, 0, st>>>(a);
-  else k_cells<BC, SUMS, 1><<<(n + BC - 1) / BC, BC, 0, st>>>(a);
+  if (two_lanes(a)) launch_pdl(k_cells<BC, SUMS, 2>, (2 * n + BC - 1) / BC, BC, st, a);
+  else launch_pdl(k_cells<BC, SUMS, 1>, (n + BC - 1) / BC, BC, st, a);
 }
 
 /* CFL of a state into mst[m].dt[slot] (the initial dt, finite_volumes_method.cuf:113-116). */
@@ -261,6 +269,7 @@ __global__ void __launch_bounds__(256) k_discharge(const Slot* slots, const int2
   __shared__ double si[256], so[256];
   const int m = blockIdx.x;
   const MemberDev& M = mdev[m];
+  pdl_begin();
   double qi = 0.0, qo = 0.0;
   /* the boundary edges in reference order (element, local edge): thread t sums entries t, t + 256,
    * ..., then a fixed tree, an order a decomposed mesh reproduces from its parts' entries */
@@ -621,7 +630,7 @@ int launch_probe_fp64(double* out, int32_t nblocks, int64_t iters, stream_t s) {
 
 int launch_step(const StepArgs& a, stream_t s, void* ev_mid, void* ev_end) {
   cudaStream_t st = reinterpret_cast<cudaStream_t>(s);
-  if (a.phys_inflow) k_surf<<<a.nmembers, 32, 0, st>>>(a);
+  if (a.phys_inflow) launch_pdl(k_surf, a.nmembers, 32, st, a);
   int rc;
   switch (a.iflux) {
     case 1: rc = launch_edges_1(a, s); break;
@@ -636,7 +645,7 @@ int launch_step(const StepArgs& a, stream_t s, void* ev_mid, void* ev_end) {
   if (a.sums_out) launch_cells<128, true>(a, n, st);
   else if (a.cblock == 128) launch_cells<128, false>(a, n, st);
   else launch_cells<256, false>(a, n, st);
-  if (a.steady) k_discharge<<<a.nmembers, 256, 0, st>>>(a.slots, a.ecell, a.bq, a.mdev, a.mst, 1);
+  if (a.steady) launch_pdl(k_discharge, a.nmembers, 256, st, a.slots, a.ecell, a.bq, a.mdev, a.mst, 1);
   if (ev_end) cudaEventRecord(reinterpret_cast<cudaEvent_t>(ev_end), st);
   return check(cudaGetLastError());
 }
