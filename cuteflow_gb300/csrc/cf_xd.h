@@ -487,6 +487,19 @@ struct MulInt {
 };
 XD_HD XD<false> rcbrt(const XD<false>& a) { return XD<false>(rcbrt(a.v)); }
 XD_HD XD<true> rcbrt(const XD<true>& a) { return XD<true>(rcbrt_of<MulInt>(a.v)); }
+template <bool MUL> XD_HD bool is_zero(const XD<MUL>& x) { return xzero(x.v); }
+/* a b with a zero a on the fast path */
+XD_HD XD<false> mulz(const XD<false>& a, const XD<false>& b) { return a * b; }
+XD_HD XD<true> mulz(const XD<true>& a, const XD<true>& b) {
+  uint32_t al, ah, bl, bh;
+  xwords(a.v, al, ah);
+  xwords(b.v, bl, bh);
+  bool bad;
+  double r = em_mul_fast(a.v, b.v, bad);
+  const bool z = (((ah << 1) | al) == 0) & ((~bh & 0x7ff00000u) != 0);
+  if (__builtin_expect(bad & !z, 0)) r = em_mul_rest(a.v, b.v);
+  return XD<true>(z ? xjoin(0u, (ah ^ bh) & 0x80000000u) : r);
+}
 /* 0 - x but for the sign of a zero, which the update adds to a depth */
 template <bool MUL> XD_HD XD<MUL> zero_minus(const XD<MUL>& x) { return -x; }
 /* a where b and c are finite (0 b and 0 c are zeros then) */
