@@ -138,8 +138,10 @@ int status_code(uint32_t st) {
   return CF_OK;
 }
 
-int enqueue_step(cf_ctx* c, int parity, bool timed) {
+int enqueue_step(cf_ctx* c, int parity, bool timed, bool surf_done = false, bool surf_next = false) {
   StepArgs a = step_args(c, parity);
+  a.surf_done = surf_done;
+  a.surf_next = surf_next;
   int rc = launch_step(a, reinterpret_cast<stream_t>(c->stream), timed ? c->ev[1] : nullptr,
                        timed ? c->ev[2] : nullptr);
   if (rc != CF_OK) return fail(c, rc, rc == CF_ENOTSUP ? "iflux not supported by the GPU step" : "kernel launch failed");
@@ -151,7 +153,9 @@ int build_graph(cf_ctx* c, int nsteps, cudaGraphExec_t* out) {
   cudaGraph_t g = nullptr;
   CF_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
   int rc = CF_OK;
-  for (int k = 0; k < nsteps && rc == CF_OK; ++k) rc = enqueue_step(c, k & 1, false);
+  const bool chain = c->any_phys_inflow && c->any_steady;   /* k_between in the graph (its first step has k_surf) */
+  for (int k = 0; k < nsteps && rc == CF_OK; ++k)
+    rc = enqueue_step(c, k & 1, false, chain && k > 0, chain && k + 1 < nsteps);
   cudaError_t e = cudaStreamEndCapture(c->stream, &g);
   if (rc != CF_OK) {
     if (g) cudaGraphDestroy(g);

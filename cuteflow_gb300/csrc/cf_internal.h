@@ -125,7 +125,9 @@ struct StepArgs {
   int32_t iflux, ilimiteur, flux_mode;
   int32_t nmembers;
   int32_t phys_inflow;       /* some member uses inlet 3: k_surf runs before the edges */
-  int32_t steady;            /* some member tests for steady state: k_steady runs after the cells */
+  int32_t steady;            /* some member tests for steady state: k_discharge runs after the cells */
+  int32_t surf_done;         /* phys_inflow and steady: the step before has left this step's inlet sums */
+  int32_t surf_next;         /* ... and this step leaves the next one's (k_between in k_discharge's place) */
   int32_t xd_cmp;            /* edge kernel: 1 = comparisons on integer keys (cf_xd.h) */
   int32_t xd_mul_mask;       /* with xd_cmp: the edges of warp w (0-3) of an edge tile with bit w set,
                                 and with bit 4 (XD_CELLS) the element kernel, form products,
