@@ -58,8 +58,9 @@ __device__ __forceinline__ size_t hidx(int n, int m, int nm) { return (size_t)n 
 /* The replays keep the forward kernels' occupancy, 1024 threads per SM (64 registers), where the latency
  * of the integer-pipe chains is hidden by more warps. */
 template <int IFLUX>
-__global__ void __launch_bounds__(2 * TILE_E, 4) k_rep_edges(StepArgs a, const double* dt_hist, const double* t_hist, int n) {
+__global__ void __launch_bounds__(2 * TILE_E, 4) k_rep_edges(StepArgs a, StepRec r, const double* dt_hist, const double* t_hist, int n) {
   const int tile = blockIdx.x;
+  if (tile == a.n_etiles) return record_gauges(r, a.Uin);
   const int m = __ldg(a.etile_mem + tile);
   const MemberDev& M = a.mdev[m];
   const int e = tile * TILE_E + (threadIdx.x >> 1);
@@ -114,21 +115,8 @@ __global__ void __launch_bounds__(128, 8) k_rep_cells(StepArgs a, const double* 
   }
 }
 
-/* After step n: the gauge elevations h + z of the new state and, when recording, every
- * member's dt and start time of the step (read from its record of parity p). */
-__global__ void k_record(const double4* Unew, const double* zcell, const MemberState* S, int nm, int p, int n,
-                         double* dt_hist, double* t_hist, const int32_t* gcell, int G, double* eta) {
-  pdl_begin();
-  for (int g = threadIdx.x; g < G; g += blockDim.x) {
-    const int c = gcell[g];
-    eta[(size_t)n * G + g] = Unew[c].x + zcell[c];
-  }
-  if (S)
-    for (int m = threadIdx.x; m < nm; m += blockDim.x) {
-      dt_hist[hidx(n, m, nm)] = S[m].dt[p];
-      t_hist[hidx(n, m, nm)] = S[m].t[p];
-    }
-}
+/* The gauge elevations of the last state (a step's edge launch records those of the state before it). */
+__global__ void k_record(StepRec r, const double4* U) { record_gauges(r, U); }
 
 /* ---- adjoint of the element stage --------------------------------------------------------- */
 
@@ -410,12 +398,13 @@ int chk(cudaError_t e) { return e == cudaSuccess ? CF_OK : CF_ECUDA; }
 }  // namespace
 
 int launch_replay_step(const StepArgs& a, const double* dt_hist, const double* t_hist, int n, uint32_t* flag,
-                       Slot* sums, stream_t s) {
+                       Slot* sums, stream_t s, const StepRec& rec) {
   cudaStream_t st = reinterpret_cast<cudaStream_t>(s);
+  const int nb = a.n_etiles + (rec.eta ? 1 : 0);
   switch (a.iflux) {
-    case 1: launch_pdl(k_rep_edges<1>, a.n_etiles, 2 * TILE_E, st, a, dt_hist, t_hist, n); break;
-    case 2: launch_pdl(k_rep_edges<2>, a.n_etiles, 2 * TILE_E, st, a, dt_hist, t_hist, n); break;
-    case 3: launch_pdl(k_rep_edges<3>, a.n_etiles, 2 * TILE_E, st, a, dt_hist, t_hist, n); break;
+    case 1: launch_pdl(k_rep_edges<1>, nb, 2 * TILE_E, st, a, rec, dt_hist, t_hist, n); break;
+    case 2: launch_pdl(k_rep_edges<2>, nb, 2 * TILE_E, st, a, rec, dt_hist, t_hist, n); break;
+    case 3: launch_pdl(k_rep_edges<3>, nb, 2 * TILE_E, st, a, rec, dt_hist, t_hist, n); break;
     default: return CF_ENOTSUP;
   }
   const int nc = a.n_ctiles * TILE_C;
@@ -424,9 +413,8 @@ int launch_replay_step(const StepArgs& a, const double* dt_hist, const double* t
   return chk(cudaGetLastError());
 }
 
-int launch_record(const double4* Unew, const double* zcell, const MemberState* S, int nm, int p, int n, double* dt_hist,
-                  double* t_hist, const int32_t* gcell, int G, double* eta, stream_t s) {
-  launch_pdl(k_record, 1, 256, reinterpret_cast<cudaStream_t>(s), Unew, zcell, S, nm, p, n, dt_hist, t_hist, gcell, G, eta);
+int launch_record(const StepRec& r, const double4* U, stream_t s) {
+  launch_pdl(k_record, 1, 256, reinterpret_cast<cudaStream_t>(s), r, U);
   return chk(cudaGetLastError());
 }
 

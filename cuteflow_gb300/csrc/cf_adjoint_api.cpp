@@ -309,6 +309,15 @@ int forward_impl(cf_adjoint* a, int32_t replay, double* eta_out, double* state_o
   const int32_t Mc = a->Mc;
   double4* X = Mc > 0 ? a->pp : a->seg;
   int p = p0;
+  auto record_row = [&](int32_t k) {   /* the gauges of U^k, the state after step k - 1 */
+    StepRec r{};
+    if (a->G == 0 || k == 0) return r;
+    r.eta = a->eta + (size_t)(k - 1) * a->G;
+    r.gcell = a->gcell;
+    r.zcell = c->zcell;
+    r.ng = a->G;
+    return r;
+  };
   for (int32_t k = 0; k < a->N; ++k) {
     if ((k < Mc && k % a->K == 0) || (k == Mc && k > 0))
       CF_CUDA(c, cudaMemcpyAsync(a->ckpt + (size_t)(k < Mc ? k / a->K : a->nseg) * np, X, np * sizeof(double4),
@@ -320,20 +329,20 @@ int forward_impl(cf_adjoint* a, int32_t replay, double* eta_out, double* state_o
     sa.Uin = X;
     sa.Uout = Y;
     sa.steady = 0;   /* the adjoint's run has N steps: no steady-state stop */
+    StepRec rec = record_row(k);
     if (!replay) {
       sa.mst = a->mst;
+      rec.dt = a->dt_hist + (size_t)k * a->nm;
+      rec.t = a->t_hist + (size_t)k * a->nm;
       sa.sums_out = sums;   /* the element kernel stores the step's sums for the stored records */
-      if ((rc = launch_step(sa, st, nullptr, nullptr))) return fail(c, rc, "step launch failed");
-      rc = launch_record(Y, c->zcell, a->mst, a->nm, p, k, a->dt_hist, a->t_hist, a->gcell, a->G, a->eta, st);
-    } else {
-      if ((rc = launch_replay_step(sa, a->dt_hist, a->t_hist, k, a->flag, sums, st)))
-        return fail(c, rc, "replay launch failed");
-      rc = launch_record(Y, c->zcell, nullptr, a->nm, 0, k, a->dt_hist, a->t_hist, a->gcell, a->G, a->eta, st);
+      if ((rc = launch_step(sa, st, nullptr, nullptr, &rec))) return fail(c, rc, "step launch failed");
+    } else if ((rc = launch_replay_step(sa, a->dt_hist, a->t_hist, k, a->flag, sums, st, rec))) {
+      return fail(c, rc, "replay launch failed");
     }
-    if (rc) return fail(c, rc, "record launch failed");
     X = Y;
     p ^= 1;
   }
+  if (a->G > 0 && (rc = launch_record(record_row(a->N), X, st))) return fail(c, rc, "record launch failed");
   if (state_out && (rc = gather_members(a, X, state_out, 3))) return rc;
   if ((rc = to_user(c, eta_out, a->eta, (size_t)a->N * a->G))) return rc;
   uint32_t flag = 0;

@@ -141,6 +141,18 @@ struct StepArgs {
                                 step (the expressions k_rep_cells stores), or NULL */
 };
 
+/* What a step of the adjoint's forward records: the step's dt and start time of every member (NULL for a
+ * replay), and the elevations h + z of ng gauge elements (gcell) of the state the step starts from (NULL
+ * for the first). */
+struct StepRec {
+  double* dt;
+  double* t;
+  double* eta;
+  const int32_t* gcell;
+  const double* zcell;
+  int32_t ng;
+};
+
 /* ---- host preprocessing (cf_mesh.cpp) ---------------------------------------------- */
 
 struct HostEdge {
@@ -201,12 +213,12 @@ int prepare_mesh(const cf_mesh* m, const cf_params* p, Prep& out, std::string& e
 
 typedef struct CUstream_st* stream_t;
 
-int launch_step(const StepArgs& a, stream_t s, void* ev_mid, void* ev_end);
+int launch_step(const StepArgs& a, stream_t s, void* ev_mid, void* ev_end, const StepRec* rec = nullptr);
 /* the edge kernel of one scheme in the shape a.eblock x a.ept (cf_edges_<IFLUX>.cu) */
-int launch_edges_1(const StepArgs& a, stream_t s);
-int launch_edges_2(const StepArgs& a, stream_t s);
-int launch_edges_3(const StepArgs& a, stream_t s);
-int launch_edges_4(const StepArgs& a, stream_t s);
+int launch_edges_1(const StepArgs& a, stream_t s, const StepRec* rec = nullptr);
+int launch_edges_2(const StepArgs& a, stream_t s, const StepRec* rec = nullptr);
+int launch_edges_3(const StepArgs& a, stream_t s, const StepRec* rec = nullptr);
+int launch_edges_4(const StepArgs& a, stream_t s, const StepRec* rec = nullptr);
 int launch_probe_fp64(double* out, int32_t nblocks, int64_t iters, stream_t s);  /* nblocks x 256 outputs */
 int launch_selftest_xd(int64_t n, uint64_t seed, unsigned long long* bad, int32_t nblocks, stream_t s);
 int launch_cfl(const double4* U, const double4* cstat, const int32_t* ctile_mem, int32_t tile_begin,
@@ -280,10 +292,9 @@ struct AdjArgs {
  * NULL) and, if sums is not NULL, every element's flux and bed sums; non-finite results are
  * OR-ed into *flag. */
 int launch_replay_step(const StepArgs& a, const double* dt_hist, const double* t_hist, int n, uint32_t* flag,
-                       Slot* sums, stream_t s);
-/* gauge elevations h + z of Unew into eta row n; with S, also dt / t of parity p into the histories */
-int launch_record(const double4* Unew, const double* zcell, const MemberState* S, int nm, int p, int n, double* dt_hist,
-                  double* t_hist, const int32_t* gcell, int G, double* eta, stream_t s);
+                       Slot* sums, stream_t s, const StepRec& rec = StepRec{});
+/* the gauge elevations of U */
+int launch_record(const StepRec& r, const double4* U, stream_t s);
 int launch_adjoint_step(const AdjArgs& A, stream_t s);
 /* lambda^0 = lam_own + the edge contributions of the last reverse step, into lam_own */
 int launch_adjoint_final(const AdjArgs& A, stream_t s);

@@ -682,15 +682,15 @@ int launch_probe_fp64(double* out, int32_t nblocks, int64_t iters, stream_t s) {
   return check(cudaGetLastError());
 }
 
-int launch_step(const StepArgs& a, stream_t s, void* ev_mid, void* ev_end) {
+int launch_step(const StepArgs& a, stream_t s, void* ev_mid, void* ev_end, const StepRec* rec) {
   cudaStream_t st = reinterpret_cast<cudaStream_t>(s);
   if (a.phys_inflow && !a.surf_done) launch_pdl(k_surf, a.nmembers, 32, st, a);
   int rc;
   switch (a.iflux) {
-    case 1: rc = launch_edges_1(a, s); break;
-    case 2: rc = launch_edges_2(a, s); break;
-    case 3: rc = launch_edges_3(a, s); break;
-    case 4: rc = launch_edges_4(a, s); break;
+    case 1: rc = launch_edges_1(a, s, rec); break;
+    case 2: rc = launch_edges_2(a, s, rec); break;
+    case 3: rc = launch_edges_3(a, s, rec); break;
+    case 4: rc = launch_edges_4(a, s, rec); break;
     default: return CF_ENOTSUP;
   }
   if (rc != CF_OK) return rc;
