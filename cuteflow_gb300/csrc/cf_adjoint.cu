@@ -305,8 +305,12 @@ struct AdjLanePair {
 /* First-order HLLC (flux_mode 0): the closed-form reverse edge (AdjSide), two lanes per edge as in the
  * edge kernel: ~3,000 instructions a lane, 59 of them FP64 ones.  Us per reverse step, 22k / 51k
  * triangles: 25 / 33 (one thread per edge: 39, latency-bound / 38; on four dual lanes 339 at 200k).
- * 24 warps per SM at 80 registers; 16 at 128 and 20 at 102 measured the same. */
-__global__ void __launch_bounds__(2 * TILE_E, 3) k_adj_edges_hllc(AdjArgs A) {
+ * BLOCKS per SM: 3 (80 registers; 16 and 20 warps per SM measured the same), or 4 (64 registers, some
+ * spilled) where that makes all edges resident at once and 3 would leave a second, nearly empty wave: us
+ * per reverse step at 44k / 51k triangles 46.7 / 48.7 with 3, 44.5 / 45.0 with 4; at 10k / 38k (one wave
+ * either way) 28.3 / 37.9 with 3, 29.3 / 39.2 with 4; at 200k 138.3 with 3, 140.5 with 4. */
+template <int BLOCKS>
+__global__ void __launch_bounds__(2 * TILE_E, BLOCKS) k_adj_edges_hllc(AdjArgs A) {
   const StepArgs& a = A.s;
   const int tile = blockIdx.x;
   const int m = __ldg(a.etile_mem + tile);
@@ -418,13 +422,19 @@ int launch_record(const StepRec& r, const double4* U, stream_t s) {
   return chk(cudaGetLastError());
 }
 
+static void adj_edges_hllc(const AdjArgs& A, cudaStream_t st) {
+  const int n = A.s.n_etiles, sms = 152;
+  if (n > 3 * sms && n <= 4 * sms) launch_pdl(k_adj_edges_hllc<4>, n, 2 * TILE_E, st, A);
+  else launch_pdl(k_adj_edges_hllc<3>, n, 2 * TILE_E, st, A);
+}
+
 int launch_adjoint_step(const AdjArgs& A, stream_t s) {
   cudaStream_t st = reinterpret_cast<cudaStream_t>(s);
   const StepArgs& a = A.s;
   launch_pdl(k_adj_cells, a.n_ctiles * (TILE_C / ADJ_CELLS_BLOCK), ADJ_CELLS_BLOCK, st, A);
   switch (a.iflux) {
     case 1:
-      if (a.flux_mode == 0) launch_pdl(k_adj_edges_hllc, a.n_etiles, 2 * TILE_E, st, A);
+      if (a.flux_mode == 0) adj_edges_hllc(A, st);
       else launch_pdl(k_adj_edges<1, 6>, a.n_etiles, TILE_E, st, A);
       break;
     case 2: launch_pdl(k_adj_edges<2, 3>, a.n_etiles, TILE_E, st, A); break;
