@@ -292,6 +292,7 @@ int create_impl(const cf_mesh* meshes, const cf_params* params, int32_t nm, cf_c
   c->ne_pad = (int32_t)eoff;
   c->n_ctiles = c->n_pad / TILE_C;
   c->n_etiles = c->ne_pad / TILE_E;
+  c->eblock = 2 * c->ne_pad <= ONE_WAVE_LANES ? 64 : 256;
   cudaError_t e = cudaGetDevice(&c->device);
   if (e != cudaSuccess) return done(cuda_fail(c, e, "cudaGetDevice"));
   e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);

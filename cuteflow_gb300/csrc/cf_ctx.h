@@ -18,6 +18,7 @@
 
 namespace cf {
 
+constexpr int ONE_WAVE_LANES = 152 * 1024;   /* edge sides resident at once: 1024 threads on each SM */
 constexpr int GRAPH_RUN = 16;   /* steps of the longer captured graph */
 
 /* One simulation of a context: its inputs, host tables and place in the flat space. */
@@ -73,9 +74,12 @@ struct cf_ctx {
    * 46, WAF 25k 51 / 35, descent of 22k 191 / 160), so that a caller who does not tune has it too. */
   int32_t xd_cmp = 1;                  /* integer comparisons */
   int32_t xd_mul_mask = 0x1f;          /* warps multiplying on the integer pipes, XD_CELLS */
-  /* launch shape (cf_set_launch_shape): the autotuner's usual choice on the 1M WAF step, 2-3 %
-   * faster there than (128, 1, 256) */
-  int32_t eblock = 256, ept = 1;       /* edge kernel: threads per block, edges per thread */
+  /* launch shape (cf_set_launch_shape): threads per block of the edge kernel and sides that each lane
+   * evaluates.  Blocks of 64 where all edges are resident at once (small blocks spread over more SMs),
+   * of 256 on larger meshes (one program's instructions serve more warps); us per step with 64 / 256:
+   * canal 1.4k triangles 19.1 / 19.4, reach 6k 22.2 / 22.6, WAF 25k 30.0 / 30.8; ensemble of 150k
+   * 81.4 / 82.0, dam break 134k 59.1 / 58.9, WAF 201k 154 / 149, 1M 245 / 242, MUSCL 201k 126 / 122. */
+  int32_t eblock = 256, ept = 1;
   int32_t cblock = 128;                /* threads per block of the element kernel */
   cf::MemberState* host_state = nullptr;   /* pinned, one record per member */
   bool direct_io = true;               /* kernels read / write callers' pinned host states directly */

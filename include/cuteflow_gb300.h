@@ -305,16 +305,17 @@ int cf_part_apply_discharges(cf_ctx* ctx, double q_in, double q_out);
 /* How the step shares its FP64 work between GB300's FP64 pipe and its integer pipes (results
  * are identical bit for bit in every setting): int_compare 1 evaluates the edge kernel's
  * comparisons on integer keys of the bit patterns; bits 0-3 of int_mul_warps are a mask over
- * the 4 warps of an edge block, and the warps whose bit is set form products, quotients, square
- * roots and scalings by 2^k in exact integer arithmetic on the significands (correctly rounded,
- * the IEEE results); bit 4 does the same for the element kernel.  Default (0, 0): every
- * operation on the FP64 pipe.  cf_autotune picks a setting by timing. */
+ * the four groups of 32 edges of a tile of 128, and the groups whose bit is set form products, quotients,
+ * square roots and scalings by 2^k in exact integer arithmetic on the significands (correctly rounded,
+ * the IEEE results); bit 4 does the same for the element kernel.  Default (1, 0x1f): everything but the
+ * sums on the integer pipes.  cf_autotune picks a setting by timing. */
 int cf_set_tuning(cf_ctx* ctx, int32_t int_compare, int32_t int_mul_warps);
 int cf_get_tuning(cf_ctx* ctx, int32_t* int_compare, int32_t* int_mul_warps);
 /* Launch shape of the step (no counterpart in the reference, whose launch shapes are fixed,
- * finite_volumes_method.cuf:85-109): threads per block of the edge kernel (64, 128 or 256), edges
- * each of its threads evaluates (1 or 2), threads per block of the element kernel (128 or 256).
- * Default (256, 1, 128).  Results are identical bit for bit in every shape. */
+ * finite_volumes_method.cuf:85-109): threads per block of the edge kernel (64, 128 or 256; two
+ * threads evaluate an edge), sides of edges each of its threads evaluates (1 or 2), threads per block
+ * of the element kernel (128 or 256).  Default (64, 1, 128) up to 77,824 edges, (256, 1, 128) above.
+ * Results are identical bit for bit in every shape. */
 int cf_set_launch_shape(cf_ctx* ctx, int32_t edge_block, int32_t edges_per_thread, int32_t cell_block);
 int cf_get_launch_shape(cf_ctx* ctx, int32_t* edge_block, int32_t* edges_per_thread, int32_t* cell_block);
 /* Autotuner: times steps_per_trial steps on the context's own state and keeps the fastest
