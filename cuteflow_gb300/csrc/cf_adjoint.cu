@@ -23,7 +23,8 @@
  * floors, the wet/dry clamp of the update) is the one the forward took.  For an edge the D
  * derivative lanes run in chunks over its 6 (first order) or 10 (WAF: + the upwind
  * reconstructions) inputs; D trades registers for repeated value lanes.  The element stage
- * is transposed by hand (adj_element), and so is the first-order HLLC edge (adj_edge_hllc).
+ * is transposed by hand (adj_element), and so is the first-order HLLC edge of flux_mode 0 (AdjSide, two
+ * lanes per edge).
  *
  * Replay kernels (k_rep_edges, k_rep_cells) advance a state with a recorded dt / time
  * sequence; they run the step's own edge_lanes / element_update, so a replayed trajectory is

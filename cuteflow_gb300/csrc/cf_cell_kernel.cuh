@@ -6,8 +6,8 @@
  * instructions for it, which is the least work; two neighbouring lanes, one for each component of the
  * momentum (ElemSide in cf_flux.h), take ~2,260 each, with the depth's part on both.  So small meshes,
  * whose elements leave the GPU partly idle, go by two lanes and large ones by one thread: us per step
- * by two lanes / by one, 1.4k triangles 21.6 / 24.0, 6k 27.8 / 30.3, 25k 33.3 / 34.7, 51k (gradient) 96.8
- * / 96.6, dam break 80k 49.8 / 44.7, 134k 70.6 / 64.1, WAF 1M 274 / 248.
+ * by two lanes / by one, when the line was drawn: 1.4k triangles 21.6 / 24.0, 6k 27.8 / 30.3, 25k 33.3 /
+ * 34.7, 51k (gradient) 96.8 / 96.6, dam break 80k 49.8 / 44.7, 134k 70.6 / 64.1, WAF 1M 274 / 248.
  */
 #ifndef CF_CELL_KERNEL_CUH
 #define CF_CELL_KERNEL_CUH

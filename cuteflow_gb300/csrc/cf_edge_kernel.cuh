@@ -8,11 +8,13 @@
  * TILE_E = 128 edges, each owned by one member, whatever the shape: a lane looks up its edge's member,
  * and the integer-pipe warp mask bit w applies to the edges (e mod 128) / 32 = w of a tile.  Every
  * shape evaluates the same edges with the same arithmetic, so results do not depend on it (the
- * autotuner chooses one).
+ * autotuner chooses one; cf_ctx.h has the one a context starts with).
  *
- * What bounds it: a wet WAF side is ~4,100 instructions of which 55 are FP64 ones (76 cycles each on
+ * What bounds it: a wet WAF side is ~4,000 instructions of which 55 are FP64 ones (76 cycles each on
  * their pipe): issue slots 58 %, FP64 pipe 65 %, the two integer pipes 56 and 41 % busy, waits on
- * fixed latencies and on instruction fetch between them (WAF 201k triangles, fully wet).
+ * fixed latencies and on instruction fetch between them (WAF 201k triangles, fully wet: 185 us
+ * per step with one thread per edge for both sides, 153 with two lanes, 149 with the limiter's shared
+ * branches and overlapping launches).
  *
  * Register budget: every IFLUX 1-3 shape keeps 1024 threads per SM (at most 64 registers); 768, 1280
  * and 1536 threads measured the same within 3 % or slower (WAF 201k: 168 us per step at 1024; 172, 175,

@@ -129,11 +129,11 @@ struct StepArgs {
   int32_t surf_done;         /* phys_inflow and steady: the step before has left this step's inlet sums */
   int32_t surf_next;         /* ... and this step leaves the next one's (k_between in k_discharge's place) */
   int32_t xd_cmp;            /* edge kernel: 1 = comparisons on integer keys (cf_xd.h) */
-  int32_t xd_mul_mask;       /* with xd_cmp: the edges of warp w (0-3) of an edge tile with bit w set,
-                                and with bit 4 (XD_CELLS) the element kernel, form products,
+  int32_t xd_mul_mask;       /* with xd_cmp: the edges 32 w .. 32 w + 31 (w 0-3) of an edge tile with bit
+                                w set, and with bit 4 (XD_CELLS) the element kernel, form products,
                                 quotients and roots on the integer pipes */
   int32_t eblock, ept;       /* launch shape of the edge kernel: threads per block (64, 128, 256) and
-                                edges per thread (1, 2) */
+                                sides that each thread evaluates (1, 2) */
   int32_t cblock;            /* threads per block of the element kernel (128, 256) */
   int32_t c_lo, c_hi;        /* elements the element kernel updates: [c_lo, c_hi) of the flat space */
   const int32_t* bq;         /* boundary edges of every member in reference order (MemberDev.bq_*) */

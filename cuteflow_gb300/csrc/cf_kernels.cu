@@ -3,26 +3,25 @@
  *
  * One step is two kernels on the context's stream:
  *
- *   k_edges : one thread per edge (cf_edge_kernel.cuh, in every launch shape).  Loads both elements' {h, hu, hv, z}, solves the Riemann
- *             problem once (wave speeds, physical and HLL fluxes), and writes into the edge's
- *             two slots the flux each side computes for itself in the reference
- *             (flux_riemann.cuf:33-426 evaluates every interior edge from both elements).
- *             The two evaluations share everything but a few branch decisions and, for WAF,
- *             the limiter ratios; those are re-evaluated for the second side from exact
- *             mirror identities, so the result is the reference's two-sided flux at about
- *             the cost of one evaluation.  flux_mode 1 writes the negated A-side flux to side
- *             B instead (exactly conservative).  The bed-slope source of each side
- *             (source_terms.cuf:54-100) is computed here as well.
- *   k_cells : one thread per element.  Gathers its three slots in the reference's edge order,
+ *   k_edges : two neighbouring lanes per edge, one for each side (cf_edge_kernel.cuh, in every
+ *             launch shape).  The reference evaluates every interior edge from both elements
+ *             (flux_riemann.cuf:33-426); each lane evaluates its side's share of the wave speeds,
+ *             physical fluxes and limiter ratios, takes the other side's from its neighbour, where
+ *             exact mirror identities make them the same values, and writes its side's slot.
+ *             flux_mode 1 writes the negated A-side flux to side B instead (exactly
+ *             conservative).  The bed-slope source of each side (source_terms.cuf:54-100) is
+ *             computed here as well.
+ *   k_cells : one thread per element, or two lanes on small meshes.  Gathers its three slots in the reference's edge order,
  *             applies Manning friction with the semi-implicit (I - dt/2 J)^-1 matrix
  *             (source_terms.cuf:102-210), updates with the wet/dry clamp
  *             (finite_volumes_method.cuf:283-303), and evaluates the CFL time step of the new
  *             state (cfl_condition.cuf:20-37); a warp-shuffle + block minimum per tile folds
  *             it into the member's next dt with one ordered-integer atomicMin.
  *
- * Everything is FP64.  The step is bound by the FP64 pipe (GB300: 2 DFMA/clk/SM), not by
- * HBM, so the code spends FP64 instructions carefully: geometry is precomputed, divisions
- * that share a denominator become one reciprocal, and sign tests are integer tests.
+ * Everything is FP64.  The step is bound by arithmetic, not by HBM: the FP64 pipe (GB300: one
+ * instruction per warp and SM sub-partition in 76 cycles) carries the sums, the integer pipes the
+ * exact products, quotients, roots and comparisons (cf_xd.h), and neither is idle.  So geometry is
+ * precomputed and divisions that share a denominator become one reciprocal.
  */
 #include <cuda_runtime.h>
 

@@ -26,7 +26,7 @@
  *
  * What is expanded in place and what is called is a matter of the instruction cache: products and
  * quotients are in place (a call costs ~13 instructions), roots, the products and quotients outside the
- * fast path and the limiter are called.  WAF 201k triangles / dam break 134k, us per step: 154 / 65;
+ * fast path and the limiter are called.  WAF 201k triangles / dam break 134k, us per step, when it was decided: 154 / 65;
  * with the uncovered products in place 162 / 65; with every quotient called 156 / 66; with every
  * product called too 173 / 74.
  */
