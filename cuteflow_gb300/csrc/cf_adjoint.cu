@@ -124,9 +124,8 @@ __global__ void k_record(StepRec r, const double4* U) { record_gauges(r, U); }
 /* lambda^{n+1} of element c: its own part plus the contributions the edge adjoint of step n+1
  * left in its three slots and in the upwind entries it belongs to, plus the objective's
  * weights of the gauges it carries; fixed order. */
-__device__ __forceinline__ double4 gather_lambda(const AdjArgs& A, int c, const double* gw) {
+__device__ __forceinline__ double4 gather_lambda(const AdjArgs& A, int c, const int4& sl, int2 gauges, const double* gw) {
   double4 L = ld4(A.lam_own + c);
-  const int4 sl = __ldg(A.s.cslot + c);
   const double4 e0 = ld4(A.eadj + sl.x), e1 = ld4(A.eadj + sl.y), e2 = ld4(A.eadj + sl.z);
   L.x = L.x + e0.x + e1.x + e2.x;
   L.y = L.y + e0.y + e1.y + e2.y;
@@ -140,14 +139,14 @@ __device__ __forceinline__ double4 gather_lambda(const AdjArgs& A, int c, const 
     }
   }
   if (gw)
-    for (int j = __ldg(A.goff + c), j1 = __ldg(A.goff + c + 1); j < j1; ++j) L.x += gw[__ldg(A.gidx + j)];
+    for (int j = gauges.x; j < gauges.y; ++j) L.x += gw[__ldg(A.gidx + j)];
   return L;
 }
 
 /* The transposed element stage (adj_element) of every element, with lambda gathered first.  Its values
- * and lone products run on the integer pipes, its sums and multiply-adds on the FP64 pipe: ~60 FP64
+ * and lone products run on the integer pipes, its sums and multiply-adds on the FP64 pipe: ~40 FP64
  * instructions per element, 243 while the friction ran on four dual lanes (51k triangles, with the
- * reverse edge at its own four blocks: backward and forward of 50 steps 5.9 -> 4.8 ms).  Five, six and
+ * reverse edge then at one thread per edge: backward and forward of 50 steps 5.9 -> 4.8 ms).  Five, six and
  * eight blocks per SM measure the same within 3 %. */
 constexpr int ADJ_CELLS_BLOCK = 128;
 __global__ void __launch_bounds__(ADJ_CELLS_BLOCK, 6) k_adj_cells(AdjArgs A) {
@@ -155,15 +154,23 @@ __global__ void __launch_bounds__(ADJ_CELLS_BLOCK, 6) k_adj_cells(AdjArgs A) {
   const int c = blockIdx.x * ADJ_CELLS_BLOCK + threadIdx.x;
   const int mem = __ldg(a.ctile_mem + c / TILE_C);
   const MemberDev& M = a.mdev[mem];
+  const bool active = c < M.cell_end;
+  int4 sl = make_int4(0, 0, 0, 0);
+  int2 gauges = make_int2(0, 0);
+  if (active) {   /* the tables before the wait (here and below; 10k triangles 28.5 -> 27.9 us per reverse step) */
+    sl = __ldg(a.cslot + c);
+    if (A.gw) gauges = make_int2(__ldg(A.goff + c), __ldg(A.goff + c + 1));
+  }
   pdl_begin();
-  if (c >= M.cell_end) return;
-  const double4 L = A.gather ? gather_lambda(A, c, A.gw) : ld4(A.lam_init + c);
+  if (!active) return;
   const double dt = A.dt_hist[hidx(A.n, mem, a.nmembers)];
+  const double4 U = ld4(a.Uin + c), st = ld4(a.cstat + c);
   const Slot sums = load_slot(A.sums + c);
+  const double4 L = A.gather ? gather_lambda(A, c, sl, gauges, A.gw) : ld4(A.lam_init + c);
   double4 own;
   Slot w;
   double nb;
-  adj_element(M, ld4(a.Uin + c), ld4(a.cstat + c), sums, L, dt, own, w, nb);
+  adj_element(M, U, st, sums, L, dt, own, w, nb);
   A.lam_own[c] = own;
   store_slot(A.cadj + c, w.f1, w.f2, w.f3, w.bx, w.by, w.q);
   A.gman[c] += nb;
@@ -317,16 +324,18 @@ __global__ void __launch_bounds__(2 * TILE_E, BLOCKS) k_adj_edges_hllc(AdjArgs A
   const int m = __ldg(a.etile_mem + tile);
   const MemberDev& M = a.mdev[m];
   const int e = tile * TILE_E + (threadIdx.x >> 1), side = threadIdx.x & 1;
-  pdl_begin();
   const bool live = e < M.edge_end;
-  int2 ab = make_int2(0, -3);
-  if (live) ab = ldro(a.ecell + e);
+  EdgeHead E;
+  E.load(a, e, live);
+  double2 z = make_double2(0.0, 0.0);
+  if (live) z = ldro(reinterpret_cast<const double2*>(a.ez + e));
+  pdl_begin();
+  const int2 ab = E.ab;
   const bool run = live && ab.y >= 0;
   const unsigned mask = __ballot_sync(0xffffffffu, run);
   if (run) {
     const int c = side ? ab.y : ab.x;
-    const double4 geo = ld4(a.egeo + e), U = ld4(a.Uin + c);
-    const double2 z = ldro(reinterpret_cast<const double2*>(a.ez + e));
+    const double4 geo = E.geo, U = ld4(a.Uin + c);
     const Slot wc = load_slot(A.cadj + c);
     const double w[5] = {wc.f1, wc.f2, wc.f3, wc.bx, wc.by};
     AdjLanePair p;
@@ -346,7 +355,7 @@ __global__ void __launch_bounds__(TILE_C) k_adj_final(AdjArgs A) {
   const MemberDev& M = A.s.mdev[__ldg(A.s.ctile_mem + tile)];
   const int c = tile * TILE_C + threadIdx.x;
   if (c >= M.cell_end) return;
-  A.lam_own[c] = gather_lambda(A, c, nullptr);
+  A.lam_own[c] = gather_lambda(A, c, __ldg(A.s.cslot + c), make_int2(0, 0), nullptr);
 }
 
 /* lambda.h += the objective's weights of the gauges an element carries (the final state's
