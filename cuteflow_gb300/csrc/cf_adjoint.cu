@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(2 * TILE_E, 4) k_rep_edges(StepArgs a, StepRec
   E.load(a, e, e < M.edge_end);
   pdl_begin();
   const size_t h = hidx(n, m, a.nmembers);
-  edge_lanes<IFLUX>(a, M, E, e, threadIdx.x & 1, e < M.edge_end, dt_hist[h], t_hist[h], nullptr);
+  edge_lanes<IFLUX>(a, M, E, e, e, threadIdx.x & 1, e < M.edge_end, dt_hist[h], t_hist[h], nullptr);
 }
 
 template <int LANES>

@@ -6,7 +6,8 @@
  * sides (EdgeSide in cf_flux.h: what the sides share goes through shuffles), each lane evaluating EPT
  * sides (i, i + BE, ... of its block's BE * EPT consecutive ones).  Edges keep their layout of tiles of
  * TILE_E = 128 edges, each owned by one member, whatever the shape: a lane looks up its edge's member,
- * and the integer-pipe warp mask bit w applies to the edges (e mod 128) / 32 = w of a tile.  Every
+ * and the integer-pipe warp mask bit w applies to the edges (e mod 128) / 32 = w of a tile (of a list: by
+ * their position in it).  Every
  * shape evaluates the same edges with the same arithmetic, so results do not depend on it (the
  * autotuner chooses one; cf_ctx.h has the one a context starts with).
  *
@@ -119,12 +120,14 @@ struct EdgeHead {
   }
 };
 
-/* Edge e of a step on the lanes of its two sides, in the context's arithmetic type.  Every lane of the
- * warp comes here; live: the lane's edge is one to evaluate (the 16 edges of a warp belong to one
- * tile, so to one member and one setting of the integer-pipe mask). */
+/* Edge e of a step, at position pos of the kernel's order, on the lanes of its two sides, in the
+ * context's arithmetic type.  Every lane of the warp comes here; live: the lane's edge is one to evaluate.
+ * The shuffles name every lane whose edge is evaluated, so the 16 edges of a warp have to be of one member
+ * and of one arithmetic type: int_products goes by the position, which a warp's edges share up to the last
+ * four bits, and not by the edge's number (those of a list are of any tile). */
 template <int IFLUX>
-__device__ __forceinline__ void edge_lanes(const StepArgs& a, const MemberDev& M, const EdgeHead& E, int e, int side,
-                                           bool live, double dt, double t, const double* surf) {
+__device__ __forceinline__ void edge_lanes(const StepArgs& a, const MemberDev& M, const EdgeHead& E, int e, int pos,
+                                           int side, bool live, double dt, double t, const double* surf) {
   const int2 ab = E.ab;
   const double4 geo = E.geo;
   double4 U = make_double4(0.0, 0.0, 0.0, 0.0);
@@ -142,7 +145,7 @@ __device__ __forceinline__ void edge_lanes(const StepArgs& a, const MemberDev& M
     if (a.xd_cmp) {
       /* the same arithmetic with exact integer comparisons and, in the warps of xd_mul_mask, exact
        * integer products, quotients and roots: the FP64 pipe and the integer pipes share the work */
-      if ((a.xd_mul_mask >> ((e % TILE_E) >> 5)) & 1) edge_side<IFLUX, XD<true>>(a, M, mask, e, side, geo, U, dt);
+      if (int_products(a.xd_mul_mask, pos)) edge_side<IFLUX, XD<true>>(a, M, mask, e, side, geo, U, dt);
       else edge_side<IFLUX, XD<false>>(a, M, mask, e, side, geo, U, dt);
     } else {
       edge_side<IFLUX, double>(a, M, mask, e, side, geo, U, dt);
@@ -177,7 +180,7 @@ __device__ __forceinline__ void edges_block(const StepArgs& a, const StepRec* r)
       }
       step_start(M, S, p);
     }
-    edge_lanes<IFLUX>(a, M, E, e, i & 1, e < M.edge_end, dt, t, S->surf);
+    edge_lanes<IFLUX>(a, M, E, e, e, i & 1, e < M.edge_end, dt, t, S->surf);
   }
 }
 
@@ -208,7 +211,7 @@ __global__ void __launch_bounds__(TILE_E, (IFLUX == 4) ? 4 : 8) k_edges_list(Ste
   const int e = i < n ? list[i] : 0;
   EdgeHead E;
   E.load(a, e, i < n && e < M.edge_end);
-  edge_lanes<IFLUX>(a, M, E, e, threadIdx.x & 1, i < n && e < M.edge_end, S->dt[a.parity], S->t[a.parity], S->surf);
+  edge_lanes<IFLUX>(a, M, E, e, i, threadIdx.x & 1, i < n && e < M.edge_end, S->dt[a.parity], S->t[a.parity], S->surf);
 }
 
 template <int IFLUX, int BE, int EPT>

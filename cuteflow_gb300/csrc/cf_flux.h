@@ -1474,6 +1474,10 @@ CF_HD CF_INLINE void boundary_slot(const StepArgs& a, const MemberDev& M, int e,
   store_slot(a.slots + 2 * (size_t)e, f1 * len, f2 * len, f3 * len, 0.0, 0.0, q * len);
 }
 
+/* Whether the edge at position pos of the order in which a kernel takes its edges forms its products on
+ * the integer pipes, by the tuning mask: one answer for each 32 consecutive positions. */
+CF_HD CF_INLINE bool int_products(int32_t mask, int pos) { return (mask >> ((pos % TILE_E) >> 5)) & 1; }
+
 /* A side's flux times the length, and its bed source, into its slot */
 template <class T>
 CF_HD CF_INLINE void store_side(Slot* p, const T out[5], double len) {

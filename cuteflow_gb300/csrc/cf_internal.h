@@ -129,8 +129,8 @@ struct StepArgs {
   int32_t surf_done;         /* phys_inflow and steady: the step before has left this step's inlet sums */
   int32_t surf_next;         /* ... and this step leaves the next one's (k_between in k_discharge's place) */
   int32_t xd_cmp;            /* edge kernel: 1 = comparisons on integer keys (cf_xd.h) */
-  int32_t xd_mul_mask;       /* with xd_cmp: the edges 32 w .. 32 w + 31 (w 0-3) of an edge tile with bit
-                                w set, and with bit 4 (XD_CELLS) the element kernel, form products,
+  int32_t xd_mul_mask;       /* with xd_cmp: the edges 32 w .. 32 w + 31 (w 0-3) of an edge tile (of a
+                                list: of 128 entries) with bit w set, and with bit 4 (XD_CELLS) the element kernel, form products,
                                 quotients and roots on the integer pipes */
   int32_t eblock, ept;       /* launch shape of the edge kernel: threads per block (64, 128, 256) and
                                 sides that each thread evaluates (1, 2) */

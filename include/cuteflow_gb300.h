@@ -305,7 +305,7 @@ int cf_part_apply_discharges(cf_ctx* ctx, double q_in, double q_out);
 /* How the step shares its FP64 work between GB300's FP64 pipe and its integer pipes (results
  * are identical bit for bit in every setting): int_compare 1 evaluates the edge kernel's
  * comparisons on integer keys of the bit patterns; bits 0-3 of int_mul_warps are a mask over
- * the four groups of 32 edges of a tile of 128, and the groups whose bit is set form products, quotients,
+ * the four groups of 32 edges of a tile of 128 (of a part: of 128 edges of its phase's list), and the groups whose bit is set form products, quotients,
  * square roots and scalings by 2^k in exact integer arithmetic on the significands (correctly rounded,
  * the IEEE results); bit 4 does the same for the element kernel.  Default (1, 0x1f): everything but the
  * sums on the integer pipes.  cf_autotune picks a setting by timing. */
