@@ -170,7 +170,9 @@ __device__ __forceinline__ void edges_block(const StepArgs& a, const StepRec* r)
     EdgeHead E;
     E.load(a, e, e < M.edge_end);
     if (j == 0) pdl_begin();
-    if (S->status) continue;
+    /* one answer for the warp, whose lanes shuffle below: the member's first lane, in another warp, may be
+     * setting the status, and an earlier side may have split this one */
+    if (__any_sync(0xffffffffu, S->status != 0)) continue;
     const double dt = S->dt[p];
     const double t = S->t[p];
     if (i == 2 * M.edge_begin) {
@@ -207,7 +209,7 @@ __global__ void __launch_bounds__(TILE_E, (IFLUX == 4) ? 4 : 8) k_edges_list(Ste
   const int i = (blockIdx.x * TILE_E + threadIdx.x) >> 1;
   const MemberDev& M = a.mdev[0];
   MemberState* S = a.mst;
-  if (S->status) return;
+  if (__any_sync(0xffffffffu, S->status != 0)) return;
   const int e = i < n ? list[i] : 0;
   EdgeHead E;
   E.load(a, e, i < n && e < M.edge_end);
