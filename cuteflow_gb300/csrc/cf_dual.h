@@ -260,7 +260,7 @@ struct AdjSide : EdgeSide<1, XD<true>> {
   }
   CFD_HD void values1() {
     speeds1();
-    odd = hraw != hr;            /* the other side is nearly dry */
+    odd = hraw != hr || film();  /* the other side is nearly dry, or both are films */
   }
   CFD_HD void values2() {
     const X ar = y[0];
@@ -381,7 +381,7 @@ struct AdjSide : EdgeSide<1, XD<true>> {
       ga = twice(gsr) - gsl;
     }
     if (wl) gh = gh + ga * ConstOps<X>::half(g) / a;   /* a = sqrt(g h) */
-    if (dry) gh = gu = gv = X(0.0);
+    if (dry()) gh = gu = gv = X(0.0);
     bool sh = wet && hw > 0. && !(h < tolisec), su = wet && !(h < tolisec);
     if (one) {
       gh = X(one[0]);

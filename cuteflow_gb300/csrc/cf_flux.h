@@ -986,18 +986,19 @@ template <class T>
 inline T side_limiter(int ilim, T r, T c) { return waf_limiter(ilim, r, c); }
 #endif
 
-/* The flux of a side with the reconstructed state (h, u, v) towards a nearly dry other side at rest of
- * depth hr (IFLUX 1, 2): rare, out of line, in plain doubles (the same bits). */
 #ifdef __CUDACC__
-template <int IFLUX>
-static __host__ __device__ __noinline__ void nearly_dry_flux(double g, double nx, double ny, double h, double u,
-                                                             double v, double hr, double o[3]) {
+#define CF_RARE static __host__ __device__ __noinline__
 #else
-template <int IFLUX>
-static void nearly_dry_flux(double g, double nx, double ny, double h, double u, double v, double hr, double o[3]) {
+#define CF_RARE static
 #endif
+/* The flux of a side with the reconstructed state (h, u, v) towards the right state (hr, ur, vr), by
+ * itself, where the other side's is not its mirror image (IFLUX 1, 2): rare, out of line, in plain doubles
+ * (the same bits). */
+template <int IFLUX>
+CF_RARE void one_sided_flux(double g, double nx, double ny, double h, double u, double v, double hr, double ur, double vr,
+                            double o[3]) {
   TwoFluxT<double> F;
-  first_order_flux<IFLUX>(g, nx, ny, h, u, v, hr, 0.0, 0.0, F);
+  first_order_flux<IFLUX>(g, nx, ny, h, u, v, hr, ur, vr, F);
   o[0] = F.a1;
   o[1] = F.a2;
   o[2] = F.a3;
@@ -1046,10 +1047,17 @@ struct EdgeSide {
   T hup, uup, vup, sloc, sloct, up_h, up_v, upr_h, upr_v;   /* WAF */
   T e1, e2, e3;                  /* IFLUX 2 */
   double dt, d_mrl, y_mrl, d_up, y_up;
-  bool dry;                      /* both reconstructed depths below eps: zero flux */
+  bool thin;                     /* neither reconstructed depth above eps */
   T hraw;                        /* first order: the other side's reconstruction from its raw depth */
 
   static constexpr double eps() { return IFLUX == 1 ? EPS_HLLC : IFLUX == 2 ? EPS_RIADH : EPS_SECOND; }
+  /* both reconstructed depths below eps: zero flux */
+  CF_HD CF_INLINE bool dry() const { return thin && h < eps() && hr < eps(); }
+  /* a depth of exactly eps and none above: the reference's wave speeds of the two sides are then not mirror
+   * images of one another (each takes the right state's for both), so that each side evaluates its own.  (Not
+   * so with WAF, whose eps is a depth of 1e-16: the code of the case alone cost its step 2 % in spilled
+   * registers, 201k triangles 149 -> 153 us.) */
+  CF_HD CF_INLINE bool film() const { return IFLUX <= 2 && thin && !(h < eps() && hr < eps()); }
 
   /* U: own state; z, zo: beds of the own and of the other element */
   CF_HD CF_INLINE void frame(const MemberDev& M, int side_, double nx_, double ny_, double len_, const double4& U,
@@ -1102,7 +1110,7 @@ struct EdgeSide {
     ur = -y[1];
     vr = -y[2];
     if (IFLUX <= 2) hraw = y[3];
-    dry = h < eps() && hr < eps();
+    thin = !(h > eps()) && !(hr > eps());
     gh = g * h;
     a = sqrt(gh);
     s = (side ? ur : h) + (side ? -u : hr);
@@ -1213,11 +1221,11 @@ struct EdgeSide {
     out[0] = x1;
     out[1] = nx * x2 - ny * x3;
     out[2] = ny * x2 + nx * x3;
-    if (dry) out[0] = out[1] = out[2] = T(0.0);
-    if (IFLUX <= 2 && hraw != hr) {
-      /* a nearly dry other side (0 < h <= tolisec), whose raw depth reaches the higher bed */
+    if (dry()) out[0] = out[1] = out[2] = T(0.0);
+    if (IFLUX <= 2 && (hraw != hr || film())) {
+      /* a nearly dry other side at rest (0 < h <= tolisec), whose raw depth reaches the higher bed */
       double o[3];
-      nearly_dry_flux<IFLUX>(g, nx, ny, val(h), val(u), val(v), val(hraw), o);
+      one_sided_flux<IFLUX>(g, nx, ny, val(h), val(u), val(v), val(hraw), val(ur), val(vr), o);
       out[0] = T(o[0]);
       out[1] = T(o[1]);
       out[2] = T(o[2]);
