@@ -146,6 +146,11 @@ template <class T>
 CF_HD CF_INLINE T mulz(const T& a, const T& b) { return a * b; }
 CF_HD CF_INLINE bool is_zero(double x) { return x == 0.0; }
 
+/* -x of a difference x that the other side has formed: a side's own difference of equal numbers is +0 like
+ * the other one's, and not its negation */
+template <class T>
+CF_HD CF_INLINE T mirrored(const T& x) { return 0.0 - x; }
+
 /* 0 - x, and the first row (1, 0, 0) of the semi-implicit matrix applied to (a, b, c); cf_xd.h forms
  * them for its type without the arithmetic where that does not change the value */
 template <class T>
@@ -1011,7 +1016,7 @@ CF_HD CF_INLINE double zero_like(double a, double b, double c) {
 
 /* Both sides of an interior edge, evaluated in lockstep, each in its own frame (normal out of its own
  * element) exactly as the reference evaluates the edge from each of its elements
- * (flux_riemann.cuf:33-426).  On the GPU the two sides are two neighbouring lanes; on the host two
+ * (flux_riemann.cuf:33-426), the sign of a zero wave speed included (mirrored()).  On the GPU the two sides are two neighbouring lanes; on the host two
  * objects.  What one side computes the other one needs mirrored (depths equal, normal and tangential
  * velocities negated, s_L' = -s_R, the mass flux negated: all exact), so every quantity of one side is
  * computed once, by its side, and offered to the other in x[]; after an exchange y[] holds the other
@@ -1138,7 +1143,7 @@ struct EdgeSide {
     x[3] = f2;
   }
   CF_HD CF_INLINE void hll() {
-    sr = -y[0];
+    sr = IFLUX == 3 ? mirrored(y[0]) : -y[0];   /* only WAF looks at the sign of a zero speed */
     s = y[1];                      /* the other side's denominator term, negated in the own frame */
     fr1 = -y[2];
     fr2 = y[3];
@@ -1172,7 +1177,7 @@ struct EdgeSide {
     x[0] = t2;
   }
   CF_HD CF_INLINE void contact2() {
-    const T num = side ? -y[0] : t2, denom = side ? t2 : y[0];
+    const T num = side ? (IFLUX == 3 ? mirrored(y[0]) : -y[0]) : t2, denom = side ? t2 : y[0];
     if (fabs(denom) < eps()) set = halve(u + ur) - (hr - h) * as_ / (h + hr);
     else set = num / denom;
     if (IFLUX == 2) {

@@ -500,6 +500,11 @@ XD_HD XD<true> mulz(const XD<true>& a, const XD<true>& b) {
   if (__builtin_expect(bad & !z, 0)) r = em_mul_rest(a.v, b.v);
   return XD<true>(z ? xjoin(0u, (ah ^ bh) & 0x80000000u) : r);
 }
+template <bool MUL> XD_HD XD<MUL> mirrored(const XD<MUL>& x) {
+  uint32_t lo, hi;
+  xwords(x.v, lo, hi);
+  return XD<MUL>(xjoin(lo, ((hi << 1) | lo) == 0 ? 0u : hi ^ 0x80000000u));
+}
 /* 0 - x but for the sign of a zero, which the update adds to a depth */
 template <bool MUL> XD_HD XD<MUL> zero_minus(const XD<MUL>& x) { return -x; }
 /* a where b and c are finite (0 b and 0 c are zeros then) */
