@@ -1055,7 +1055,7 @@ struct EdgeSide {
   bool thin;                     /* neither reconstructed depth above eps */
   T hraw;                        /* first order: the other side's reconstruction from its raw depth */
 
-  static constexpr double eps() { return IFLUX == 1 ? EPS_HLLC : IFLUX == 2 ? EPS_RIADH : EPS_SECOND; }
+  static constexpr CF_HD CF_INLINE double eps() { return IFLUX == 1 ? EPS_HLLC : IFLUX == 2 ? EPS_RIADH : EPS_SECOND; }
   /* both reconstructed depths below eps: zero flux */
   CF_HD CF_INLINE bool dry() const { return thin && h < eps() && hr < eps(); }
   /* a depth of exactly eps and none above: the reference's wave speeds of the two sides are then not mirror
