@@ -334,6 +334,7 @@ int forward_impl(cf_adjoint* a, int32_t replay, double* eta_out, double* state_o
       sa.mst = a->mst;
       rec.dt = a->dt_hist + (size_t)k * a->nm;
       rec.t = a->t_hist + (size_t)k * a->nm;
+      recording_shape(sa, c->shape_chosen);
       sa.sums_out = sums;   /* the element kernel stores the step's sums for the stored records */
       if ((rc = launch_step(sa, st, nullptr, nullptr, &rec))) return fail(c, rc, "step launch failed");
     } else if ((rc = launch_replay_step(sa, a->dt_hist, a->t_hist, k, a->flag, sums, st, rec))) {

@@ -829,6 +829,7 @@ int cf_set_launch_shape(cf_ctx* ctx, int32_t edge_block, int32_t edges_per_threa
   if ((edge_block != 64 && edge_block != 128 && edge_block != 256) || (edges_per_thread != 1 && edges_per_thread != 2) ||
       (cell_block != 128 && cell_block != 256))
     return fail(ctx, CF_EINVAL, "launch shape: edge_block 64, 128 or 256, edges_per_thread 1 or 2, cell_block 128 or 256");
+  ctx->shape_chosen = true;
   if (ctx->eblock != edge_block || ctx->ept != edges_per_thread || ctx->cblock != cell_block) {
     ctx->eblock = edge_block;
     ctx->ept = edges_per_thread;
@@ -866,6 +867,7 @@ int cf_autotune(cf_ctx* ctx, int32_t steps_per_trial, int32_t* int_compare, int3
   std::vector<MemberState> ms(c->host_state, c->host_state + nm);
   const int64_t launched0 = c->launched;
   const int32_t cmp0 = c->xd_cmp, mul0 = c->xd_mul_mask, eb0 = c->eblock, ept0 = c->ept, cb0 = c->cblock;
+  const bool chosen0 = c->shape_chosen;
   auto restore = [&]() -> int {
     CF_CUDA(c, cudaMemcpyAsync(c->U[0], saved, np * sizeof(double4), cudaMemcpyDeviceToDevice, c->stream));
     CF_CUDA(c, cudaMemcpyAsync(c->U[1], saved + np, np * sizeof(double4), cudaMemcpyDeviceToDevice, c->stream));
@@ -941,6 +943,7 @@ int cf_autotune(cf_ctx* ctx, int32_t steps_per_trial, int32_t* int_compare, int3
   if (rc != CF_OK) {
     cf_set_tuning(c, cmp0, mul0);
     cf_set_launch_shape(c, eb0, ept0, cb0);
+    c->shape_chosen = chosen0;
     restore();
     return rc;
   }

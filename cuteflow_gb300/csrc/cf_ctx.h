@@ -80,6 +80,7 @@ struct cf_ctx {
    * canal 1.4k triangles 19.1 / 19.4, reach 6k 22.2 / 22.6, WAF 25k 30.0 / 30.8; ensemble of 150k
    * 81.4 / 82.0, dam break 134k 59.1 / 58.9, WAF 201k 154 / 149, 1M 245 / 242, MUSCL 201k 126 / 122. */
   int32_t eblock = 256, ept = 1;
+  bool shape_chosen = false;           /* by cf_set_launch_shape or cf_autotune */
   int32_t cblock = 128;                /* threads per block of the element kernel */
   cf::MemberState* host_state = nullptr;   /* pinned, one record per member */
   bool direct_io = true;               /* kernels read / write callers' pinned host states directly */

@@ -194,12 +194,10 @@ __global__ void __launch_bounds__(BE, ((IFLUX == 4) ? 512 : 1024) / BE) k_edges(
 /* The adjoint's forward: a step that also records what the reverse sweep and the objective need of it,
  * the gauges by one block more.  (By a kernel after every step: ~2 us a step; gradient over 51k triangles
  * 4.08 -> 4.00 ms, batched descent iteration 2.74 -> 2.69 ms.) */
-constexpr int REC_BLOCK = 256;
-
-template <int IFLUX>
-__global__ void __launch_bounds__(REC_BLOCK, 1024 / REC_BLOCK) k_edges_rec(StepArgs a, StepRec r) {
+template <int IFLUX, int BE, int EPT>
+__global__ void __launch_bounds__(BE, 1024 / BE) k_edges_rec(StepArgs a, StepRec r) {
   if (r.eta && blockIdx.x == gridDim.x - 1) return record_gauges(r, a.Uin);
-  edges_block<IFLUX, REC_BLOCK, 1, true>(a, &r);
+  edges_block<IFLUX, BE, EPT, true>(a, &r);
 }
 
 /* The edges of a list (a part's phase of its step; a part is a context of one member): TILE_E lanes per
@@ -217,10 +215,16 @@ __global__ void __launch_bounds__(TILE_E, (IFLUX == 4) ? 4 : 8) k_edges_list(Ste
 }
 
 template <int IFLUX, int BE, int EPT>
-void launch_edges_shape(const StepArgs& a, cudaStream_t st) {
+int launch_edges_shape(const StepArgs& a, cudaStream_t st, const StepRec* rec) {
   const int nside = 2 * a.n_etiles * TILE_E;
-  const int per = BE * EPT;
-  launch_pdl(k_edges<IFLUX, BE, EPT>, (nside + per - 1) / per, BE, st, a);
+  const int nb = (nside + BE * EPT - 1) / (BE * EPT);
+  if (!rec) {
+    launch_pdl(k_edges<IFLUX, BE, EPT>, nb, BE, st, a);
+  } else {
+    if constexpr (IFLUX <= 3) launch_pdl(k_edges_rec<IFLUX, BE, EPT>, nb + (rec->eta ? 1 : 0), BE, st, a, *rec);
+    else return CF_ENOTSUP;
+  }
+  return cudaGetLastError() == cudaSuccess ? CF_OK : CF_ECUDA;
 }
 
 }  // namespace
@@ -235,23 +239,16 @@ int launch_edges_list_iflux(const StepArgs& a, const int32_t* list, int32_t n, c
 /* The shapes a context can choose (cf_set_launch_shape): BE in {64, 128, 256}, EPT in {1, 2}. */
 template <int IFLUX>
 int launch_edges_iflux(const StepArgs& a, cudaStream_t st, const StepRec* rec) {
-  if (rec) {
-    if constexpr (IFLUX <= 3)
-      launch_pdl(k_edges_rec<IFLUX>, 2 * a.n_etiles * TILE_E / REC_BLOCK + (rec->eta ? 1 : 0), REC_BLOCK, st, a, *rec);
-    else return CF_ENOTSUP;
-    return cudaGetLastError() == cudaSuccess ? CF_OK : CF_ECUDA;
-  }
   const int key = a.eblock * 10 + a.ept;
   switch (key) {
-    case 641: launch_edges_shape<IFLUX, 64, 1>(a, st); break;
-    case 642: launch_edges_shape<IFLUX, 64, 2>(a, st); break;
-    case 1281: launch_edges_shape<IFLUX, 128, 1>(a, st); break;
-    case 1282: launch_edges_shape<IFLUX, 128, 2>(a, st); break;
-    case 2561: launch_edges_shape<IFLUX, 256, 1>(a, st); break;
-    case 2562: launch_edges_shape<IFLUX, 256, 2>(a, st); break;
+    case 641: return launch_edges_shape<IFLUX, 64, 1>(a, st, rec);
+    case 642: return launch_edges_shape<IFLUX, 64, 2>(a, st, rec);
+    case 1281: return launch_edges_shape<IFLUX, 128, 1>(a, st, rec);
+    case 1282: return launch_edges_shape<IFLUX, 128, 2>(a, st, rec);
+    case 2561: return launch_edges_shape<IFLUX, 256, 1>(a, st, rec);
+    case 2562: return launch_edges_shape<IFLUX, 256, 2>(a, st, rec);
     default: return CF_EINVAL;
   }
-  return cudaGetLastError() == cudaSuccess ? CF_OK : CF_ECUDA;
 }
 
 }  // namespace cf

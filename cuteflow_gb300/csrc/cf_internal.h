@@ -153,6 +153,14 @@ struct StepRec {
   int32_t ng;
 };
 
+/* The edge kernel's shape in a recording forward: the caller's, else 256 x 1 also where the steps start with
+ * blocks of 64 (gradient of 51k triangles 1.1 %, batched descent 1.5 % slower with those). */
+inline void recording_shape(StepArgs& a, bool chosen) {
+  if (chosen) return;
+  a.eblock = 256;
+  a.ept = 1;
+}
+
 /* ---- host preprocessing (cf_mesh.cpp) ---------------------------------------------- */
 
 struct HostEdge {

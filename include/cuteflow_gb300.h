@@ -315,6 +315,7 @@ int cf_get_tuning(cf_ctx* ctx, int32_t* int_compare, int32_t* int_mul_warps);
  * finite_volumes_method.cuf:85-109): threads per block of the edge kernel (64, 128 or 256; two
  * threads evaluate an edge), sides of edges each of its threads evaluates (1 or 2), threads per block
  * of the element kernel (128 or 256).  Default (64, 1, 128) up to 77,824 edges, (256, 1, 128) above.
+ * An adjoint's recording forward takes the shape that was set, or 256 and 1 for its edges if none was.
  * Results are identical bit for bit in every shape. */
 int cf_set_launch_shape(cf_ctx* ctx, int32_t edge_block, int32_t edges_per_thread, int32_t cell_block);
 int cf_get_launch_shape(cf_ctx* ctx, int32_t* edge_block, int32_t* edges_per_thread, int32_t* cell_block);

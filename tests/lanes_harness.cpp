@@ -6,6 +6,17 @@
 
 using namespace cf;
 
+/* The edge kernel's shape in a recording forward of a context with the given shape */
+extern "C" void harness_recording_shape(int32_t eblock, int32_t ept, int32_t chosen, int32_t* out) {
+  StepArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.eblock = eblock;
+  a.ept = ept;
+  recording_shape(a, chosen != 0);
+  out[0] = a.eblock;
+  out[1] = a.ept;
+}
+
 /* The warps of the list kernel over both phases of a part (16 edges each, two lanes an edge): how many hold
  * edges of both arithmetic types under the tuning mask, by the kernel's rule, and by the edges' numbers. */
 extern "C" int harness_list_warps(const cf_mesh* m, const cf_params* p, const int32_t* elem_class, int32_t mask,

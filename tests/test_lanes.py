@@ -39,3 +39,13 @@ def test_a_warp_of_a_parts_list_has_one_arithmetic_type(lib, iflux, nparts):
             assert n[0].value > 0 and n[1].value == 0
             by_number += n[2].value
     assert by_number > 0   # the lists do hold warps whose edges' numbers differ in the mask's bit
+
+
+def test_a_recording_forward_takes_the_shape_that_was_set(lib):
+    out = (C.c_int32 * 2)()
+    for eb in (64, 128, 256):
+        for ept in (1, 2):
+            lib.harness_recording_shape(eb, ept, 1, out)
+            assert tuple(out) == (eb, ept)
+            lib.harness_recording_shape(eb, ept, 0, out)
+            assert tuple(out) == (256, 1)
