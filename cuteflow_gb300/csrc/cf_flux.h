@@ -1497,8 +1497,25 @@ CF_HD CF_INLINE void store_side(Slot* p, const T out[5], double len) {
   store_slot(p, val(out[0] * len), val(out[1] * len), val(out[2] * len), val(out[3]), val(out[4]), 0.0);
 }
 
+/* Interior edge e on the host, whatever its depths: the stages that the edge kernel runs on two lanes */
+template <int IFLUX, class T = double>
+inline void edge_interior(const StepArgs& a, const MemberDev& M, int e, double dt) {
+  const int2 ab = a.ecell[e];
+  const double4 geo = a.egeo[e];
+  Slot* sa = a.slots + 2 * (size_t)e;
+  HostPair<IFLUX, T> p;
+  side_load(a, M, e, 0, geo, a.Uin[ab.x], dt, p.s[0]);
+  side_load(a, M, e, 1, geo, a.Uin[ab.y], dt, p.s[1]);
+  const double4 dk = IFLUX >= 3 ? a.edk[e] : make_double4(0.0, 0.0, 0.0, 0.0);
+  side_stages<IFLUX>(p, a.ilimiteur, dk.x, dk.z, dk.y, dk.w);
+  if (a.flux_mode == 1)
+    for (int k = 0; k < 3; ++k) p.out[1][k] = -p.out[0][k];
+  store_side(sa, p.out[0], geo.z);
+  store_side(sa + 1, p.out[1], geo.z);
+}
+
 /* Fluxes (times the edge length) and bed sources of edge e into its two slots, from the state U of step
- * n, on the host: the stages that the edge kernel runs on two lanes. */
+ * n, on the host. */
 template <int IFLUX, class T = double>
 inline void edge_body(const StepArgs& a, const MemberDev& M, int e, double dt, double t, const double* surf = nullptr) {
   const int2 ab = a.ecell[e];
@@ -1511,15 +1528,7 @@ inline void edge_body(const StepArgs& a, const MemberDev& M, int e, double dt, d
   const double4 UB = a.Uin[ab.y];
   /* an edge between two dry elements (most of a flood plain that the water has not reached) */
   if ((dbits_hd(UA.x) | dbits_hd(UB.x)) == 0 && dry_edge_slots<IFLUX>(M.gp, a.flux_mode, geo, sa, dt)) return;
-  HostPair<IFLUX, T> p;
-  side_load(a, M, e, 0, geo, UA, dt, p.s[0]);
-  side_load(a, M, e, 1, geo, UB, dt, p.s[1]);
-  const double4 dk = IFLUX >= 3 ? a.edk[e] : make_double4(0.0, 0.0, 0.0, 0.0);
-  side_stages<IFLUX>(p, a.ilimiteur, dk.x, dk.z, dk.y, dk.w);
-  if (a.flux_mode == 1)
-    for (int k = 0; k < 3; ++k) p.out[1][k] = -p.out[0][k];
-  store_side(sa, p.out[0], geo.z);
-  store_side(sa + 1, p.out[1], geo.z);
+  edge_interior<IFLUX, T>(a, M, e, dt);
 }
 
 /* ---- one element ------------------------------------------------------------------------ */
