@@ -249,8 +249,6 @@ int launch_inlet_terms(const StepArgs& a, const double4* U, int32_t count, doubl
 int launch_bq_terms(const Slot* slots, const int32_t* bq, const MemberDev* mdev, int32_t count, double* out, stream_t s);
 /* member 0's discharges and steady-state test with given (whole-mesh) discharges */
 int launch_steady_apply(const MemberDev* mdev, MemberState* mst, double qi, double qo, stream_t s);
-/* phys_inflow inlet sums of the state U into mst[m].surf (every member with inlet 3) */
-int launch_surf(const StepArgs& a, const double4* U, stream_t s);
 /* hu3 (reference order, one member) <-> U (new order); perm/iperm/zcell/U point at the member's
  * first element, the permutations hold member-local indices. */
 int launch_scatter_state(const double* hu3, const int32_t* perm_new2old, const double* zcell,
