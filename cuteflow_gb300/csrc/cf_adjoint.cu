@@ -315,8 +315,9 @@ struct AdjLanePair {
  * triangles: 25 / 33 (one thread per edge: 39, latency-bound / 38; on four dual lanes 339 at 200k).
  * BLOCKS per SM: 3 (80 registers; 16 and 20 warps per SM measured the same), or 4 (64 registers, some
  * spilled) where that makes all edges resident at once and 3 would leave a second, nearly empty wave: us
- * per reverse step at 44k / 51k triangles 46.7 / 48.7 with 3, 44.5 / 45.0 with 4; at 10k / 38k (one wave
- * either way) 28.3 / 37.9 with 3, 29.3 / 39.2 with 4; at 200k 138.3 with 3, 140.5 with 4. */
+ * per reverse step with 3 / 4 at 39.4k triangles 42.2 / 39.7, 42k 43.9 / 42.0, 48k 46.2 / 42.9, 51.6k 46.8 /
+ * 43.1; on either side of that, 38.6k 34.5 / 35.5 and 52.4k 47.0 / 49.4.  Where 4 saves the third wave it does
+ * not pay: 79k 61.9 / 61.6, 90k 65.5 / 64.8, 96k 67.5 / 69.2, 103k 70.0 / 71.5; at 200k 138.3 / 140.5. */
 template <int BLOCKS>
 __global__ void __launch_bounds__(2 * TILE_E, BLOCKS) k_adj_edges_hllc(AdjArgs A) {
   const StepArgs& a = A.s;
@@ -433,8 +434,8 @@ int launch_record(const StepRec& r, const double4* U, stream_t s) {
 }
 
 static void adj_edges_hllc(const AdjArgs& A, cudaStream_t st) {
-  const int n = A.s.n_etiles, sms = 152;
-  if (n > 3 * sms && n <= 4 * sms) launch_pdl(k_adj_edges_hllc<4>, n, 2 * TILE_E, st, A);
+  const int n = A.s.n_etiles;
+  if (adj_hllc_blocks(n, A.s.sms) == 4) launch_pdl(k_adj_edges_hllc<4>, n, 2 * TILE_E, st, A);
   else launch_pdl(k_adj_edges_hllc<3>, n, 2 * TILE_E, st, A);
 }
 

@@ -68,6 +68,7 @@ StepArgs step_args(const cf_ctx* c, int parity) {
   a.mst = c->mst;
   a.n_etiles = c->n_etiles;
   a.n_ctiles = c->n_ctiles;
+  a.sms = c->sms;
   a.parity = parity;
   a.iflux = c->iflux;
   a.ilimiteur = c->ilimiteur;
@@ -292,9 +293,11 @@ int create_impl(const cf_mesh* meshes, const cf_params* params, int32_t nm, cf_c
   c->ne_pad = (int32_t)eoff;
   c->n_ctiles = c->n_pad / TILE_C;
   c->n_etiles = c->ne_pad / TILE_E;
-  c->eblock = 2 * c->ne_pad <= ONE_WAVE_LANES ? 64 : 256;
   cudaError_t e = cudaGetDevice(&c->device);
   if (e != cudaSuccess) return done(cuda_fail(c, e, "cudaGetDevice"));
+  e = cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device);
+  if (e != cudaSuccess) return done(cuda_fail(c, e, "cudaDeviceGetAttribute"));
+  c->eblock = first_edge_block(c->ne_pad, c->sms);
   e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) return done(cuda_fail(c, e, "cudaStreamCreate"));
   for (auto& ev : c->ev) {

@@ -5,8 +5,8 @@
  * An element's update is a chain of dependent quotients, products and roots.  One thread takes ~2,900
  * instructions for it, which is the least work; two neighbouring lanes, one for each component of the
  * momentum (ElemSide in cf_flux.h), take ~2,260 each, with the depth's part on both.  So small meshes,
- * whose elements leave the GPU partly idle, go by two lanes and large ones by one thread: us per step
- * by two lanes / by one, when the line was drawn: 1.4k triangles 21.6 / 24.0, 6k 27.8 / 30.3, 25k 33.3 /
+ * whose elements leave the GPU partly idle, go by two lanes and large ones by one thread (two_lanes: the
+ * line is at 38,912 elements on 152 SMs): us per step by two lanes / by one, when the line was drawn: 1.4k triangles 21.6 / 24.0, 6k 27.8 / 30.3, 25k 33.3 /
  * 34.7, 51k (gradient) 96.8 / 96.6, dam break 80k 49.8 / 44.7, 134k 70.6 / 64.1, WAF 1M 274 / 248.
  */
 #ifndef CF_CELL_KERNEL_CUH
@@ -19,10 +19,6 @@
 
 namespace cf {
 namespace {
-
-/* The line between the two: up to 512 lanes for each of the 152 SMs */
-constexpr int TWO_LANE_ELEMENTS = 152 * 256;
-inline bool two_lanes(const StepArgs& a) { return a.n_ctiles * TILE_C <= TWO_LANE_ELEMENTS; }
 
 __device__ __forceinline__ Slot load_slot(const Slot* p) {
   const double2* q = reinterpret_cast<const double2*>(p);

@@ -18,7 +18,6 @@
 
 namespace cf {
 
-constexpr int ONE_WAVE_LANES = 152 * 1024;   /* edge sides resident at once: 1024 threads on each SM */
 constexpr int GRAPH_RUN = 16;   /* steps of the longer captured graph */
 
 /* One simulation of a context: its inputs, host tables and place in the flat space. */
@@ -36,6 +35,7 @@ struct Member {
 
 struct cf_ctx {
   int device = 0;
+  int32_t sms = 0;                     /* its SMs */
   int32_t iflux = 1, ilimiteur = 1, flux_mode = 0;
   std::vector<cf::Member> mem;
   int32_t n_pad = 0, ne_pad = 0, n_etiles = 0, n_ctiles = 0, max_n = 0;
@@ -79,7 +79,7 @@ struct cf_ctx {
    * of 256 on larger meshes (one program's instructions serve more warps); us per step with 64 / 256:
    * canal 1.4k triangles 19.1 / 19.4, reach 6k 22.2 / 22.6, WAF 25k 30.0 / 30.8; ensemble of 150k
    * 81.4 / 82.0, dam break 134k 59.1 / 58.9, WAF 201k 154 / 149, 1M 245 / 242, MUSCL 201k 126 / 122. */
-  int32_t eblock = 256, ept = 1;
+  int32_t eblock = 256, ept = 1;       /* eblock: first_edge_block */
   bool shape_chosen = false;           /* by cf_set_launch_shape or cf_autotune */
   int32_t cblock = 128;                /* threads per block of the element kernel */
   cf::MemberState* host_state = nullptr;   /* pinned, one record per member */

@@ -121,6 +121,7 @@ struct StepArgs {
   const int32_t* inl_cell;   /* phys_inflow entry tables (NULL without phys_inflow) */
   const double* inl_len;
   int32_t n_etiles, n_ctiles;
+  int32_t sms;               /* SMs of the context's device */
   int32_t parity;
   int32_t iflux, ilimiteur, flux_mode;
   int32_t nmembers;
@@ -152,6 +153,17 @@ struct StepRec {
   const double* zcell;
   int32_t ng;
 };
+
+/* The dispatch rules that go by what is resident at once on the device's SMs (GB300: 152); the reasons and
+ * both sides' times stand at their uses. */
+/* cf_ctx.h: blocks of 64 where all sides of the edges are resident, 1024 on each SM */
+inline int32_t first_edge_block(int64_t ne_pad, int32_t sms) { return 2 * ne_pad <= (int64_t)sms * 1024 ? 64 : 256; }
+/* cf_cell_kernel.cuh: an element on two lanes up to 512 lanes for each SM */
+inline bool two_lanes(const StepArgs& a) { return (int64_t)a.n_ctiles * TILE_C <= (int64_t)a.sms * 256; }
+/* k_adj_edges_hllc: four blocks per SM where that makes one wave and three would make two */
+inline int32_t adj_hllc_blocks(int32_t n_etiles, int32_t sms) {
+  return n_etiles > 3 * sms && n_etiles <= 4 * sms ? 4 : 3;
+}
 
 /* The edge kernel's shape in a recording forward: the caller's, else 256 x 1 also where the steps start with
  * blocks of 64 (gradient of 51k triangles 1.1 %, batched descent 1.5 % slower with those). */

@@ -17,6 +17,17 @@ extern "C" void harness_recording_shape(int32_t eblock, int32_t ept, int32_t cho
   out[1] = a.ept;
 }
 
+/* The dispatch rules on a device of sms SMs */
+extern "C" int harness_edge_block(long long ne_pad, int32_t sms) { return first_edge_block(ne_pad, sms); }
+extern "C" int harness_adj_blocks(int32_t n_etiles, int32_t sms) { return adj_hllc_blocks(n_etiles, sms); }
+extern "C" int harness_two_lanes(int32_t n_ctiles, int32_t sms) {
+  StepArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.n_ctiles = n_ctiles;
+  a.sms = sms;
+  return two_lanes(a);
+}
+
 /* The warps of the list kernel over both phases of a part (16 edges each, two lanes an edge): how many hold
  * edges of both arithmetic types under the tuning mask, by the kernel's rule, and by the edges' numbers. */
 extern "C" int harness_list_warps(const cf_mesh* m, const cf_params* p, const int32_t* elem_class, int32_t mask,

@@ -49,3 +49,12 @@ def test_a_recording_forward_takes_the_shape_that_was_set(lib):
             assert tuple(out) == (eb, ept)
             lib.harness_recording_shape(eb, ept, 0, out)
             assert tuple(out) == (256, 1)
+
+
+def test_the_lines_of_the_dispatch_follow_the_number_of_sms(lib):
+    lib.harness_edge_block.argtypes = [C.c_longlong, C.c_int32]
+    for sms in (152, 76, 132):
+        assert lib.harness_edge_block(512 * sms, sms) == 64 and lib.harness_edge_block(512 * sms + 128, sms) == 256
+        assert lib.harness_two_lanes(sms, sms) == 1 and lib.harness_two_lanes(sms + 1, sms) == 0
+        assert [lib.harness_adj_blocks(n, sms) for n in (3 * sms, 3 * sms + 1, 4 * sms, 4 * sms + 1)] == [3, 4, 4, 3]
+    assert lib.harness_edge_block(1 << 30, 152) == 256   # no overflow at the largest context
