@@ -146,6 +146,13 @@ template <class T>
 CF_HD CF_INLINE T mulz(const T& a, const T& b) { return a * b; }
 CF_HD CF_INLINE bool is_zero(double x) { return x == 0.0; }
 
+/* the value of a wave speed for its sign alone, negated for the other side: a zero stays as it is */
+template <class T>
+CF_HD CF_INLINE T opposite(const T& x) {
+  const double v = val(x);
+  return T(zero_u(dbits_hd(v)) ? v : -v);
+}
+
 /* -x of a difference x that the other side has formed: a side's own difference of equal numbers is +0 like
  * the other one's, and not its negation */
 template <class T>
@@ -552,11 +559,12 @@ CF_HD CF_INLINE void waf_flux(double g, int ilim, double nx, double ny, double d
     const T ll = waf_limiter(ilim, rl, -cr);
     const T lr = waf_limiter(ilim, rr, -cl);
     const T le = waf_limiter(ilim, ret_b, -cet);
-    const T wl = halve(1. + sgnmul(-sr, ll));
-    const T wlet = halve(1. + sgnmul(-set, le));
-    const T wlr = halve(sgnmul(-sl, lr) - sgnmul(-sr, ll));
-    const T wr = halve(1. - sgnmul(-sl, lr));
-    const T wret = halve(1. - sgnmul(-set, le));
+    const T nsl = opposite(sl), nsr = opposite(sr), nset = opposite(set);
+    const T wl = halve(1. + sgnmul(nsr, ll));
+    const T wlet = halve(1. + sgnmul(nset, le));
+    const T wlr = halve(sgnmul(nsl, lr) - sgnmul(nsr, ll));
+    const T wr = halve(1. - sgnmul(nsl, lr));
+    const T wret = halve(1. - sgnmul(nset, le));
     /* mirrored physical fluxes: FL' = (-fr1, fr2), FR' = (-fl1, fl2), HLL' = (-hb1, hb2) */
     const T fw1 = -(wl * fr1 + wlr * hb1 + wr * fl1);
     const T fw2 = wl * fr2 + wlr * hb2 + wr * fl2;
