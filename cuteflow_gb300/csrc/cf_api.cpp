@@ -942,14 +942,16 @@ int cf_autotune(cf_ctx* ctx, int32_t steps_per_trial, int32_t* int_compare, int3
       bcb = cb;
     }
   }
-  cudaFree(saved);
-  if (rc != CF_OK) {
+  if (rc != CF_OK) {   /* a trial failed: its message stays, its state and settings do not */
+    const std::string msg = c->err;
     cf_set_tuning(c, cmp0, mul0);
     cf_set_launch_shape(c, eb0, ept0, cb0);
     c->shape_chosen = chosen0;
     restore();
-    return rc;
+    cudaFree(saved);
+    return fail(c, rc, msg);
   }
+  cudaFree(saved);
   if ((rc = cf_set_tuning(c, bc, bm)) || (rc = cf_set_launch_shape(c, beb, bept, bcb))) return rc;
   if (int_compare) *int_compare = bc;
   if (int_mul_warps) *int_mul_warps = bm;
