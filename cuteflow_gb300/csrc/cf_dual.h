@@ -404,8 +404,8 @@ struct AdjSide : EdgeSide<1, XD<true>> {
   }
 };
 
-/* The stages of both sides (P as in side_stages; P::any: some pair at hand takes the one-sided
- * evaluation) */
+/* The stages of both sides (P as in side_stages; P::finish: the last stage, with the one-sided evaluation for
+ * the pairs that take it) */
 template <class P>
 CFD_HD void adj_stages(P& p) {
   p.exchange(4);

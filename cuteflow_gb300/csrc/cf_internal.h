@@ -40,8 +40,8 @@
 
 namespace cf {
 
-constexpr int TILE_E = 128;  /* edges per tile (= edge-kernel block) */
-constexpr int TILE_C = 256;  /* cells per tile (= cell-kernel block) */
+constexpr int TILE_E = 128;  /* edges per tile; an edge kernel's block holds a part of one, or several */
+constexpr int TILE_C = 256;  /* cells per tile; a cell kernel's block lies within one */
 constexpr int32_t XD_CELLS = 0x10;  /* tuning-mask bit of the element kernel */
 
 /* Fortran default-real literals of the reference, rounded to single precision. */

@@ -11,8 +11,8 @@
  *             flux_mode 1 writes the negated A-side flux to side B instead (exactly
  *             conservative).  The bed-slope source of each side (source_terms.cuf:54-100) is
  *             computed here as well.
- *   k_cells : one thread per element, or two lanes on small meshes.  Gathers its three slots in the reference's edge order,
- *             applies Manning friction with the semi-implicit (I - dt/2 J)^-1 matrix
+ *   k_cells : one thread per element, or two lanes on small meshes.  Gathers its three slots in the
+ *             reference's edge order, applies Manning friction with the semi-implicit (I - dt/2 J)^-1 matrix
  *             (source_terms.cuf:102-210), updates with the wet/dry clamp
  *             (finite_volumes_method.cuf:283-303), and evaluates the CFL time step of the new
  *             state (cfl_condition.cuf:20-37); a warp-shuffle + block minimum per tile folds
@@ -279,9 +279,8 @@ constexpr int BQ_BLOCK = 256;
 __device__ __forceinline__ void bq_sync() { asm volatile("bar.sync 1, %0;" ::"n"(BQ_BLOCK) : "memory"); }
 
 /* Discharge diagnostics of the last step (debit_entree_sum, debit_sortie,
- * finite_volumes_method.cuf:197-214): per member, fixed-order sums over its boundary edges
- *.  With steady set (the
- * launch at the end of every step of a context that tests for steady state) it also applies
+ * finite_volumes_method.cuf:197-214): per member, fixed-order sums over its boundary edges.  With steady
+ * set (the launch at the end of every step of a context that tests for steady state) it also applies
  * check_steady_state (finite_volumes_method.cuf:370-393) to the members that stepped:
  * Q_in > 1e-8 (single precision) and |Q_in - Q_out| / Q_in < tol_reg_perm counts a step, any
  * other step resets the count, and more than steady_count stops the member. */

@@ -17,8 +17,12 @@
 namespace cf {
 namespace {
 
-/* Every kernel launched by launch_pdl, or before one that is, calls this before it touches memory that
- * a kernel may have written (a no-op for a kernel without a programmatic dependency). */
+/* A thread of a kernel launched by launch_pdl calls this before it touches memory that a kernel, or a copy
+ * made by a call, may have written; what it may read earlier are the tables (member constants among them)
+ * that the host copied when the context or the adjoint was made.  Some thread of such a kernel calls it in
+ * any case, since its dependents take its end for the end of all kernels before it.  A kernel launched
+ * plainly needs nothing, whichever way its neighbours are launched: it begins when all before it have
+ * ended, and a dependent of it waits here for its end. */
 __device__ __forceinline__ void pdl_begin() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
