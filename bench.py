@@ -173,6 +173,9 @@ def run_reference(args):
     print(json.dumps(line), flush=True)
 
 
+GRAPH_STEPS = 18   # a run of so many steps captures both of the graphs that longer runs replay
+
+
 def ensemble(nmembers: int, steps: int, warmup: int, seed: int = 3):
     """Batched ensemble vs the same members run one after another through the plain API.
 
@@ -189,6 +192,9 @@ def ensemble(nmembers: int, steps: int, warmup: int, seed: int = 3):
     for i, m in enumerate(members):
         b.set_state(i, m.U0)
     tune = b.autotune(20)   # the same setting runs in both forms below (results identical in any)
+    b.step(GRAPH_STEPS, check=False)
+    for i, m in enumerate(members):
+        b.set_state(i, m.U0)
     warm = b.step(warmup, check=False)
     torch.cuda.synchronize()
     t0 = time.perf_counter()
@@ -201,6 +207,8 @@ def ensemble(nmembers: int, steps: int, warmup: int, seed: int = 3):
     for m in members:
         s = Solver(m)
         s.set_tuning(tune[0], tune[1])
+        s.set_state(m.U0)
+        s.step(GRAPH_STEPS, check=False)
         s.set_state(m.U0)
         s.step(warmup, check=False)
         torch.cuda.synchronize()
@@ -243,6 +251,8 @@ def ensemble_sizes(steps: int = 200, warmup: int = 10, sizes=(20000, 50000, 1000
             with Solver(c) as s:
                 s.set_state(c.U0)
                 s.set_tuning(1, 31)
+                s.step(GRAPH_STEPS)
+                s.set_state(c.U0)
                 s.step(warmup)
                 torch.cuda.synchronize()
                 t0 = time.perf_counter()
@@ -254,6 +264,9 @@ def ensemble_sizes(steps: int = 200, warmup: int = 10, sizes=(20000, 50000, 1000
             for i, c in enumerate(mem):
                 b.set_state(i, c.U0)
             b.set_tuning(1, 31)
+            b.step(GRAPH_STEPS, check=False)
+            for i, c in enumerate(mem):
+                b.set_state(i, c.U0)
             b.step(warmup, check=False)
             torch.cuda.synchronize()
             t0 = time.perf_counter()
@@ -311,7 +324,7 @@ def adjoint_leg(steps: int, warmup: int, obs_every: float = 10.0, budget_gb: flo
     # calibration guess: warm-up, then the timed legs
     s.set_manning(n0)
     s.set_state(c.U0)
-    s.step(warmup)
+    s.step(max(warmup, GRAPH_STEPS))
     s.set_state(c.U0)
     _, fwd_ms = timed(lambda: s.step(steps))
     s.set_state(c.U0)
@@ -549,7 +562,7 @@ def run_ours(args):
             for cb in (256, 128):
                 s.set_launch_shape(eb, ept, cb)
                 s.set_state(case.U0)
-                s.step(18)   # both of the graphs that the timed steps replay
+                s.step(GRAPH_STEPS)
                 torch.cuda.synchronize()
                 a0, a1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
                 a0.record(stream)
@@ -560,7 +573,7 @@ def run_ours(args):
     s.set_launch_shape(*shape)
 
     # ---- device-resident throughput (value) ----
-    s.step(18)   # the graphs of the setting, whatever the number of warm-up steps
+    s.step(GRAPH_STEPS)   # whatever the number of warm-up steps
     s.set_state(case.U0)
     s.step(args.warmup)
     barrier()
