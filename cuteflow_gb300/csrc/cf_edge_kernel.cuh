@@ -15,7 +15,7 @@
  * their pipe): issue slots 58 %, FP64 pipe 65 %, the two integer pipes 56 and 41 % busy, waits on
  * fixed latencies and on instruction fetch between them (WAF 201k triangles, fully wet: 185 us
  * per step with one thread per edge for both sides, 153 with two lanes, 149 with the limiter's shared
- * branches and overlapping launches).
+ * branches and overlapping launches, 150 with the signs of zero wave speeds kept).
  *
  * Register budget: every IFLUX 1-3 shape keeps 1024 threads per SM (at most 64 registers); 768, 1280
  * and 1536 threads measured the same within 3 % or slower (WAF 201k: 168 us per step at 1024; 172, 175,
